@@ -259,7 +259,8 @@ void solve_prepare(Ctx *c, const double *centers_dev, const double *radii_dev, c
         res.t_tree_ms = std::chrono::duration<double, std::milli>(w1 - w0).count();
         trace_mark("solve: plan synced");
         if (cfg.precision == IBIM_PRECISION_FP64 || !m2l_tc_supported()) {
-            fmm_prepare_operators(*P, cfg.kp, IBIM_PRECISION_FP64);
+            if (cfg.precision == IBIM_PRECISION_FP64) fmm_prepare_fp64(*P, cfg.kp);
+            else fmm_prepare_operators(*P, cfg.kp, IBIM_PRECISION_FP64);
             if (cfg.precision == IBIM_PRECISION_MIXED) fmm_prepare_operators(*P, cfg.kp, IBIM_PRECISION_MIXED);
         } else {
             // Mixed path in the scaled FP16 form: the FP16 images of the mixed operator and the
@@ -834,6 +835,14 @@ int ibim_tree_lists_host(const double *points, long n, int maxpoint, int maxleve
     });
 }
 
+// Wait for the plan's stream; an M2L wait that ran out of its bound is an error.
+static void sync_checked(Plan &P) {
+    int e = 0;
+    if (P.tc_err.ptr) P.tc_err.download(&e, 1);
+    IBIM_CUDA(cudaStreamSynchronize(P.ctx->stream));
+    if (e) throw Error(IBIM_ERR_LIMIT, "tensor-core M2L: an MMA completion wait exceeded its bound");
+}
+
 int ibim_fmm_apply(ibim_plan p, int kernel, const ibim_kernel_params *kp, const double *in, double *out) {
     return guard([&] {
         IBIM_REQUIRE(p && kp && in && out, "null argument");
@@ -865,7 +874,7 @@ int ibim_fmm_apply(ibim_plan p, int kernel, const ibim_kernel_params *kp, const 
             permute(c, nt, S.perm_d.ptr, S.out4.ptr + kKernelMap[kernel].field * nt, hout.ptr, true);
         }
         hout.download(out, (size_t)rows * nt);
-        IBIM_CUDA(cudaStreamSynchronize(s));
+        sync_checked(P);
         if (rows == 1 && kKernelMap[kernel].sign < 0)
             for (long i = 0; i < nt; ++i) out[i] = -out[i];
     });
@@ -891,7 +900,7 @@ int ibim_bie_matvec(ibim_plan p, const ibim_kernel_params *kp, const double *x, 
         permute(c, n, P.src_perm.ptr, ty.ptr, hy.ptr, true);
         permute(c, n, P.src_perm.ptr, ty.ptr + n, hy.ptr + n, true);
         hy.download(y, 2 * n);
-        IBIM_CUDA(cudaStreamSynchronize(s));
+        sync_checked(P);
     });
 }
 
@@ -944,7 +953,7 @@ int ibim_gmres_solve(ibim_plan p, const ibim_kernel_params *kp, const double *b,
         permute(c, n, P.src_perm.ptr, tx.ptr, hx.ptr, true);
         permute(c, n, P.src_perm.ptr, tx.ptr + n, hx.ptr + n, true);
         hx.download(x, 2 * n);
-        IBIM_CUDA(cudaStreamSynchronize(s));
+        sync_checked(P);
         if (iters) *iters = st.iters;
         if (gmres_status) *gmres_status = rc;
         if (residual) *residual = st.residual;

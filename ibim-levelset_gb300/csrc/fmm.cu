@@ -316,26 +316,124 @@ __global__ void __launch_bounds__(128) k_m2l_x64(const ChebTables *__restrict__ 
 // Near field + L2P for one target leaf per block (downPass leaf, bbfmm.h:571-609): U and W
 // lists direct (source ranges in tree order), then the local expansion at the targets.
 // Threads = targets x source phases; sources staged in shared memory tiles.
-constexpr int NEAR_T = 128, NEAR_TILE = 128;
-__global__ void __launch_bounds__(NEAR_T) k_near64(const ChebTables *__restrict__ tab, KParams kp,
-                                                   const int4 *__restrict__ segs,
-                                                   const int *__restrict__ near_range, const int *__restrict__ tb_,
-                                                   const int *__restrict__ te_, const double *__restrict__ ctr,
-                                                   const double *__restrict__ rad, const double *__restrict__ sx,
-                                                   const double *__restrict__ sy, const double *__restrict__ sz,
-                                                   const double *__restrict__ dens, long ns,
-                                                   const double *__restrict__ tx, const double *__restrict__ ty,
-                                                   const double *__restrict__ tz, long nt,
-                                                   const double *__restrict__ local, double *out, int l2p_mask,
-                                                   int nseg, int *next) {
-    __shared__ ChebTables T;
-    __shared__ double S[7][NEAR_TILE];
-    __shared__ double red[NEAR_T][4];
+//
+// Bound by GB300's narrow FP64 pipe (2 lanes a cycle per SM: 16 cycles a warp instruction, whatever
+// else the SM does), so the count of FP64 instructions a pair is the kernel's time.  near64_pair
+// takes 51 (22 without screening) where the formulas as written took about 103: seeds, rounding
+// and comparisons on the integer and FP32 pipes, one cubic step for 1 / r, a 128-entry table and a
+// degree-5 polynomial for the exponential, and the constant factors applied once per target instead of
+// once per pair.  16 warps a SM keep the pipe busy; two CTAs of 11 KB leave the rest of the SM to
+// the tensor-core M2L that runs beside it.  On a 2,000-atom protein (5.2e8 pairs): 82 -> 49 ms alone
+// (51 instructions take 41 ms), 55 ms beside the M2L.
+constexpr int NEAR_T = 256, NEAR_TILE = 128, NEAR_CPS = 2;  // threads, sources a tile, CTAs a SM
+constexpr int NEAR_EXP = 128;                               // steps of 2^-x in the table
+enum { NEAR_GENERAL = 0, NEAR_YUKAWA = 1, NEAR_LAPLACE = 2 };
+
+struct Near64K {
+    double vr2, eps, ieps, kappa, kl;  // kl = kappa log2 e
+    double sk, k2c;                    // k3f / q4pi; k2in k3f / q4pi^2 (the cutoff's K2 in A0's units)
+    double psi_f, f0, fg;              // staged psi = psi psi_f; F = f0 A0, G = fg A
+    float klt;                         // kl NEAR_EXP
+    KParams kp;
+};
+
+Near64K make_near64(const KParams &k) {
+    Near64K n{};
+    n.kp = k;
+    n.vr2 = k.vr2;
+    n.eps = k.eps;
+    n.ieps = k.ieps;
+    n.kappa = k.kappa;
+    n.kl = k.kappa * 1.4426950408889634074;
+    n.sk = k.k3f / k.q4pi;
+    n.psi_f = k.q4pi / k.k3f;
+    n.k2c = k.k2in * (n.sk / k.q4pi);
+    n.f0 = k.q4pi;
+    n.fg = k.k3f;
+    n.klt = (float)(n.kl * NEAR_EXP);
+    return n;
+}
+
+// FP32 value of a positive double by its bits (truncated; 2^127 and above, 2^-126 and below clamp).
+__device__ __forceinline__ float near64_f32(double v) {
+    const int hi = min(max(__double2hiint(v), 0x38000000), 0x47dfffff);
+    return __int_as_float(((hi - 0x38000000) << 3) | ((unsigned)__double2loint(v) >> 29));
+}
+// The double equal to a non-negative normal float (0 becomes 2^-127).
+__device__ __forceinline__ double near64_f64(float v) {
+    const int b = __float_as_int(v);
+    return __hiloint2double((b >> 3) + 0x38000000, b << 29);
+}
+
+// One source -> target update of the fused block (kblock64's formulas) for d2 >= vr2, with
+// M = d.m / r^3 shared by K1 and K3, psi staged times q4pi / k3f, and the factors q4pi (F) and
+// k3f (G) left to the caller.  1 / r: FP32 seed y (relative error below 2^-22), then
+// y (1 + e/2 + 3 e^2/8) with e = 1 - d2 y^2, whose error is about 5/16 e^3 < 2^-64.
+// e^{-kappa r} = 2^{-n/128} 2^{-g}: n from FP32, g exact, |g| < 2^-7.8, Taylor to degree 5 (below 2^-58).
+template <int MODE>
+__device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__restrict__ e2, double dx, double dy,
+                                            double dz, double m0, double m1, double m2, double psi, double acc[4]) {
+    const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    // both non-negative: the order of the bits is the order of the values
+    if (__double_as_longlong(d2) < __double_as_longlong(k.vr2)) {
+        if (MODE == NEAR_YUKAWA) acc[0] = fma(-k.k2c, psi, acc[0]);
+        return;
+    }
+    const float d2f = near64_f32(d2);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(d2f));
+    const double y = near64_f64(yf);
+    const double e0 = fma(-(d2 * y), y, 1.0);
+    const double ir = fma(y, fma(e0, 0.375, 0.5) * e0, y);
+    const double ir2 = ir * ir, ir3 = ir2 * ir;
+    const double M = fma(dx, m0, fma(dy, m1, dz * m2)) * ir3;
+    const double w = ir3 * psi;
+    if (MODE == NEAR_LAPLACE) {  // e = 1: K2 = K3 = 0
+        acc[0] += M;
+        acc[1] = fma(dx, w, acc[1]);
+        acc[2] = fma(dy, w, acc[2]);
+        acc[3] = fma(dz, w, acc[3]);
+        return;
+    }
+    const double r = d2 * ir, t = k.kappa * r;
+    const float xm = fminf(d2f * yf * k.klt, 128000.f) + 12582912.f;  // n in the low bits
+    const int n = __float_as_int(xm) - 0x4b400000;
+    const double g = fma(k.kl, r, -near64_f64((xm - 12582912.f) * (1.f / NEAR_EXP)));
+    double q = fma(g, -1.3333558146428443e-3, 9.6181291076284772e-3);
+    q = fma(g, q, -5.5504108664821580e-2);
+    q = fma(g, q, 2.4022650695910072e-1);
+    q = fma(g, q, -6.9314718055994531e-1) * g;
+    const double2 tb = e2[n & (NEAR_EXP - 1)];
+    const double ef = tb.x + fma(tb.x, q, tb.y);
+    const double e = n >= 128000 ? 0.0
+                                 : __hiloint2double(__double2hiint(ef) - ((n / NEAR_EXP) << 20), __double2loint(ef));
+    const double et1 = fma(e, t, e);
+    acc[0] = fma(fma(k.eps, et1, -1.0), M, acc[0]);
+    acc[0] = fma(-(fma(-k.sk, e, k.sk) * ir), psi, acc[0]);
+    const double ho = fma(e, fma(t + 3.0, t, 3.0), -3.0);
+    const double cm = fma(-fma(-k.ieps, et1, 1.0), w, ho * (ir2 * M));
+    const double hd = (1.0 - et1) * ir3;
+    acc[1] = fma(dx, cm, fma(hd, m0, acc[1]));
+    acc[2] = fma(dy, cm, fma(hd, m1, acc[2]));
+    acc[3] = fma(dz, cm, fma(hd, m2, acc[3]));
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave the M2L its own
+    k_near64(const ChebTables *__restrict__ tab, const double2 *__restrict__ etab, Near64K kp, const int4 *__restrict__ segs,
+             const int *__restrict__ near_range, const int *__restrict__ tb_, const int *__restrict__ te_,
+             const double *__restrict__ ctr, const double *__restrict__ rad, const double *__restrict__ sx,
+             const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ dens, long ns,
+             const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz, long nt,
+             const double *__restrict__ local, double *out, int l2p_mask, int nseg, int *next) {
+    __shared__ double2 S[NEAR_TILE][4];  // x y | z m_x | m_y m_z | psi -
+    __shared__ double2 e2[MODE == NEAR_YUKAWA ? NEAR_EXP : 1];  // 2^(-j / 128), high and low word
     __shared__ int cur;
-    for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
-        reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
-    // with a work counter the CTA takes segments until none is left (several launches may drain
-    // the same counter); without one it does segment blockIdx.x
+    double(*red)[4] = reinterpret_cast<double(*)[4]>(S);  // [NEAR_T][4], once the tiles are done
+    static_assert(sizeof(S) >= sizeof(double) * 4 * NEAR_T, "reduction scratch");
+    if (MODE == NEAR_YUKAWA && threadIdx.x < NEAR_EXP) e2[threadIdx.x] = etab[threadIdx.x];
+    const double psi_f = MODE == NEAR_GENERAL ? 1.0 : kp.psi_f;
+    // with a work counter the CTA takes segments until none is left; without one it does segment blockIdx.x
     for (int it = 0;; ++it) {
         int si;
         if (next) {
@@ -365,22 +463,36 @@ __global__ void __launch_bounds__(NEAR_T) k_near64(const ChebTables *__restrict_
                 for (int s0 = b; s0 < e; s0 += NEAR_TILE) {
                     const int cnt = min(NEAR_TILE, e - s0);
                     __syncthreads();
-                    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-                        S[0][q] = sx[s0 + q];
-                        S[1][q] = sy[s0 + q];
-                        S[2][q] = sz[s0 + q];
-                        S[3][q] = dens[s0 + q];
-                        S[4][q] = dens[ns + s0 + q];
-                        S[5][q] = dens[2 * ns + s0 + q];
-                        S[6][q] = dens[3 * ns + s0 + q];
+                    // two threads a source
+                    const int q = threadIdx.x >> 1;
+                    if (q < cnt) {
+                        const long i = s0 + q;
+                        if (threadIdx.x & 1) {
+                            S[q][2] = make_double2(dens[ns + i], dens[2 * ns + i]);
+                            S[q][3] = make_double2(dens[3 * ns + i] * psi_f, 0.);
+                        } else {
+                            S[q][0] = make_double2(sx[i], sy[i]);
+                            S[q][1] = make_double2(sz[i], dens[i]);
+                        }
                     }
                     __syncthreads();
                     if (active)
-                        for (int q = ph; q < cnt; q += nph)
-                            near_pair64(kp, S[0][q] - X, S[1][q] - Y, S[2][q] - Z, S[3][q], S[4][q], S[5][q], S[6][q],
-                                        acc);
+                        for (int q2 = ph; q2 < cnt; q2 += nph) {
+                            const double2 a0 = S[q2][0], a1 = S[q2][1], a2 = S[q2][2];
+                            const double psi = S[q2][3].x;
+                            if (MODE == NEAR_GENERAL)
+                                near_pair64(kp.kp, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
+                            else
+                                near64_pair<MODE>(kp, e2, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
+                        }
                 }
             }
+            if (MODE != NEAR_GENERAL) {
+                // without screening the pairs carry c1 = eps - 1 and -c4 = 1/eps - 1 here
+                acc[0] *= MODE == NEAR_LAPLACE ? kp.f0 * (kp.eps - 1.0) : kp.f0;
+                for (int o = 1; o < 4; ++o) acc[o] *= MODE == NEAR_LAPLACE ? kp.fg * (kp.ieps - 1.0) : kp.fg;
+            }
+            __syncthreads();  // every thread is done with the last tile
             for (int o = 0; o < 4; ++o) red[threadIdx.x][o] = acc[o];
             __syncthreads();
             if (threadIdx.x < nT) {
@@ -390,6 +502,7 @@ __global__ void __launch_bounds__(NEAR_T) k_near64(const ChebTables *__restrict_
                 // L2P (bbfmm.h:600): local expansion at the target, by the leaf's first segment
                 double l2p[4] = {0., 0., 0., 0.};
                 if (mode & l2p_mask & 1) {
+                    const ChebTables &T = *tab;
                     double Sp[3][MAXP];
                     const double xyz[3] = {X, Y, Z};
                     for (int a = 0; a < 3; ++a) interp1(T, (xyz[a] - ctr[3 * leaf + a]) / rad[3 * leaf + a], Sp[a]);
@@ -413,7 +526,8 @@ __global__ void __launch_bounds__(NEAR_T) k_near64(const ChebTables *__restrict_
 
 // L2P alone (bbfmm.h:600), one target leaf per block, added to the near-field sums already in
 // `out`: the form used when the near field runs beside the far field.
-__global__ void __launch_bounds__(NEAR_T) k_l2p64(const ChebTables *__restrict__ tab, const int *__restrict__ tleaf,
+constexpr int L2P_T = 128;
+__global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ tab, const int *__restrict__ tleaf,
                                                   const int *__restrict__ tb_, const int *__restrict__ te_,
                                                   const double *__restrict__ ctr, const double *__restrict__ rad,
                                                   const double *__restrict__ tx, const double *__restrict__ ty,
@@ -421,7 +535,7 @@ __global__ void __launch_bounds__(NEAR_T) k_l2p64(const ChebTables *__restrict__
                                                   const double *__restrict__ local, double *out) {
     __shared__ ChebTables T;
     __shared__ double Ls[4 * MAXR];                // the leaf's local expansion
-    __shared__ double W[3][NEAR_T][MAXP + 1];      // per-thread interpolation weights (odd stride)
+    __shared__ double W[3][L2P_T][MAXP + 1];      // per-thread interpolation weights (odd stride)
     for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
         reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
     const int leaf = tleaf[blockIdx.x];
@@ -826,6 +940,12 @@ static void build_target_lists(Plan &P, TargetSet &S, OpIndex &opid) {
     cut(chunks_tc, M2L_CHTC);
     cut(chunks_tc2, 2 * M2L_CHTC);
     cut(chunks_oz, M2L_CHOZ);
+    if (P.oz64_ok) {
+        std::vector<int> chunks_oz64;
+        cut(chunks_oz64, M2L_CHOZ64);
+        S.nchunks_oz64 = (int)chunks_oz64.size() / 3;
+        up_int(S.v_chunk_oz64, chunks_oz64, s);
+    }
     trace_mark("lists: pairs grouped");
     S.nvpairs = npair;
     S.nchunks = (int)chunks.size() / 3;
@@ -962,6 +1082,7 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
     P->maxlevel = maxlevel;
     P->precision = precision;
     P->tune = tuning_for(order, ns);
+    P->oz64_ok = precision == IBIM_PRECISION_FP64 && m2l_oz64_fits(order, 0.);
     try {
         trace_mark("plan: coordinates downloaded");
         P->tree = build_tree(pts.data(), ns, pts.data(), ns, maxpoint, maxlevel);
@@ -1042,6 +1163,7 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
             trace_mark("plan: extra target lists");
         }
         P->nops = (int)opid.keys.size() / 5;
+        P->oz64_ok = P->oz64_ok && m2l_oz64_fits(order, P->nops);
         P->op_key_h = opid.keys;
         if (P->op_key_h.empty()) P->op_key_h.assign(5, 0);
         up_int(P->op_key, P->op_key_h, s);
@@ -1055,10 +1177,14 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
         P->local.alloc((size_t)nn * n4, s);
         P->dens4.alloc((size_t)4 * ns, s);
         const size_t smem_k = sizeof(double) * 3 * n4;
-        if (smem_k > 48 * 1024) {
+        if (smem_k + sizeof(ChebTables) > 48 * 1024) {  // the kernels' own tables count too (order 8)
             IBIM_CUDA(cudaFuncSetAttribute(k_m2m64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
             IBIM_CUDA(cudaFuncSetAttribute(k_l2l64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
         }
+        for (const void *k : {(const void *)k_near64<NEAR_GENERAL>, (const void *)k_near64<NEAR_YUKAWA>,
+                              (const void *)k_near64<NEAR_LAPLACE>, (const void *)k_p2m64, (const void *)k_m2m64,
+                              (const void *)k_l2l64, (const void *)k_l2p64})
+            side_by_side(k);
         const size_t sm = sizeof(double) * M2L_CH * n4;
         if (sm > 48 * 1024)
             IBIM_CUDA(cudaFuncSetAttribute(k_m2l_v64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1200,7 +1326,10 @@ void near64_lists(Plan &P, TargetSet &S) {
     }
     std::vector<int> ntk(tl.size()), seg;
     for (size_t k = 0; k < tl.size(); ++k) ntk[k] = (int)(S.end[tl[k]] - S.begin[tl[k]]);
-    S.near_atomic = near_segments(tl, ntk, nptr, nr, true, seg);
+    // at least eight segments a CTA of the launch (2^11 to 2^14 pairs): with 2^17 the last segments
+    // ran alone for most of a small plan's launch (60 atoms: 195 segments, 9.5 ms for 2.6e7 pairs)
+    const long cap = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (8L * NEAR_CPS * P.ctx->num_sms)));
+    S.near_atomic = near_segments(tl, ntk, nptr, nr, true, seg, cap, 32);
     S.nnear_seg = tl.empty() ? 0 : (int)seg.size() / 4;
     up_int(S.near_seg, seg, s);
     up_int(S.near_ptr, nptr, s);
@@ -1208,12 +1337,47 @@ void near64_lists(Plan &P, TargetSet &S) {
     S.near64_ready = true;
 }
 
+// The FP64 operator's digit images: the operators in blocks of at most 1 GB, each cut and dropped.
+bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp) {
+    if (!P.oz64_ok) return false;
+    double key[5];
+    kp_key(kp, key);
+    if (P.oz64.ready && same_key(P.oz64.key, key)) return true;
+    P.oz64.ready = false;
+    cudaStream_t s = P.ctx->stream;
+    const int R = P.R, n4 = 4 * R;
+    const KParams k = make_kparams(kp, P.tube->h);
+    const size_t per = (size_t)n4 * n4;
+    const int block = (int)std::max<size_t>(1, std::min<size_t>(std::max(1, P.nops), (1UL << 30) / (8 * per)));
+    m2l_oz64_alloc(P);
+    DevBuf<double> ops;
+    ops.alloc(per * block, s);
+    ProfScope ps_(PROF_OPS);
+    for (int o = 0; o < P.nops; o += block) {
+        const int nb = std::min(block, P.nops - o);
+        (count_launch(), k_make_ops64<<<dim3(div_up((long)R * R, 256), nb), 256, 0, s>>>(P.tables.ptr, P.op_key.ptr + 5 * o,
+                                                                                       P.root_r.ptr, k, ops.ptr));
+        IBIM_CHECK_LAUNCH();
+        m2l_oz64_pack(P, ops.ptr, o, nb);
+    }
+    for (int i = 0; i < 5; ++i) P.oz64.key[i] = key[i];
+    P.oz64.ready = true;
+    return true;
+}
+
+void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp) {
+    if (!fmm_ensure_oz64_images(P, kp)) fmm_prepare_operators(P, kp, IBIM_PRECISION_FP64);
+}
+
 // One FP64 FMM: dens (4 x ns, tree order) -> out (4 x nt of target set ts, tree order).
 void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *dens, double *out, bool m2l_sliced) {
     IBIM_REQUIRE(ts >= 0 && ts < (int)P.targets.size(), "no such target set");
     const bool use_oz = m2l_sliced && (4 * P.R + 15) / 16 * 16 <= M2L_OZ_MAXK;
+    const bool use_oz64 = !m2l_sliced && P.oz64_ok;
     if (use_oz)
         fmm_ensure_oz_images(P, kpp);
+    else if (use_oz64)
+        fmm_ensure_oz64_images(P, kpp);
     else
         fmm_prepare_operators(P, kpp, IBIM_PRECISION_FP64);
     const TargetSet &S = *P.targets[ts];
@@ -1249,18 +1413,31 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         }
         ProfScope ps_(PROF_NEAR64, count_work ? 70.0 * S.near_pairs : 0., count_work ? 56.0 * P.ns + 40.0 * S.nt : 0.,
                       st);
-        (count_launch(), k_near64<<<grid, NEAR_T, 0, st>>>(P.tables.ptr, kp, reinterpret_cast<const int4 *>(S.near_seg.ptr),
-                                                         S.near_range.ptr, S.tbeg.ptr, S.tend.ptr, P.ncenter.ptr,
-                                                         P.nradius.ptr, P.sx.ptr, P.sy.ptr, P.sz.ptr, dens, P.ns, tx,
-                                                         ty, tz, S.nt, P.local.ptr, out, l2p_mask, S.nnear_seg, next));
+        const Near64K nk = make_near64(kp);
+        // the fast forms take FP32 seeds of d2 >= (tau h)^2 and n >= 0 of 2^-n/128
+        const int mode = !(kp.vr2 >= 1e-30) ? NEAR_GENERAL
+                                            : (kp.kappa > 0. ? NEAR_YUKAWA : (kp.kappa == 0. ? NEAR_LAPLACE : NEAR_GENERAL));
+        auto kern = mode == NEAR_YUKAWA ? k_near64<NEAR_YUKAWA>
+                                        : (mode == NEAR_LAPLACE ? k_near64<NEAR_LAPLACE> : k_near64<NEAR_GENERAL>);
+        (count_launch(), kern<<<grid, NEAR_T, 0, st>>>(P.tables.ptr, P.exp_tab.ptr, nk, reinterpret_cast<const int4 *>(S.near_seg.ptr),
+                                                       S.near_range.ptr, S.tbeg.ptr, S.tend.ptr, P.ncenter.ptr,
+                                                       P.nradius.ptr, P.sx.ptr, P.sy.ptr, P.sz.ptr, dens, P.ns, tx, ty,
+                                                       tz, S.nt, P.local.ptr, out, l2p_mask, S.nnear_seg, next));
     };
     const bool overlap = near_overlap() && S.ntleaves > 0;
-    static const int occ64 = [] {
-        int b = 0;
-        IBIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_near64, NEAR_T, 0));
-        return std::max(1, b);
-    }();
-    const int full = (ff ? near_ff_occupancy() : occ64) * c->num_sms;
+    if (!P.exp_tab.ptr) {
+        // 2^(-j / 128) as high and low words, from the host's long double
+        std::vector<double2> h(NEAR_EXP);
+        for (int j = 0; j < NEAR_EXP; ++j) {
+            const long double v = std::exp2(-(long double)j / NEAR_EXP);
+            h[j].x = (double)v;
+            h[j].y = (double)(v - h[j].x);
+        }
+        P.exp_tab.alloc(NEAR_EXP, s);
+        P.exp_tab.upload(h.data(), NEAR_EXP);
+        IBIM_CUDA(cudaStreamSynchronize(s));
+    }
+    const int full = (ff ? near_ff_occupancy() : NEAR_CPS) * c->num_sms;
     const int side = near_side_ctas() > 0 ? near_side_ctas() * c->num_sms : full;
     if (overlap) {
         if (!P.near_next.ptr) P.near_next.alloc(1, s);
@@ -1289,6 +1466,8 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         P.local.zero();
         if (use_oz) {
             m2l_oz_run(P, S);
+        } else if (use_oz64) {
+            m2l_oz64_run(P, S);
         } else if (S.nchunks > 0) {
             ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
                           8.0 * n4 * (2.0 * S.nvpairs + (double)n4 * P.nops));
@@ -1323,7 +1502,7 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         }
         if (overlap || ff) {  // the L2P runs on its own after the near field
             ProfScope ps_(PROF_L2P64, (10.0 * R + 6.0 * P.p * P.p) * S.nt, 32.0 * n4 * S.ntleaves + 88.0 * S.nt);
-            (count_launch(), k_l2p64<<<S.ntleaves, NEAR_T, 0, s>>>(P.tables.ptr, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr,
+            (count_launch(), k_l2p64<<<S.ntleaves, L2P_T, 0, s>>>(P.tables.ptr, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr,
                                                                    P.ncenter.ptr, P.nradius.ptr, tx, ty, tz, S.nt,
                                                                    P.local.ptr, out));
         }

@@ -90,6 +90,12 @@ struct DevBuf {
     }
 };
 
+// Kernels that run beside each other on an SM ask for the same split of L1 and shared memory (all
+// shared): with the default each kernel picks its own, and an SM changes its split only when idle.
+inline void side_by_side(const void *kernel) {
+    IBIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+}
+
 // Host scratch array without value-initialisation, for large arrays that are written in full
 // (by several threads) before they are read: a std::vector's zero fill is one serial pass.
 template <class T> struct HostArr {
@@ -244,6 +250,8 @@ struct TargetSet {
     int nchunks_tc2 = 0;
     DevBuf<int> v_chunk_oz;            // chunks of the sliced FP64-class contraction (<= 64 pairs)
     int nchunks_oz = 0;
+    DevBuf<int> v_chunk_oz64;          // chunks of the FP64 operator's digit contraction (<= 64 pairs)
+    int nchunks_oz64 = 0;
     DevBuf<int> chunk_mol_tc, chunk_mol_oz;  // merged plans: the molecule of each chunk
     long nvpairs = 0;                  // pairs of the operator contraction (V, plus X when x_as_ops)
     DevBuf<int> x_src, x_tgt;          // X pairs evaluated on the fly (when not x_as_ops)
@@ -327,6 +335,7 @@ struct Plan {
     // tables and workspaces
     DevBuf<ChebTables> tables;
     DevBuf<double> root_r;
+    DevBuf<double2> exp_tab;  // the FP64 near field's table of powers of two, made on its first use
     DevBuf<double> mult, local, dens4;
     DevBuf<float> mult32, local32, dens32;
     DevBuf<float4> src8;           // near-field source records (mixed): {x, y, z, m_x}, {m_y, m_z, psi, 0}
@@ -354,6 +363,15 @@ struct Plan {
     int oz_kpad = 0, oz_mtiles = 0, oz_s = 7;  // digit images: K padded, row tiles, digits
     DevBuf<uint16_t> oz_a, oz_b;
     DevBuf<double> oz_sig, oz_tau;
+    // the FP64 operator's own digit images (m2l_oz64_run), on FP64 plans whose images fit (oz64_ok)
+    bool oz64_ok = false;
+    struct {
+        bool ready = false;
+        double key[5] = {-1, -1, -1, -1, -1};
+        int kpad = 0, mtiles = 0, s = 8;
+        DevBuf<uint16_t> a, b;
+        DevBuf<double> sig, tau;
+    } oz64;
     double kp64[5] = {-1, -1, -1, -1, -1}, kp32[5] = {-1, -1, -1, -1, -1};  // kernel parameters of the cached operators
     bool ops64_ready = false, ops32_ready = false;
     // a plan merged over several molecules (batch.cu): the molecule of every node and each
@@ -408,10 +426,22 @@ void m2l_pack_images_ff(Plan &P, const float2 *ff);
 // Test check: the one-pass images equal the separate passes' word for word (throws otherwise).
 void m2l_check_images_ff(Plan &P, const float2 *ff);
 void m2l_oz_run(Plan &P, const TargetSet &S);
+// The FP64 operator's M2L as digit products: bytes of one operator's images at order p (0: the order
+// has none), whether nops of them may be kept on this device, the buffers, the cut of operators
+// [o, o + n) from FP64 ones, one contraction.
+double m2l_oz64_op_bytes(int p);
+bool m2l_oz64_fits(int p, double nops);
+void m2l_oz64_alloc(Plan &P);
+void m2l_oz64_pack(Plan &P, const double *ops, int o, int n);
+void m2l_oz64_run(Plan &P, const TargetSet &S);
 // Operator images for kernel parameters kp, built when missing or stale: the TF32 images (from
 // FP32 operators, which are then released) and the digit images (from the FP64 operators).
 void fmm_ensure_tc_images(Plan &P, const ibim_kernel_params &kp);
 void fmm_ensure_oz_images(Plan &P, const ibim_kernel_params &kp);
+// The FP64 operator's digit images; false when the plan has none.
+bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp);
+// What an FP64 matvec needs: its digit images, or the FP64 operators.
+void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp);
 // The mixed path's FP16 images and the FP64-class digit images together, from one set of
 // float-float operators (scaled FP16 form, float-float operators enabled); false otherwise.
 bool fmm_ensure_images_ff(Plan &P, const ibim_kernel_params &kp);

@@ -19,6 +19,7 @@
 // epilogue reads the accumulators with tcgen05.ld (each warp its 32 TMEM lanes) and adds them
 // into the target nodes' local expansions.
 
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <type_traits>
@@ -1384,18 +1385,28 @@ __global__ void k_split_mult_h16(long nnodes, int n4, int kpad, const float *__r
 // one thread issues the bulk copies, one the MMAs, six warps gather; they meet on mbarriers only.
 // ---------------------------------------------------------------------------------------------
 
-constexpr int OZ_M = 128, OZ_N = 128, OZ_KS = 16, OZ_ACC = 4;
+constexpr int OZ_M = 128, OZ_KS = 16;
 constexpr int OZ_THREADS = 256, OZ_BPROD = 192;
 constexpr int OZ_ATILE = OZ_M * OZ_KS * 2;                 // 4 KB
-constexpr int OZ_BTILE = OZ_N * OZ_KS * 2;                 // 4 KB
-constexpr int OZ_K7 = 800;                                  // largest K for 7-bit digits (S = 6)
-static_assert(OZ_N * OZ_ACC <= 512, "TMEM columns");
+constexpr int OZ_K7 = 800;                                  // largest K for 7-bit digits with S = 6
 
+// S digits of D bits; N pairs a chunk and ACC accumulators (groups 0 .. ACC - 2 exact, the rest
+// shared).  S = 6, 7: the 42-bit cut of the refinement residual.  S = 8 (56 bits, orders <= 5) and
+// 9 (54 bits, orders 6 and 7): the FP64 operator itself (see m2l_oz64_run).
 template <int S> struct OzShape {
-    static constexpr int D = 42 / S;                        // bits per digit
-    static_assert(S * D == 42, "42-bit cut");
-    static constexpr int STAGE = S * (OZ_ATILE + OZ_BTILE);  // 48 KB (S 6), 56 KB (S 7)
-    static constexpr int NST = (200 * 1024) / STAGE;        // 4 or 3 stage buffers
+    static_assert(S >= 6 && S <= 9, "digit counts");
+    static constexpr int D = S % 2 == 0 ? 7 : 6;             // bits per digit
+    static constexpr int BITS = S * D;                      // 42, 42, 56, 54
+    static constexpr int N = S <= 7 ? 128 : 64;
+    static constexpr int ACC = S <= 7 ? 4 : (S == 8 ? 7 : 8);
+    static_assert(N * ACC <= 512, "TMEM columns");
+    static constexpr int F = 2 * D + 24;                    // fraction bits of the epilogue (S 6 and 7)
+    static constexpr int CW = S <= 7 ? 16 : 8;              // accumulator columns a read of the epilogue
+    static constexpr int BTILE = N * OZ_KS * 2;             // 4 KB (N 128), 2 KB (N 64)
+    static constexpr int STAGE = S * (OZ_ATILE + BTILE);    // 48, 56, 48, 54 KB
+    // stage buffers: 4 or 3; three for the FP64 operator, which leaves the near field's CTAs their
+    // shared memory beside it
+    static constexpr int NST = S <= 7 ? (200 * 1024) / STAGE : 3;
     static constexpr int LAG = 1;                           // copy lag (NST - 2: 14.49 against 14.24 ms)
     static constexpr int SMEM = NST * STAGE;
 };
@@ -1441,8 +1452,8 @@ __device__ __forceinline__ long long scaled_rint_bits(double v, int s) {
     return (u >> 63) ? -m : m;
 }
 
-// Balanced base-2^D digits of m = rint(x 2^42), |x| <= 1, stored scaled: dig[i] = a_i 2^(-D i)
-// with x = sum_i a_i 2^(-D(i+1)) up to 2^-43 (a_i in [-2^(D-1), 2^(D-1)) for i >= 1,
+// Balanced base-2^D digits of m = rint(x 2^(S D)), |x| <= 1, stored scaled: dig[i] = a_i 2^(-D i)
+// with x = sum_i a_i 2^(-D(i+1)) up to 2^-(S D + 1) (a_i in [-2^(D-1), 2^(D-1)) for i >= 1,
 // |a_0| <= 2^D).
 template <int S>
 __device__ __forceinline__ void oz_digits_of(long long m, uint16_t *dig) {
@@ -1461,7 +1472,7 @@ __device__ __forceinline__ void oz_digits_of(long long m, uint16_t *dig) {
 // power-of-two scale 2^e.
 template <int S>
 __device__ __forceinline__ void oz_digits(double v, int e, uint16_t *dig) {
-    oz_digits_of<S>(scaled_rint_bits(v, 42 - e), dig);
+    oz_digits_of<S>(scaled_rint_bits(v, OzShape<S>::BITS - e), dig);
 }
 
 // trunc(v 2^s) toward zero from the bits of a float, |v 2^s| < 2^62.
@@ -1484,6 +1495,7 @@ __device__ __forceinline__ long long scaled_trunc_bits_f32(float v, int s) {
 // by one unit of 2^-42, below the cut's own 2^-43).
 template <int S>
 __device__ __forceinline__ void oz_digits(float2 v, int e, uint16_t *dig) {
+    static_assert(OzShape<S>::BITS == 42, "float-float values carry 2^-44");
     const long long f = scaled_trunc_bits_f32(v.x, 58 - e) + scaled_trunc_bits_f32(v.y, 58 - e);
     oz_digits_of<S>((f + (1LL << 15)) >> 16, dig);
 }
@@ -1710,6 +1722,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
     using SH = OzShape<S>;
     constexpr int NST = SH::NST, LAG = SH::LAG, STAGE = SH::STAGE;
+    constexpr int OZ_N = SH::N, OZ_ACC = SH::ACC, OZ_BTILE = SH::BTILE;
     extern __shared__ __align__(1024) unsigned char oz_smem[];
     __shared__ __align__(8) uint64_t full_a[NST], full_b[NST], empty_bar[NST], acc_bar;
     __shared__ uint32_t tmem_base;
@@ -1774,7 +1787,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 if (!mbar_wait(smem_u32(&full_a[s2 % NST]), (uint32_t)((s2 / NST) & 1))) abort_s = 1;
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // MMA issue: S (S + 1) / 2 digit-pair MMAs per stage into 4 accumulators
+        if (lane == 0) {  // MMA issue: S (S + 1) / 2 digit-pair MMAs per stage into ACC accumulators
             int last = -1;
             for (int st = 0; st < nstage; ++st) {
                 const int buf = st % NST;
@@ -1850,41 +1863,55 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     if (!ok && tid == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (ok) {
-        // warp w: TMEM lanes 32 (w % 4) .. + 31 = rows, pair columns [64 (w / 4), + 64) below neff.
-        // Integer epilogue (the FP64 pipe is narrow): T = (G_0 2^(2D) + G_1 2^D + G_2) 2^F +
-        // rint(M 2^(2D+F)) in int64 with F = 24 (|G_0 2^(2D)| < 2^38, so |T| < 2^62; M kept to
-        // 2^-(2D+24) of a group-0 unit, far below the cut's own error), then the double nearest
-        // T 2^(e_r + e_j - 4D - F) is assembled from T's bits; s_r = 2^e_r and t_j = 2^e_j.
-        constexpr int D = SH::D;
+        // warp w: TMEM lanes 32 (w % 4) .. + 31 = rows, pair columns [N/2 (w / 4), + N/2) below neff.
+        // Integer epilogue (the FP64 pipe is narrow): T = sum_k G_k 2^(F - D k) + rint(M 2^F) in
+        // int64 (|T| < 2^62; M kept to 2^-F of a group-0 unit, below the cut's own error), then
+        // the double nearest T 2^(e_r + e_j - 2D - F) is assembled from T's bits; s_r = 2^e_r and
+        // t_j = 2^e_j, and sig holds s_r 2^(-2D).
+        constexpr int D = SH::D, F = SH::F, CW = SH::CW;
         const int lg = warp & 3, h = warp >> 2;
         const int row = t * OZ_M + 32 * lg + lane;
-        const int erow = row < n4 ? exp_of_pow2(sig[(long)op * mtiles * OZ_M + row]) + 2 * D : 0;
+        const int erow = row < n4 ? exp_of_pow2(sig[(long)op * mtiles * OZ_M + row]) : 0;
 #pragma unroll 1
-        for (int c0 = 64 * h; c0 < min(64 * h + 64, neff); c0 += 16) {
-            uint32_t v[OZ_ACC][16];
+        for (int c0 = OZ_N / 2 * h; c0 < min(OZ_N / 2 * (h + 1), neff); c0 += CW) {
+            uint32_t v[OZ_ACC][CW];
 #pragma unroll
-            for (int g = 0; g < OZ_ACC; ++g)
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                    "%13, %14, %15}, [%16];"
-                    : "=r"(v[g][0]), "=r"(v[g][1]), "=r"(v[g][2]), "=r"(v[g][3]), "=r"(v[g][4]), "=r"(v[g][5]),
-                      "=r"(v[g][6]), "=r"(v[g][7]), "=r"(v[g][8]), "=r"(v[g][9]), "=r"(v[g][10]), "=r"(v[g][11]),
-                      "=r"(v[g][12]), "=r"(v[g][13]), "=r"(v[g][14]), "=r"(v[g][15])
-                    : "r"(tmem_d + ((uint32_t)(32 * lg) << 16) + (uint32_t)(g * OZ_N + c0)));
+            for (int g = 0; g < OZ_ACC; ++g) {
+                const uint32_t ta = tmem_d + ((uint32_t)(32 * lg) << 16) + (uint32_t)(g * OZ_N + c0);
+                if constexpr (CW == 16)
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                        "%12, %13, %14, %15}, [%16];"
+                        : "=r"(v[g][0]), "=r"(v[g][1]), "=r"(v[g][2]), "=r"(v[g][3]), "=r"(v[g][4]), "=r"(v[g][5]),
+                          "=r"(v[g][6]), "=r"(v[g][7]), "=r"(v[g][8]), "=r"(v[g][9]), "=r"(v[g][10]), "=r"(v[g][11]),
+                          "=r"(v[g][12]), "=r"(v[g][13]), "=r"(v[g][14]), "=r"(v[g][15])
+                        : "r"(ta));
+                else
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                        : "=r"(v[g][0]), "=r"(v[g][1]), "=r"(v[g][2]), "=r"(v[g][3]), "=r"(v[g][4]), "=r"(v[g][5]),
+                          "=r"(v[g][6]), "=r"(v[g][7])
+                        : "r"(ta));
+            }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (row < n4) {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
+                for (int q = 0; q < CW; ++q) {
                     const int tg = tgt_s[c0 + q];
-                    constexpr int F = 24;
-                    const long long g0 = __float2int_rn(__uint_as_float(v[0][q]));
-                    const long long g1 = __float2int_rn(__uint_as_float(v[1][q]) * (float)(1 << D));
-                    const long long g2 = __float2int_rn(__uint_as_float(v[2][q]) * (float)(1 << (2 * D)));
-                    const long long T = (((g0 << (2 * D)) + (g1 << D) + g2) << F) +
-                                        f32_fixed(__uint_as_float(v[3][q]), 2 * D + F);
+                    constexpr int F0 = D * (OZ_ACC - 2);  // the exact groups' own fraction bits
+                    long long T = 0;
+#pragma unroll
+                    for (int g = 0; g < OZ_ACC - 1; ++g)  // exact integers below 2^24
+                        T += (long long)__float2int_rn(__uint_as_float(v[g][q]) *
+                                                       __int_as_float((127 + D * g) << 23))
+                             << (F0 - D * g);
+                    // the shared accumulator on F bits, or for the FP64 operator on as many as the
+                    // exact sum leaves below bit 62 (entries far below their row's maximum keep theirs)
+                    int sh = F - F0;
+                    if (S > 7) sh = min(26, max(1, __clzll(T < 0 ? -T : T) - 2));
+                    T = (T << sh) + f32_fixed(__uint_as_float(v[OZ_ACC - 1][q]), F0 + sh);
                     if (tg >= 0 && T != 0)
-                        atomicAdd(local + (long)tg * n4 + row,
-                                  pow2_scaled_ll(T, erow + tau_e[c0 + q] - 4 * D - F));
+                        atomicAdd(local + (long)tg * n4 + row, pow2_scaled_ll(T, erow + tau_e[c0 + q] - F0 - sh));
                 }
             }
         }
@@ -2235,6 +2262,102 @@ void m2l_oz_run(Plan &P, const TargetSet &S) {
                                                             P.oz_tau.ptr, P.local.ptr, P.tc_err.ptr, S.chunk_mol_oz.ptr,
                                                             P.mol_active.ptr, P.mol_img.ptr));
     }
+    IBIM_CHECK_LAUNCH();
+}
+
+// ---------------------------------------------------------------------------------------------
+// M2L of the FP64 operator (IBIM_PRECISION_FP64) as digit products.  GB300 does 1.25 TFLOP/s on the
+// FP64 pipe and 1.9 PFLOP/s of BF16 MMAs, so the 36 (45) digit pairs of a 56-bit (54-bit) cut cost a
+// fifteenth of the FP64 contraction: 744 -> 38 ms a product on a 2,000-atom protein (1.70 M pairs,
+// order 5), 54 ms beside the near field, which has the FP64 pipe to itself.  It is no less exact: with K = 4p^3 terms the FP64 chain of K multiply-adds leaves about
+// sqrt(K / 2) 2^-53 of its partial sums, the cut 2^-57 (2^-55) of row and column maximum per term,
+// groups 0 .. 5 (0 .. 6) exact in FP32 (|G_k| <= K 2^(2D) (1 + (k - 1) / 4) <= 2^24 for K = 500,
+// D = 7 and K = 1372, D = 6) and the last two, 2^-42 below, sharing one accumulator.
+// Seven (eight) accumulators leave 64 pairs a chunk in the 512 TMEM columns.  Orders up to 7; order
+// 8 (K = 2048, exact groups only up to 5) and plans whose images would take over a third of the
+// device's memory keep k_m2l_v64.
+// ---------------------------------------------------------------------------------------------
+static int oz64_digits(int p) { return p <= 5 ? 8 : 9; }
+
+double m2l_oz64_op_bytes(int p) {
+    if (p > 7) return 0.;
+    const int n4 = 4 * p * p * p;
+    const double kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS, mpad = (n4 + OZ_M - 1) / OZ_M * OZ_M;
+    return 2.0 * oz64_digits(p) * kpad * mpad;
+}
+
+bool m2l_oz64_fits(int p, double nops) {
+    if (p > 7 || !m2l_tc_supported()) return false;
+    if (nops <= 0.) return true;
+    static std::atomic<size_t> total[64];  // each device's memory, asked for once
+    int dev = 0;
+    IBIM_CUDA(cudaGetDevice(&dev));
+    size_t t = dev < 64 ? total[dev].load() : 0;
+    if (t == 0) {
+        size_t free_b = 0;
+        IBIM_CUDA(cudaMemGetInfo(&free_b, &t));
+        if (dev < 64) total[dev].store(t);
+    }
+    return m2l_oz64_op_bytes(p) * nops <= t / 3.0;
+}
+
+void m2l_oz64_alloc(Plan &P) {
+    cudaStream_t s = P.ctx->stream;
+    auto &Z = P.oz64;
+    const int n4 = 4 * P.R;
+    Z.kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS;
+    Z.mtiles = (n4 + OZ_M - 1) / OZ_M;
+    Z.s = oz64_digits(P.p);
+    const size_t stages = Z.kpad / OZ_KS, rows = (size_t)P.nops * Z.mtiles;
+    if (Z.a.n != rows * stages * Z.s * (OZ_ATILE / 2)) {
+        Z.a.alloc(rows * stages * Z.s * (OZ_ATILE / 2), s);
+        Z.sig.alloc(rows * OZ_M, s);
+        Z.b.alloc((size_t)P.tree.nnodes * stages * Z.s * OZ_KS, s);
+        Z.tau.alloc((size_t)P.tree.nnodes, s);
+    }
+    if (!P.tc_err.ptr) {
+        P.tc_err.alloc(1, s);
+        P.tc_err.zero();
+    }
+    IBIM_CUDA(cudaFuncSetAttribute(k_m2l_oz<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzShape<8>::SMEM));
+    IBIM_CUDA(cudaFuncSetAttribute(k_m2l_oz<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzShape<9>::SMEM));
+    for (const void *k : {(const void *)k_m2l_oz<8>, (const void *)k_m2l_oz<9>, (const void *)k_split_mult_oz<8>,
+                          (const void *)k_split_mult_oz<9>})
+        side_by_side(k);
+}
+
+void m2l_oz64_pack(Plan &P, const double *ops, int o, int n) {
+    cudaStream_t s = P.ctx->stream;
+    auto &Z = P.oz64;
+    const int n4 = 4 * P.R, D = Z.s == 8 ? OzShape<8>::D : OzShape<9>::D;
+    const long rows = (long)n * Z.mtiles * OZ_M;
+    DevBuf<int> sexp;
+    sexp.alloc((size_t)rows, s);
+    const int gs = (int)std::min<long>((rows + 255) / 256, 32L * P.ctx->num_sms);
+    const int gp = (int)std::min<long>((rows * (Z.kpad / 8) + 255) / 256, 64L * P.ctx->num_sms);
+    const size_t row0 = (size_t)o * Z.mtiles;
+    (count_launch(), k_scale_ops_oz<double><<<gs, 256, 0, s>>>(n4, Z.mtiles, n, 2 * D, ops, Z.sig.ptr + row0 * OZ_M,
+                                                               sexp.ptr));
+    uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr + row0 * (Z.kpad / OZ_KS) * Z.s * (OZ_ATILE / 2));
+    auto kern = Z.s == 8 ? k_pack_ops_oz<8, double> : k_pack_ops_oz<9, double>;
+    (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr));
+    IBIM_CHECK_LAUNCH();
+}
+
+void m2l_oz64_run(Plan &P, const TargetSet &S) {
+    if (S.nchunks_oz64 == 0) return;
+    cudaStream_t s = P.ctx->stream;
+    auto &Z = P.oz64;
+    const int n4 = 4 * P.R;
+    ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
+                  2.0 * Z.s * Z.kpad * ((double)Z.mtiles * OZ_M * P.nops + (double)S.nvpairs));
+    auto split = Z.s == 8 ? k_split_mult_oz<8> : k_split_mult_oz<9>;
+    (count_launch(), split<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, Z.kpad, P.mult.ptr, Z.b.ptr, Z.tau.ptr));
+    auto kern = Z.s == 8 ? k_m2l_oz<8> : k_m2l_oz<9>;
+    const int smem = Z.s == 8 ? OzShape<8>::SMEM : OzShape<9>::SMEM;
+    (count_launch(), kern<<<dim3(S.nchunks_oz64, Z.mtiles), OZ_THREADS, smem, s>>>(
+        n4, Z.kpad, Z.mtiles, S.v_chunk_oz64.ptr, S.v_src.ptr, S.v_tgt.ptr, Z.a.ptr, Z.sig.ptr, Z.b.ptr, Z.tau.ptr,
+        P.local.ptr, P.tc_err.ptr, nullptr, nullptr, nullptr));
     IBIM_CHECK_LAUNCH();
 }
 

@@ -81,22 +81,24 @@ double estimate_levelset_bytes(const ibim_config &cfg) {
 // points and 624,673 for 16.5 M at leaf 128), operators ~600 per tree level (2,239 for the
 // 2,000-atom protein at 5 levels, 4,290 for 20,000 atoms at 7), each at the peak of its images
 // (mixed: FP16 hi / lo tiles, BF16 digit tiles and the float-float operators they are cut from;
-// FP64: the FP64 operator), per node the expansions and multipole images, per point ~1.1 KB plus
+// FP64: its digit tiles, cut from blocks of FP64 operators, or those operators), per node the expansions and multipole images, per point ~1.1 KB plus
 // the Krylov basis.
 static double fmm_bytes(const ibim_config &cfg, double N, double nodes, double ops) {
     const double n4 = 4.0 * cfg.np * cfg.np * cfg.np;
     const double kpad = std::ceil(n4 / 16.0) * 16.0, mpad = std::ceil(n4 / 128.0) * 128.0;
     const double digits = kpad <= 800 ? 6.0 : 7.0;
-    double per_op, per_node;
+    double per_op, per_node, scratch = 0.0;
     if (cfg.precision == IBIM_PRECISION_FP64) {
-        per_op = n4 * n4 * 8.0;
-        per_node = n4 * 16.0;
+        const bool cut = m2l_oz64_fits(cfg.np, ops);
+        per_op = cut ? m2l_oz64_op_bytes(cfg.np) : n4 * n4 * 8.0;
+        per_node = n4 * 16.0 + (cut ? 20.0 * kpad : 0.0);
+        scratch = cut ? std::min(ops * n4 * n4 * 8.0, 1.1e9) : 0.0;
     } else {
         per_op = 2.0 * mpad * kpad * 2.0 + digits * mpad * kpad * 2.0 + n4 * n4 * 8.0;
         per_node = n4 * 24.0 + kpad * 4.0 + digits * kpad * 2.0;
     }
     const double per_point = 1100.0 + 16.0 * (std::min(cfg.restart, 250) + 1);
-    return ops * per_op + nodes * per_node + N * per_point;
+    return ops * per_op + nodes * per_node + N * per_point + scratch;
 }
 
 double estimate_fmm_bytes(const ibim_config &cfg, long npoints) {
