@@ -115,18 +115,72 @@ __global__ void k_expand(typename OrdT<T>::type *g, Dims d, double sx, double sy
     }
 }
 
-// Divisions of the WENO5 and RK3 formulas.  FP64 (the reference path) keeps IEEE divisions as
-// written in levelset.cpp; FP32 (mixed path) multiplies by reciprocal constants and uses the fast
-// hardware reciprocal (about 1 ulp), which the FP32 tolerance absorbs.
+// Reciprocal and square root of the FP64 stencils.  A WENO stage as levelset.cpp writes it has 45
+// FP64 divisions a cell, each a dozen instructions of GB300's narrow FP64 pipe, which is what bounds
+// the stage; these take 3 to 6 from an FP32 seed made of the operand's own bits (the exponent is
+// handled apart, so any normal operand will do) and one cubic step, to about an ulp.
+
+// 1 / x for normal x > 0: seed y within 2^-23, e = 1 - x y, y (1 + e + e^2).
+__device__ __forceinline__ double rcp64(double x) {
+    const int hi = __double2hiint(x);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;"
+        : "=f"(y)
+        : "f"(__int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | ((unsigned)__double2loint(x) >> 29))));
+    const int yb = __float_as_int(y);
+    const double d = __hiloint2double((yb >> 3) + 0x38000000 - ((hi & 0x7ff00000) - 0x3ff00000), yb << 29);
+    const double e = fma(-x, d, 1.0);
+    return fma(d, fma(e, e, e), d);
+}
+// 1 / sqrt(x) for normal x > 0: seed of x 2^(-2k) in [1, 4), y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2.
+__device__ __forceinline__ double rsqrt64n(double x) {
+    const int hi = __double2hiint(x), E = (hi >> 20) - 1023;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;"
+        : "=f"(y)
+        : "f"(__int_as_float(((127 + (E & 1)) << 23) | ((hi & 0xfffff) << 3) | ((unsigned)__double2loint(x) >> 29))));
+    const int yb = __float_as_int(y);
+    const double d = __hiloint2double((yb >> 3) + 0x38000000 - ((E >> 1) << 20), yb << 29);
+    const double e = fma(-(x * d), d, 1.0);
+    return fma(d * e, fma(e, 0.375, 0.5), d);
+}
+__device__ __forceinline__ bool is_normal_pos(double x) {
+    return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;
+}
+
+// Divisions and square roots of the stages.  FP64: the forms above.  FP32 (mixed path): reciprocal
+// constants and the fast hardware reciprocal (about 1 ulp), which the FP32 tolerance absorbs.
 struct Div64 {
     __device__ static double q(double x, double c) { return x / c; }
     __device__ static double rcp(double x) { return 1.0 / x; }
-    __device__ static double over_sqrt(double x, double y) { return x / sqrt(y); }
+    __device__ static double third(double x) {  // the residual's correction makes an infinity a NaN
+        const double r = x * (1.0 / 3.0);
+        return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000 ? r : fma(fma(-3.0, r, x), 1.0 / 3.0, r);
+    }
+    __device__ static double over_sqrt(double x, double y) { return is_normal_pos(y) ? x * rsqrt64n(y) : x / sqrt(y); }
+    __device__ static double root(double v) {
+        if (!is_normal_pos(v)) return sqrt(v);
+        const double y = rsqrt64n(v), r = v * y;
+        return fma(fma(-r, r, v), 0.5 * y, r);
+    }
+    // max(x, 0) and max(-x, 0), 0 for NaN, and the larger of two such values: on the integer pipe
+    __device__ static double pos(double x) {
+        return (unsigned long long)__double_as_longlong(x) <= 0x7ff0000000000000ULL ? x : 0.0;
+    }
+    __device__ static double neg(double x) { return pos(-x); }
+    __device__ static double larger(double a, double b) {
+        return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+    }
 };
 struct Div32 {
     __device__ static float q(float x, float c) { return x * __fdividef(1.0f, c); }
     __device__ static float rcp(float x) { return __fdividef(1.0f, x); }
+    __device__ static float third(float x) { return q(x, 3.0f); }
     __device__ static float over_sqrt(float x, float y) { return x * rsqrtf(y); }
+    __device__ static float root(float v) { return sqrt(v); }
+    __device__ static float pos(float x) { return x > 0.f ? x : 0.f; }
+    __device__ static float neg(float x) { return x < 0.f ? -x : 0.f; }
+    __device__ static float larger(float a, float b) { return fmax(a, b); }
 };
 template <class T> struct DivOf;
 template <> struct DivOf<double> { using type = Div64; };
@@ -164,6 +218,56 @@ __device__ __forceinline__ void weno5(const T w[7], T h, T &up, T &un) {
     un = D::q(df - D::q(w0 * (a - 2 * b + c), (T)3.0) - D::q((w2 - (T)0.5) * (b - 2 * c + d), (T)6.0), h);
 }
 
+// The FP64 form, with one reciprocal a side.  With q_k = (eps + s_k)^2 the weights' common factor
+// q_0 q_1 q_2 leaves w_0 = q_1 q_2 / S and w_2 = 3 q_0 q_1 / S, S = q_1 q_2 + 6 q_0 q_2 + 3 q_0 q_1, and
+//   12 h up = -b + 7 (c + d) - e - B + (4 q_1 q_2 A + 6 q_0 q_1 B) / S    (a .. f first differences,
+// A and B the second differences of the second differences), un its mirror image.  The indicators carry
+// 1/3 (13/3 x^2 + y^2; the weights do not change when every q does by the same factor) and
+// share their squares between the sides.  266 FP64 instructions a cell and stage instead of about 1070:
+// 2.0 -> 0.60 ms a stage on a 105^3 grid, the FP64 pipe 84 % busy.
+// S holds eighth powers of differences: beyond 2^60 (and for infinities and NaN) the cell takes the
+// formulas as written.
+__device__ __noinline__ double2 weno5_wide(double w0, double w1, double w2, double w3, double w4, double w5, double w6,
+                                           double h) {
+    const double w[7] = {w0, w1, w2, w3, w4, w5, w6};
+    double2 r;
+    weno5<double>(w, h, r.x, r.y);
+    return r;
+}
+__device__ __forceinline__ void weno5(const double w[7], double h, double &up, double &un) {
+    const double EPS = 1e-6 / 3.0, K = 13.0 / 3.0;
+    const double b1 = w[2] - w[1], c1 = w[3] - w[2], d1 = w[4] - w[3], e1 = w[5] - w[4];
+    const double a = b1 - (w[1] - w[0]), b = c1 - b1, c = d1 - c1, d = e1 - d1, e = (w[6] - w[5]) - e1;
+    const double D = fma(7.0, c1 + d1, -(b1 + e1));
+    const int big = max(max(max(__double2hiint(a) & 0x7fffffff, __double2hiint(b) & 0x7fffffff),
+                            max(__double2hiint(c) & 0x7fffffff, __double2hiint(d) & 0x7fffffff)),
+                        __double2hiint(e) & 0x7fffffff);
+    if (big >= (1023 + 60) << 20) {
+        const double2 r = weno5_wide(w[0], w[1], w[2], w[3], w[4], w[5], w[6], h);
+        up = r.x;
+        un = r.y;
+        return;
+    }
+    const double xed = e - d, xdc = d - c, xcb = c - b, xba = b - a;
+    const double ped = fma(K * xed, xed, EPS), pdc = fma(K * xdc, xdc, EPS), pcb = fma(K * xcb, xcb, EPS),
+                 pba = fma(K * xba, xba, EPS);
+    const double ih = rcp64(h) * (1.0 / 12.0);
+    const double B2 = xdc - xcb;
+    auto side = [](double p0, double y0, double p1, double y1, double p2, double y2, double A_, double B_) {
+        double q0 = fma(y0, y0, p0), q1 = fma(y1, y1, p1), q2 = fma(y2, y2, p2);
+        q0 *= q0;
+        q1 *= q1;
+        q2 *= q2;
+        const double n0 = q1 * q2, n2 = q0 * q1;
+        const double S = fma(6.0, q0 * q2, fma(3.0, n2, n0));
+        return fma(n0, A_, 1.5 * n2 * B_) * rcp64(S);  // (4 n0 A + 6 n2 B) / (4 S)
+    };
+    const double ru = side(ped, fma(-2.0, d, xed), pdc, d + c, pcb, fma(2.0, c, xcb), xed - xdc, B2);
+    const double rn = side(pba, fma(2.0, b, xba), pcb, b + c, pdc, fma(2.0, c, -xdc), xcb - xba, B2);
+    up = fma(4.0, ru, D - B2) * ih;
+    un = fma(-4.0, rn, D + B2) * ih;
+}
+
 template <class T>
 __device__ __forceinline__ void gradients(const T *__restrict__ g, const Dims &dm, int i, int j, int k, T h, T up[3],
                                           T un[3]) {
@@ -182,13 +286,14 @@ __device__ __forceinline__ void gradients(const T *__restrict__ g, const Dims &d
 // levelset::getNorm(Dun, Dup) (levelset.cpp:294-301).
 template <class T>
 __device__ __forceinline__ T godunov(const T n[3], const T p[3]) {
+    using D = typename DivOf<T>::type;
     T v = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const T m = fmax(n[a] > (T)0 ? n[a] : (T)0, p[a] < (T)0 ? -p[a] : (T)0);
+        const T m = D::larger(D::pos(n[a]), D::neg(p[a]));
         v += m * m;
     }
-    return sqrt(v);
+    return D::root(v);
 }
 
 // One TVD-RK3 stage over the whole grid.  MODE 0: evolve (phi_t + vel|grad phi| = 0);
@@ -202,10 +307,29 @@ __global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, 
                                                     T *u2, const T *__restrict__ phi0, T band = (T)0,
                                                     T thres = (T)0, unsigned long long *counts = nullptr,
                                                     double *accum = nullptr) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z * blockDim.z + threadIdx.z;
-    const bool in = i < dm.nx && j < dm.ny && k < dm.nz;
+    int i, j, k;
+    bool in;
+    if constexpr (sizeof(T) == 8) {
+        // consecutive cells to consecutive threads: the FP64 pipe takes as long for a warp at a
+        // row's end with few cells as for a full one (a fifth of the warps of a 105^3 grid)
+        const long I = blockIdx.x * 256L + threadIdx.x;
+        in = I < (long)dm.nx * dm.ny * dm.nz;
+        if (I < (1L << 32)) {
+            const unsigned row = (unsigned)I / (unsigned)dm.nz;
+            k = (int)((unsigned)I - row * (unsigned)dm.nz);
+            i = (int)(row / (unsigned)dm.ny);
+            j = (int)(row - (unsigned)i * (unsigned)dm.ny);
+        } else {
+            k = (int)(I % dm.nz);
+            j = (int)(I / dm.nz % dm.ny);
+            i = (int)(I / dm.nz / dm.ny);
+        }
+    } else {
+        k = blockIdx.x * blockDim.x + threadIdx.x;
+        j = blockIdx.y * blockDim.y + threadIdx.y;
+        i = blockIdx.z * blockDim.z + threadIdx.z;
+        in = i < dm.nx && j < dm.ny && k < dm.nz;
+    }
     if (!COUNT && !in) return;
     unsigned bad = 0, tot = 0;
     double acc = 0.;
@@ -234,7 +358,7 @@ __global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, 
         else if (STAGE == 1)
             u2[I] = (3 * g[I] + u1[I] - L) * (T)0.25;
         else
-            g[I] = D::q(g[I] + 2 * (u2[I] - L), (T)3.0);
+            g[I] = D::third(g[I] + 2 * (u2[I] - L));
     }
     if (COUNT) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -645,6 +769,12 @@ inline dim3 stencil_grid(const Grid &g) {
     dim3 b = stencil_block();
     return dim3(div_up(g.nz, b.x), div_up(g.ny, b.y), div_up(g.nx, b.z));
 }
+// Launch shape of k_weno_stage<T> over nx x ny x nz cells.
+template <class T> inline void stage_shape(int nx, int ny, int nz, dim3 &gr, dim3 &bl) {
+    bl = sizeof(T) == 8 ? dim3(256) : stencil_block();
+    gr = sizeof(T) == 8 ? dim3((unsigned)(((long)nx * ny * nz + 255) / 256))
+                        : dim3(div_up(nz, bl.x), div_up(ny, bl.y), div_up(nx, bl.z));
+}
 inline Dims dims_of(const Grid &g) { return Dims{g.nx, g.ny, g.nz}; }
 
 template <class T> T *gdata(Grid &g);
@@ -680,7 +810,8 @@ void evolve_t(Grid &g, double final_t, double vel, double cfl) {
     u1.alloc(g.cells(), s);
     u2.alloc(g.cells(), s);
     const Dims dm = dims_of(g);
-    const dim3 gr = stencil_grid(g), bl = stencil_block();
+    dim3 gr, bl;
+    stage_shape<T>(g.nx, g.ny, g.nz, gr, bl);
     const T dtv = (T)(dt * vel), h = (T)g.dx;
     T *G = gdata<T>(g);
     const double fl = 350.0 * g.cells(), by = 3.0 * sizeof(T) * g.cells();
@@ -716,7 +847,8 @@ int reinit_t(Grid &g, const Grid &phi0, double final_t, double vel, double cfl, 
     unsigned long long *hcnt = nullptr;
     IBIM_CUDA(cudaMallocHost((void **)&hcnt, 2 * sizeof(unsigned long long)));
     const Dims dm = dims_of(g);
-    const dim3 gr = stencil_grid(g), bl = stencil_block();
+    dim3 gr, bl;
+    stage_shape<T>(g.nx, g.ny, g.nz, gr, bl);
     const T dtv = (T)(dt * vel), h = (T)g.dx;
     T *G = gdata<T>(g);
     const T *P0 = gdata<T>(phi0);
@@ -1040,7 +1172,8 @@ extern "C" int ibim_levelset_evolve_static(double *grid_dev, int nx, int ny, int
     const int steps = (int)(final_t / dt) + 1;
     dt = final_t / (double)steps;
     const Dims dm{nx, ny, nz};
-    const dim3 bl = stencil_block(), gr(div_up(nz, bl.x), div_up(ny, bl.y), div_up(nx, bl.z));
+    dim3 gr, bl;
+    stage_shape<double>(nx, ny, nz, gr, bl);
     const double dtv = dt * vel;
     for (int st = 0; st < steps; ++st) {
         (count_launch(), k_weno_stage<0, 0, double><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., grid_dev, grid_dev, u1, u2, nullptr));
