@@ -920,13 +920,21 @@ static void build_target_lists(Plan &P, TargetSet &S, OpIndex &opid) {
     // chunks (operator, first pair, count) of each contraction's width, in operator order:
     // counts per operator, offsets, then the operators in parallel
     std::vector<int> chunks, chunks32, chunks_tc, chunks_tc2, chunks_oz;
-    auto cut = [&](std::vector<int> &out, int width) {
+    // `even`: an operator's chunks of like size, multiples of 16, instead of full ones and a rest
+    auto cut = [&](std::vector<int> &out, int max_width, bool even = false) {
+        auto width_of = [&](int op) {
+            const long n = opbeg[op + 1] - opbeg[op], c = (n + max_width - 1) / max_width;
+            return even && c > 0 ? std::min<long>(max_width, ((n + c - 1) / c + 15) / 16 * 16) : (long)max_width;
+        };
         std::vector<long> coff(nop + 1, 0);
-        for (int op = 0; op < nop; ++op) coff[op + 1] = coff[op] + (opbeg[op + 1] - opbeg[op] + width - 1) / width;
+        for (int op = 0; op < nop; ++op) {
+            const long w = width_of(op);
+            coff[op + 1] = coff[op] + (opbeg[op + 1] - opbeg[op] + w - 1) / w;
+        }
         out.resize(3 * coff[nop]);
 #pragma omp parallel for schedule(static) if (nop >= 256)
         for (int op = 0; op < nop; ++op) {
-            const long b = opbeg[op], n = opbeg[op + 1] - opbeg[op];
+            const long b = opbeg[op], n = opbeg[op + 1] - opbeg[op], width = width_of(op);
             long c = coff[op];
             for (long q = 0; q < n; q += width, ++c) {
                 out[3 * c] = op;
@@ -938,7 +946,7 @@ static void build_target_lists(Plan &P, TargetSet &S, OpIndex &opid) {
     cut(chunks, M2L_CH);
     cut(chunks32, M2L_CH32);
     cut(chunks_tc, M2L_CHTC);
-    cut(chunks_tc2, 2 * M2L_CHTC);
+    cut(chunks_tc2, 2 * M2L_CHTC, true);
     cut(chunks_oz, M2L_CHOZ);
     if (P.oz64_ok) {
         std::vector<int> chunks_oz64;
@@ -1181,10 +1189,10 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
             IBIM_CUDA(cudaFuncSetAttribute(k_m2m64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
             IBIM_CUDA(cudaFuncSetAttribute(k_l2l64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
         }
-        for (const void *k : {(const void *)k_near64<NEAR_GENERAL>, (const void *)k_near64<NEAR_YUKAWA>,
-                              (const void *)k_near64<NEAR_LAPLACE>, (const void *)k_p2m64, (const void *)k_m2m64,
-                              (const void *)k_l2l64, (const void *)k_l2p64})
-            side_by_side(k);
+        static std::atomic<uint64_t> split;
+        side_by_side(split, {(const void *)k_near64<NEAR_GENERAL>, (const void *)k_near64<NEAR_YUKAWA>,
+                             (const void *)k_near64<NEAR_LAPLACE>, (const void *)k_p2m64, (const void *)k_m2m64,
+                             (const void *)k_l2l64, (const void *)k_l2p64, (const void *)k_gather});
         const size_t sm = sizeof(double) * M2L_CH * n4;
         if (sm > 48 * 1024)
             IBIM_CUDA(cudaFuncSetAttribute(k_m2l_v64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1438,15 +1446,26 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         IBIM_CUDA(cudaStreamSynchronize(s));
     }
     const int full = (ff ? near_ff_occupancy() : NEAR_CPS) * c->num_sms;
+    // Beside the FP64 operator's digit products the near field starts when they do, not with the P2M: the upward
+    // pass has the FP64 pipe to itself (2,000 atoms: 61.9 -> 56.9 ms a matvec).  It has to be resident
+    // before the products' CTAs queue, which a lower priority would wait for: m2l_oz64_run calls fork
+    // ahead of its split kernel.
+    const bool with_m2l = use_oz64 && S.nchunks_oz64 > 0;
     const int side = near_side_ctas() > 0 ? near_side_ctas() * c->num_sms : full;
-    if (overlap) {
-        if (!P.near_next.ptr) P.near_next.alloc(1, s);
-        IBIM_CUDA(cudaMemsetAsync(P.near_next.ptr, 0, sizeof(int), s));
-        if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
+    bool forked = false;
+    auto fork = [&] {
         IBIM_CUDA(cudaEventRecord(c->ev_near_fork, s));
         IBIM_CUDA(cudaStreamWaitEvent(c->aux, c->ev_near_fork, 0));
         near(c->aux, 0, std::min(nseg, side), P.near_next.ptr, true);
         IBIM_CUDA(cudaEventRecord(c->ev_near_join, c->aux));
+        forked = true;
+    };
+    const std::function<void()> beside = overlap && with_m2l ? std::function<void()>(fork) : nullptr;
+    if (overlap) {
+        if (!P.near_next.ptr) P.near_next.alloc(1, s);
+        IBIM_CUDA(cudaMemsetAsync(P.near_next.ptr, 0, sizeof(int), s));
+        if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
+        if (!with_m2l) fork();
     }
     try {
         if (P.np2m > 0) {
@@ -1467,7 +1486,7 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         if (use_oz) {
             m2l_oz_run(P, S);
         } else if (use_oz64) {
-            m2l_oz64_run(P, S);
+            m2l_oz64_run(P, S, beside);
         } else if (S.nchunks > 0) {
             ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
                           8.0 * n4 * (2.0 * S.nvpairs + (double)n4 * P.nops));
@@ -1489,7 +1508,7 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
             }
         }
     } catch (...) {
-        if (overlap) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
+        if (forked) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
         throw;
     }
     if (S.ntleaves > 0) {

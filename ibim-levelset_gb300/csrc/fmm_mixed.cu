@@ -445,14 +445,52 @@ __device__ __forceinline__ float exp2_ftz(float x) {
     return y;
 }
 
+// Two FP32 values in one register pair: one instruction for both (sm_100 and later).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 up2(f2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // Near field + L2P in FP32 for one target leaf per block: source leaves staged in shared memory
-// in the target leaf's frame (two 16-byte loads per source record); per-tile partial sums are
-// added with Kahan compensation.
-constexpr int NT32 = 128, TILE32 = 256;
+// in the target leaf's frame; per-tile partial sums are added with Kahan compensation.
+//
+// As scalar code it was bound by instruction issue (70 instructions a pair, 80 % of the issue slots, the
+// FMA pipe half idle).  A lane takes four sources a step as two register pairs: 37 packed
+// instructions, each two cycles of the FMA pipe, and four of the special-function unit for two pairs
+// of points.  Every warp works alone, on segments of its own (slabs of 32 targets, a tile of 64 sources as
+// seven arrays and their indices, filled up to a multiple of four with repeated points of zero
+// density), so there is no barrier, and two CTAs a SM fit beside the tensor-core M2L.  Inside the cutoff
+// 1 / r is set to 0, which leaves nothing of a pair but K2's constant, summed apart: a branch there was
+// taken by a quarter of the warps' steps.  K1 and K3 share M = d.m / r^3; G and psi carry K3's factor (k3q) outside
+// the pair loop.  Alone, on 2.05e9 pairs (5,000 atoms): 4.4 -> 3.6 ms; on 5.6e7 pairs (200 atoms, order 6):
+// 0.48 -> 0.16 ms.
+constexpr int NT32 = 128, NW32 = NT32 / 32, TILE32 = 64;  // threads, warps, sources a warp's tile
 // BATCH: a plan merged over several molecules (batch.cu); the kappa-dependent constants come from
 // the target leaf's molecule (kmol: kappa, -kappa log2 e, k2in / q4pi per molecule).
 template <bool BATCH>
-__global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict__ tab, KParams32 kp,
+__global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restrict__ tab, KParams32 kp,
                                                  const int4 *__restrict__ segs,
                                                  const int *__restrict__ nrange, const float *__restrict__ noff,
                                                  const int *__restrict__ tb_, const int *__restrict__ te_,
@@ -465,26 +503,24 @@ __global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict_
                                                  const double *__restrict__ tx64, const double *__restrict__ ty64,
                                                  const double *__restrict__ tz64, const float4 *__restrict__ kmol,
                                                  const int *__restrict__ node_mol, const int *__restrict__ mol_active) {
-    __shared__ ChebTables32 T;
-    // {x, y, z, q m_x}, {q m_y, q m_z, q psi, source index} in the target leaf's frame
-    __shared__ float4 S4[TILE32][2];
-    __shared__ float red[NT32][4];
-    __shared__ int cur;
-    load_tables(T, tab);
-    // with a work counter the CTA takes segments until none is left (several launches may drain
-    // the same counter); without one it does segment blockIdx.x
+    // x, y, z, q m_x, q m_y, q m_z, q psi / k3q, source index, in the target leaf's frame
+    __shared__ __align__(16) float S8w[NW32][8][TILE32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float(*S8)[TILE32] = S8w[warp];
+    float(*red)[4] = reinterpret_cast<float(*)[4]>(&S8[0][0]);  // [32][4], once the tiles are done
+    const float ik3q = 1.f / kp.k3q;
+    // with a work counter the warp takes segments until none is left (several launches may drain
+    // the same counter); without one it does segment blockIdx.x NW32 + warp
     for (int it = 0;; ++it) {
         int si;
         if (next) {
-            __syncthreads();  // every thread has read the previous segment number
-            if (threadIdx.x == 0) cur = atomicAdd(next, 1);
-            __syncthreads();
-            si = cur;
-            if (si >= nseg) break;
+            if (lane == 0) si = atomicAdd(next, 1);
+            si = __shfl_sync(0xffffffffu, si, 0);
         } else {
             if (it > 0) break;
-            si = blockIdx.x;
+            si = blockIdx.x * NW32 + warp;
         }
+        if (si >= nseg) break;
         const int4 sg = segs[si];
         const int leaf = sg.x, r0 = sg.y, r1 = sg.z, mode = sg.w;
         const int tb = tb_[leaf], te = te_[leaf];
@@ -496,32 +532,48 @@ __global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict_
             kl2 = km.y;
             k2q = km.z;
         }
-        __syncthreads();
-        for (int t0 = tb; t0 < te; t0 += NT32) {
-            const int nT = min(NT32, te - t0);
-            const int nph = NT32 / nT;
-            const int my_t = threadIdx.x % nT, ph = threadIdx.x / nT;
+        const bool laplace = kap == 0.f;  // e = 1: K2 = K3 = 0
+        const f2 kap2 = pk2(kap, kap), kl22 = pk2(kl2, kl2), eps2 = pk2(kp.eps, kp.eps), ieps2 = pk2(kp.ieps, kp.ieps);
+        const f2 one2 = pk2(1.f, 1.f), mone2 = pk2(-1.f, -1.f), three2 = pk2(3.f, 3.f), mthree2 = pk2(-3.f, -3.f);
+        const f2 mvr2 = pk2(-kp.vr2, -kp.vr2);
+        const f2 k3q2 = pk2(kp.k3q, kp.k3q), mk3q2 = pk2(-kp.k3q, -kp.k3q);
+        for (int t0 = tb; t0 < te; t0 += 32) {  // slabs of 32 targets; the last one's lanes take more phases
+            const int nT = min(32, te - t0);
+            const int nph = 32 / nT;
+            const int my_t = lane % nT, ph = lane / nT;
             const bool active = ph < nph;
             float X = 0.f, Y = 0.f, Z = 0.f;
             if (active) { X = tx[t0 + my_t]; Y = ty[t0 + my_t]; Z = tz[t0 + my_t]; }
+            const f2 mX = pk2(-X, -X), mY = pk2(-Y, -Y), mZ = pk2(-Z, -Z);
             const long tg64 = active ? t0 + my_t : t0;  // the target's FP64 coordinates, for the cutoff
             float sum[4] = {0.f, 0.f, 0.f, 0.f}, cmp[4] = {0.f, 0.f, 0.f, 0.f};
             // fill tiles across consecutive source leaves
             int rr = r0, pos = r1 > r0 ? nrange[2 * r0] : 0;
             while (rr < r1) {
-                __syncthreads();
+                __syncwarp();
                 int filled = 0;
-                // sequentially pack up to TILE32 sources; each thread copies its slots
+                // sequentially pack up to TILE32 sources; each lane copies its slots
                 int lrr = rr, lpos = pos;
                 while (lrr < r1 && filled < TILE32) {
                     const int e = nrange[2 * lrr + 1];
                     const int take = min(TILE32 - filled, e - lpos);
                     const float ox = noff[3 * lrr], oy = noff[3 * lrr + 1], oz = noff[3 * lrr + 2];
-                    for (int q = threadIdx.x; q < take; q += blockDim.x) {
-                        const int si = lpos + q;
-                        const float4 A = __ldg(src8 + 2 * si), B = __ldg(src8 + 2 * si + 1);
-                        S4[filled + q][0] = make_float4(A.x + ox, A.y + oy, A.z + oz, A.w);
-                        S4[filled + q][1] = make_float4(B.x, B.y, B.z, __int_as_float(si));
+                    // the last sources of the tile are repeated with zero density up to a multiple of 4
+                    const bool last = lrr + 1 >= r1 && lpos + take >= e;
+                    const int pad = last ? (-(filled + take)) & 3 : 0;
+                    for (int q = lane; q < take + pad; q += 32) {
+                        const bool own = q < take;
+                        const int sj = lpos + (own ? q : take - 1);
+                        const float4 A = __ldg(src8 + 2 * sj), B = __ldg(src8 + 2 * sj + 1);
+                        const int d = filled + q;
+                        S8[0][d] = A.x + ox;
+                        S8[1][d] = A.y + oy;
+                        S8[2][d] = A.z + oz;
+                        S8[3][d] = own ? A.w : 0.f;
+                        S8[4][d] = own ? B.x : 0.f;
+                        S8[5][d] = own ? B.y : 0.f;
+                        S8[6][d] = own ? B.z * ik3q : 0.f;
+                        S8[7][d] = __int_as_float(sj);
                     }
                     filled += take;
                     lpos += take;
@@ -532,49 +584,83 @@ __global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict_
                 }
                 rr = lrr;
                 pos = lpos;
-                __syncthreads();
+                __syncwarp();
                 if (active) {
-                    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+                    f2 a0 = 0ull, a1 = 0ull, a2 = 0ull, a3 = 0ull;
+                    float ain = 0.f;
                     // the densities carry 1 / (4 pi): the K1, K2, K4 factors lose it and the K3 ones
                     // take k3f / q4pi (near_pair64 has the unscaled form)
-                    for (int q = ph; q < filled; q += nph) {
-                        const float4 P0 = S4[q][0], P1 = S4[q][1];
-                        const float dx = P0.x - X, dy = P0.y - Y, dz = P0.z - Z;
-                        // the cutoff test is a discontinuity: d2 in the FP64 kernel's evaluation order
-                        // (near_pair64), so points at exactly tau h decide alike in both precisions
-                        const float d2 = dx * dx + dy * dy + dz * dz;
-                        if (d2 < kp.vr2_guard) {  // rare: inside the cutoff or within rounding of it
-                            bool inside = d2 < kp.vr2;
-                            if (fabsf(d2 - kp.vr2) < kp.vr2_band) {
-                                // within FP32 rounding of the cutoff: decide on the FP64 coordinates,
-                                // as the FP64 and float-float kernels do
-                                const int sj = __float_as_int(P1.w);
-                                const double ex = sx64[sj] - tx64[tg64], ey = sy64[sj] - ty64[tg64],
-                                             ez = sz64[sj] - tz64[tg64];
-                                inside = ex * ex + ey * ey + ez * ez < kp.vr2_64;
-                            }
-                            if (inside) {
-                                a0 = fmaf(-k2q, P1.z, a0);
-                                continue;
+                    for (int q = 4 * ph; q < filled; q += 4 * nph) {
+                        const ulonglong2 xs = *reinterpret_cast<const ulonglong2 *>(&S8[0][q]),
+                                         ys = *reinterpret_cast<const ulonglong2 *>(&S8[1][q]),
+                                         zs = *reinterpret_cast<const ulonglong2 *>(&S8[2][q]);
+                        const ulonglong2 m0s = *reinterpret_cast<const ulonglong2 *>(&S8[3][q]),
+                                         m1s = *reinterpret_cast<const ulonglong2 *>(&S8[4][q]),
+                                         m2s = *reinterpret_cast<const ulonglong2 *>(&S8[5][q]),
+                                         pss = *reinterpret_cast<const ulonglong2 *>(&S8[6][q]);
+                        f2 dx[2], dy[2], dz[2];
+                        float2 d2[2], u[2];  // u = d2 - (tau h)^2: negative inside the cutoff
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            dx[h] = add2(h ? xs.y : xs.x, mX);
+                            dy[h] = add2(h ? ys.y : ys.x, mY);
+                            dz[h] = add2(h ? zs.y : zs.x, mZ);
+                            const f2 dd = fma2(dz[h], dz[h], fma2(dy[h], dy[h], mul2(dx[h], dx[h])));
+                            d2[h] = up2(dd);
+                            u[h] = up2(add2(dd, mvr2));
+                        }
+                        if (fminf(fminf(fabsf(u[0].x), fabsf(u[0].y)), fminf(fabsf(u[1].x), fabsf(u[1].y))) < kp.vr2_band) {
+                            // within FP32 rounding of the cutoff: decide on the FP64 coordinates, as the
+                            // FP64 and float-float kernels do
+#pragma unroll
+                            for (int l = 0; l < 4; ++l) {
+                                float &ul = l & 1 ? u[l >> 1].y : u[l >> 1].x;
+                                if (fabsf(ul) < kp.vr2_band) {
+                                    const int sj = __float_as_int(S8[7][q + l]);
+                                    const double ex = sx64[sj] - tx64[tg64], ey = sy64[sj] - ty64[tg64],
+                                                 ez = sz64[sj] - tz64[tg64];
+                                    ul = ex * ex + ey * ey + ez * ez < kp.vr2_64 ? -1.f : 1.f;
+                                }
                             }
                         }
-                        const float ir = rsqrt_ftz(d2), r = d2 * ir, ir2 = ir * ir, ir3 = ir2 * ir;
-                        const float t = kap * r, e = exp2_ftz(kl2 * r), et1 = fmaf(e, t, e);
-                        const float h3 = ir3 * kp.k3q;
-                        const float c1 = fmaf(kp.eps, et1, -1.f) * ir3;
-                        const float c4 = fmaf(-kp.ieps, et1, 1.f) * ir3;
-                        const float k2 = (1.f - e) * ir;
-                        const float hd = (1.f - et1) * h3;
-                        const float ho = fmaf(e, fmaf(t + 3.f, t, 3.f), -3.f) * h3 * ir2;
-                        const float dm = fmaf(dx, P0.w, fmaf(dy, P1.x, dz * P1.y));
-                        a0 = fmaf(c1, dm, fmaf(-k2, P1.z, a0));
-                        const float cm = fmaf(ho, dm, -c4 * P1.z);
-                        a1 = fmaf(hd, P0.w, fmaf(dx, cm, a1));
-                        a2 = fmaf(hd, P1.x, fmaf(dy, cm, a2));
-                        a3 = fmaf(hd, P1.y, fmaf(dz, cm, a3));
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const f2 m0 = h ? m0s.y : m0s.x, m1 = h ? m1s.y : m1s.x, m2 = h ? m2s.y : m2s.x,
+                                     ps = h ? pss.y : pss.x;
+                            // inside the cutoff 1 / r = 0 leaves nothing of the pair but K2's constant
+                            const float2 P = up2(ps);
+                            if (u[h].x < 0.f) ain += P.x;
+                            if (u[h].y < 0.f) ain += P.y;
+                            const f2 ir = pk2(u[h].x < 0.f ? 0.f : rsqrt_ftz(d2[h].x), u[h].y < 0.f ? 0.f : rsqrt_ftz(d2[h].y));
+                            const f2 ir2 = mul2(ir, ir), ir3 = mul2(ir2, ir);
+                            const f2 M = mul2(fma2(dx[h], m0, fma2(dy[h], m1, mul2(dz[h], m2))), ir3);
+                            const f2 w = mul2(ps, ir3);
+                            if (laplace) {
+                                const f2 cw = mul2(add2(ieps2, mone2), w);
+                                a0 = fma2(add2(eps2, mone2), M, a0);
+                                a1 = fma2(dx[h], cw, a1);
+                                a2 = fma2(dy[h], cw, a2);
+                                a3 = fma2(dz[h], cw, a3);
+                                continue;
+                            }
+                            const f2 r = mul2(pk2(d2[h].x, d2[h].y), ir);
+                            const f2 t = mul2(kap2, r);
+                            const float2 x2 = up2(mul2(kl22, r));
+                            const f2 e = pk2(exp2_ftz(x2.x), exp2_ftz(x2.y));
+                            const f2 et1 = fma2(e, t, e);
+                            a0 = fma2(fma2(eps2, et1, mone2), M, a0);
+                            a0 = fma2(mul2(fma2(k3q2, e, mk3q2), ir), ps, a0);
+                            const f2 ho = fma2(e, fma2(add2(t, three2), t, three2), mthree2);
+                            const f2 cm = fma2(fma2(ieps2, et1, mone2), w, mul2(ho, mul2(ir2, M)));
+                            const f2 hd = mul2(fma2(et1, mone2, one2), ir3);
+                            a1 = fma2(dx[h], cm, fma2(hd, m0, a1));
+                            a2 = fma2(dy[h], cm, fma2(hd, m1, a2));
+                            a3 = fma2(dz[h], cm, fma2(hd, m2, a3));
+                        }
                     }
-                    const float part[4] = {a0, a1, a2, a3};
-    #pragma unroll
+                    const float2 b0 = up2(a0), b1 = up2(a1), b2 = up2(a2), b3 = up2(a3);
+                    const float part[4] = {fmaf(-k2q * kp.k3q, ain, b0.x + b0.y), b1.x + b1.y, b2.x + b2.y, b3.x + b3.y};
+#pragma unroll
                     for (int o = 0; o < 4; ++o) {  // Kahan: sum += part
                         const float yk = part[o] - cmp[o];
                         const float tk = sum[o] + yk;
@@ -583,15 +669,17 @@ __global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict_
                     }
                 }
             }
-            __syncthreads();
-            for (int o = 0; o < 4; ++o) red[threadIdx.x][o] = sum[o] - cmp[o];
-            __syncthreads();
-            if (threadIdx.x < nT) {
+            __syncwarp();
+            red[lane][0] = sum[0] - cmp[0];
+            for (int o = 1; o < 4; ++o) red[lane][o] = (sum[o] - cmp[o]) * kp.k3q;
+            __syncwarp();
+            if (lane < nT) {
                 double f[4] = {0., 0., 0., 0.};
                 for (int q = 0; q < nph; ++q)
-                    for (int o = 0; o < 4; ++o) f[o] += (double)red[threadIdx.x + q * nT][o];
+                    for (int o = 0; o < 4; ++o) f[o] += (double)red[lane + q * nT][o];
                 float l2p[4] = {0.f, 0.f, 0.f, 0.f};
                 if (mode & l2p_mask & 1) {  // L2P by the leaf's first segment
+                    const ChebTables32 &T = *tab;
                     float Sp[3][MAXP];
                     const float xyz[3] = {X, Y, Z};
                     for (int a = 0; a < 3; ++a) interp1f(T, xyz[a] / rad[3 * leaf + a], Sp[a]);
@@ -603,12 +691,12 @@ __global__ void __launch_bounds__(NT32) k_near32(const ChebTables32 *__restrict_
                     }
                 }
                 for (int o = 0; o < 4; ++o) {
-                    double *dst = out + o * nt + t0 + threadIdx.x;
+                    double *dst = out + o * nt + t0 + lane;
                     if (mode & 2) atomicAdd(dst, f[o] + (double)l2p[o]);
                     else *dst = f[o] + (double)l2p[o];
                 }
             }
-            __syncthreads();
+            __syncwarp();
         }
     }
 }
@@ -733,7 +821,9 @@ void mixed_lists_host(const Plan &P, TargetSet &S) {
         for (int u : T.U[i]) add_run(u);
         for (int w : T.W[i]) add_run(w);
     }
-    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, P.tune.near_seg_pairs);
+    // a segment is one warp's: at least four a resident warp, 2^11 to 2^14 pairs
+    const long cap32 = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (80L * P.ctx->num_sms)));
+    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, std::min(P.tune.near_seg_pairs, cap32), 64);
     S.nnear32_seg = tl32.empty() ? 0 : (int)S.h_seg32.size() / 4;
     S.nearff_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_segff, P.tune.nearff_seg_pairs, 128);
     S.nnearff_seg = tl32.empty() ? 0 : (int)S.h_segff.size() / 4;
@@ -922,7 +1012,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     // the auxiliary stream at full occupancy, CTAs taking work segments from a counter, and fills
     // the SMs the latency-bound far-field launches (P2M, M2M levels) leave idle; the L2P follows
     // the join.  A smaller side launch (IBIM_NEAR_SIDE CTAs per SM) leaves the rest to a drain
-    // launch after the far field
+    // launch after the far field.  All kernels ask for the same shared-memory split (side_by_side)
     auto near = [&](cudaStream_t st, int l2p_mask, int grid, int *next, double flops) {
         ProfScope ps_(PROF_NEAR, flops, flops > 0 ? 28.0 * P.ns + 40.0 * S.nt : 0., st);
         auto kern = P.batched ? k_near32<true> : k_near32<false>;
@@ -933,21 +1023,35 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
                                                   tx64, ty64, tz64, P.kmol32.ptr, P.node_mol.ptr, P.mol_active.ptr));
     };
     const bool overlap = near_overlap() && S.ntleaves > 0;
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_near32<false>, (const void *)k_near32<true>, (const void *)k_pack_src32,
+                         (const void *)k_p2m32, (const void *)k_m2m32, (const void *)k_l2l32, (const void *)k_l2p32});
     static const int occ = [] {
         int b = 0;
         IBIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_near32<false>, NT32, 0));
         return std::max(1, b);
     }();
-    const int full = occ * c->num_sms, side = near_side_ctas() > 0 ? near_side_ctas() * c->num_sms : full;
+    // Beside the pair form of the M2L (one CTA an SM) the SM has room for two near-field CTAs, and a drain
+    // launch takes what they leave; they start with it, on idle SMs (started with the P2M, three and
+    // more could come to lie on one SM, and the M2L's CTAs found no place until they were done:
+    // 7.2 or 13.3 ms a 5,000-atom matvec by chance).  The other forms fill the SM, and the near field runs first.
+    // 2,000-atom solve: 138 ms with the near field first, 147, 130 and 142 with one, two and three CTAs an SM.
+    const bool with_m2l = tc && m2l_tc_pairs(P, S) && S.nchunks_tc2 > 0;
+    const int ctas = near_side_ctas() > 0 ? near_side_ctas() : (with_m2l ? 2 : 0);
+    const int full = occ * c->num_sms, side = ctas > 0 ? ctas * c->num_sms : full;
+    bool forked = false;
+    auto fork = [&] {
+        IBIM_CUDA(cudaEventRecord(c->ev_near_fork, s));
+        IBIM_CUDA(cudaStreamWaitEvent(c->aux, c->ev_near_fork, 0));
+        near(c->aux, 0, std::min(div_up(S.nnear32_seg, NW32), side), P.near_next.ptr, 70.0 * S.near_pairs);
+        IBIM_CUDA(cudaEventRecord(c->ev_near_join, c->aux));
+        forked = true;
+    };
     if (overlap) {
         if (!P.near_next.ptr) P.near_next.alloc(1, s);
         IBIM_CUDA(cudaMemsetAsync(P.near_next.ptr, 0, sizeof(int), s));
         if (S.near32_atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
-        IBIM_CUDA(cudaEventRecord(c->ev_near_fork, s));
-        IBIM_CUDA(cudaStreamWaitEvent(c->aux, c->ev_near_fork, 0));
-        near(c->aux, 0, std::min(S.nnear32_seg, side), P.near_next.ptr,
-             70.0 * S.near_pairs);
-        IBIM_CUDA(cudaEventRecord(c->ev_near_join, c->aux));
+        if (!with_m2l) fork();
     }
     try {
         if (P.np2m > 0) {
@@ -967,7 +1071,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
         }
         P.local32.zero();
         if (tc) {
-            m2l_tc_run(P, S);
+            m2l_tc_run(P, S, overlap && with_m2l ? std::function<void()>(fork) : nullptr);
         } else if (S.nchunks32 > 0) {
             ProfScope ps_(PROF_M2L_V, 2.0 * n4 * (double)n4 * S.nvpairs, 4.0 * n4 * (2.0 * S.nvpairs + (double)n4 * P.nops));
             const dim3 grid(S.nchunks32, div_up(n4, GM_BM));
@@ -988,18 +1092,18 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
             }
         }
     } catch (...) {
-        if (overlap) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
+        if (forked) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
         throw;
     }
     if (overlap) {
-        if (side < std::min(S.nnear32_seg, full)) near(s, 0, std::min(S.nnear32_seg, full), P.near_next.ptr, 0.);
+        if (side < std::min(div_up(S.nnear32_seg, NW32), full)) near(s, 0, std::min(div_up(S.nnear32_seg, NW32), full), P.near_next.ptr, 0.);
         IBIM_CUDA(cudaStreamWaitEvent(s, c->ev_near_join, 0));
         ProfScope ps_(PROF_L2P, (10.0 * R + 6.0 * P.p * P.p) * S.nt, 16.0 * n4 * S.ntleaves + 44.0 * S.nt);
         (count_launch(), k_l2p32<<<S.ntleaves, NT32, 0, s>>>(tab, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr, P.nrad32.ptr,
                                                              tx, ty, tz, S.nt, P.local32.ptr, out));
     } else if (S.ntleaves > 0) {
         if (S.near32_atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
-        near(s, 1, S.nnear32_seg, nullptr, 70.0 * S.near_pairs);
+        near(s, 1, div_up(S.nnear32_seg, NW32), nullptr, 70.0 * S.near_pairs);
     }
     IBIM_CHECK_LAUNCH();
 }

@@ -1,10 +1,14 @@
 // Internal types shared by the translation units of libibim_gb300.so.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <functional>
+#include <initializer_list>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -92,8 +96,15 @@ struct DevBuf {
 
 // Kernels that run beside each other on an SM ask for the same split of L1 and shared memory (all
 // shared): with the default each kernel picks its own, and an SM changes its split only when idle.
-inline void side_by_side(const void *kernel) {
-    IBIM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+// `done`: the call site's own record of the devices that have it (a function's attributes are a device's).
+inline void side_by_side(std::atomic<uint64_t> &done, std::initializer_list<const void *> kernels) {
+    int dev = 0;
+    IBIM_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load() & bit) return;
+    for (const void *k : kernels)
+        IBIM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    done.fetch_or(bit);
 }
 
 // Host scratch array without value-initialisation, for large arrays that are written in full
@@ -355,6 +366,7 @@ struct Plan {
     bool tc_h16 = false;               // images in the scaled FP16 form (else TF32)
     DevBuf<float> tc_a_hi, tc_a_lo, tc_b_hi, tc_b_lo;  // raw image words
     DevBuf<float> tc_rsc, tc_csc;      // FP16 form: operator row scales, multipole column scales
+    CUtensorMap tc_map[2];             // tensor maps over the operator images hi, lo
     DevBuf<int> tc_err;
     // FP64-class V-list M2L of the refinement residual (m2l_tc.cu): operators and multipoles as
     // exact BF16 integer slices under power-of-two row / column scales
@@ -417,7 +429,10 @@ bool m2l_tc_supported();
 void m2l_tc_pack(Plan &P, const float2 *ff = nullptr);
 // Whether the mixed path's tensor-core M2L uses the scaled FP16 operand form.
 bool m2l_tc_fp16_form();
-void m2l_tc_run(Plan &P, TargetSet &S);
+// beside: called between the multipoles' split and the contraction (work for another stream, to run beside it).
+void m2l_tc_run(Plan &P, TargetSet &S, const std::function<void()> &beside = nullptr);
+// Whether a target set's M2L takes the CTA-pair form that leaves room for the near field beside it.
+bool m2l_tc_pairs(const Plan &P, const TargetSet &S);
 int m2l_tc_error(Plan &P);
 // BF16 digit images and row scales from P.ops64, or from float-float operators when ff is given.
 void m2l_oz_pack(Plan &P, const float2 *ff = nullptr);
@@ -433,7 +448,9 @@ double m2l_oz64_op_bytes(int p);
 bool m2l_oz64_fits(int p, double nops);
 void m2l_oz64_alloc(Plan &P);
 void m2l_oz64_pack(Plan &P, const double *ops, int o, int n);
-void m2l_oz64_run(Plan &P, const TargetSet &S);
+// beside: called before the multipoles' split (work for another stream that has to be on the SMs before the
+// contraction's many CTAs queue for them).
+void m2l_oz64_run(Plan &P, const TargetSet &S, const std::function<void()> &beside = nullptr);
 // Operator images for kernel parameters kp, built when missing or stale: the TF32 images (from
 // FP32 operators, which are then released) and the digit images (from the FP64 operators).
 void fmm_ensure_tc_images(Plan &P, const ibim_kernel_params &kp);
@@ -465,7 +482,7 @@ void mixed_lists_host(const Plan &P, TargetSet &S);
 // IBIM_NEAR_OVERLAP=0 runs it after the far field with the L2P fused in).
 bool near_overlap();
 // CTAs per SM of the near-field launch that runs beside the far field (IBIM_NEAR_SIDE; 0, the
-// default, is full occupancy); a drain launch after the far field takes the segments it leaves.
+// default, leaves the choice to the path); a drain launch after the far field takes the segments it leaves.
 int near_side_ctas();
 
 // Near-field work segments.  Target leaf k (node tl[k], nt[k] targets) owns source ranges

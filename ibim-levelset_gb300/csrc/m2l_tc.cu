@@ -22,8 +22,10 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdlib>
+#include <functional>
 #include <type_traits>
 
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include "fmm_common.cuh"
@@ -914,6 +916,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
     cluster_sync_all();  // neither CTA leaves while the other may still use the pair's TMEM
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TC2_PT * TC2_N));
+    __syncwarp();
+    cluster_sync_all();  // as in k_m2l_pair
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1191,6 +1195,293 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, PT == 1 
     cluster_sync_all();  // neither CTA leaves while the other may still use the pair's TMEM
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(PT * TC2_N));
+    __syncwarp();
+    cluster_sync_all();  // as in k_m2l_pair
+}
+
+// ---------------------------------------------------------------------------------------------
+// The scaled FP16 contraction on CTA pairs (the default form): a persistent kernel of one CTA per
+// SM, two to a cluster, walking units of (chunk of up to 256 pairs, two row tiles).  A unit's MMAs are
+// cta_group::2, M = 256 (each CTA's row tile) x N (the chunk's pairs rounded up to 16) x K = 16.
+//
+// What bounded the one-CTA form (two CTAs of two row tiles an SM: 4.14 ms on a 5,000-atom protein
+// at order 5, 2.35 M pairs, 0.46 of the tensor rate): 768 KB of operand copies out of L2 for every 12,288
+// cycles of MMAs, shared-memory reads at the full 128 bytes a cycle for N = 128, and a barrier round
+// trip with 192 gathering threads every 16 K elements.  Here an SM copies 512 KB for the same MMAs
+// and reads 96 bytes a cycle at N = 256 (its own 128 rows of the operator, half of the pairs), and a
+// stage is 64 K elements.  Roles: one thread copies operator tiles (TMA boxes of four 4 KB
+// tiles; both CTAs' complete on the even CTA's barrier), four warps gather multipole rows by cp.async into the
+// 128-byte swizzle (TMA gather4 took 18 cycles a row of 128 bytes, twice the MMAs' time), the even
+// CTA's MMA thread issues for the pair and its commits free a stage in both, eight warps drain one
+// accumulator slot of 256 TMEM columns while the next unit's MMAs fill the other (four warps, eight
+// columns a step, took longer than the MMAs).
+// 4.14 -> 2.48 ms, 0.77 of the tensor rate; without its MMAs' last two products 2.14, without gathers 2.12,
+// without the adds into the locals 2.20: no one part bounds it.  At order 6 on 200 atoms (100 pairs an
+// operator) 1.21 -> 1.13 ms: 4.6 GB of operators out of HBM take 0.68.
+// Every wait is bounded; one that runs out sets the error word and ends the CTA's roles.
+// ---------------------------------------------------------------------------------------------
+constexpr int HP_N = 256, HP_KB = 64, HP_NST = 3;
+constexpr int HP_GATHER = 4, HP_DRAIN = 8, HP_THREADS = 32 * (2 + HP_GATHER + HP_DRAIN);  // warps of either role
+constexpr int HP_TILE = 128 * HP_KB * 2;                      // 16 KB: 128 rows x 64 K elements
+constexpr int HP_STAGE = 4 * HP_TILE;                         // operator hi, lo, multipole hi, lo
+constexpr int HP_SMEM = HP_NST * HP_STAGE + 1024;             // the last for the stages' 1 KB alignment
+
+// Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle (rows of 128 bytes, 8-row
+// groups 1 KB apart).
+__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ void tma_box_pair(uint32_t dst, const void *map, int x, int y, uint32_t mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+        "%3}], [%4];" ::"r"(dst),
+        "l"(map), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
+}
+// 32 consecutive accumulator columns of the warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t v[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HP_THREADS, 2)  // 72 registers: the rest is the near field's
+    k_m2l_pair(int n4, int kpad, int mtiles, int nunits, const int *__restrict__ chunks, const int *__restrict__ vsrc,
+               const int *__restrict__ vtgt, const __grid_constant__ CUtensorMap map_hi,
+               const __grid_constant__ CUtensorMap map_lo, const char *__restrict__ b_hi, const char *__restrict__ b_lo,
+               const float *__restrict__ rscale, const float *__restrict__ cscale, float *local, int *err) {
+    extern __shared__ unsigned char hp_raw[];
+    __shared__ __align__(8) uint64_t full[HP_NST], empty[HP_NST], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_base;
+    __shared__ int2 pair_s[2][HP_N];  // per accumulator slot: target node (-1: none), column scale
+    __shared__ volatile int abort_s;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t smem = (smem_u32(hp_raw) + 1023u) & ~1023u;  // the same offset in both CTAs
+    const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
+    const int npt = (mtiles + 1) / 2;           // row-tile pairs
+    const int nst16 = kpad / TC_KS16;           // K = 16 steps
+    const int nkb = (nst16 + 3) / 4;            // stages a unit
+    if (tid == 0) {
+        abort_s = 0;
+        for (int i = 0; i < HP_NST; ++i) {
+            // the operator copies' expected bytes and both CTAs' gathering warps
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[i])), "r"(1 + 2 * HP_GATHER));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[i])));
+        }
+        for (int i = 0; i < 2; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[i])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[i])), "r"(2 * HP_DRAIN));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;");
+    }
+    if (warp == 0) {  // collective over the pair: both CTAs allocate, and receive the same columns
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(2 * HP_N));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    cluster_sync_all();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem_d = tmem_base;
+    // unit u: chunk u / npt against row tiles 2 T (even CTA) and 2 T + 1 (odd), T = u % npt
+    auto width = [](int cnt) { return max(16, (cnt + 15) & ~15); };
+
+    if (warp == 0) {
+        if (lane == 0) {  // this CTA's operator tiles
+            long st = 0;
+            bool ok = true;
+            for (int u = cluster; u < nunits && ok; u += nclusters) {
+                const int chunk = u / npt;
+                const int tile = min(2 * (u - chunk * npt) + (int)rank, mtiles - 1);  // past the last: not drained
+                // box row of the tile's first step: 32 rows of 128 bytes a 4 KB step
+                const int y0 = (chunks[3 * chunk] * mtiles + tile) * nst16 * 32;
+                for (int kb = 0; kb < nkb; ++kb, ++st) {
+                    const int buf = (int)(st % HP_NST);
+                    if (st >= HP_NST) ok = mbar_wait(smem_u32(&empty[buf]), (uint32_t)(((st / HP_NST) - 1) & 1));
+                    if (abort_s) ok = false;
+                    if (!ok) break;
+                    const uint32_t base = smem + (uint32_t)buf * HP_STAGE, fb = cluster_addr(smem_u32(&full[buf]), 0);
+                    if (rank == 0)  // both CTAs' bytes
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[buf])),
+                                     "r"(4 * HP_TILE)
+                                     : "memory");
+                    tma_box_pair(base, &map_hi, 0, y0 + kb * 128, fb);
+                    tma_box_pair(base + HP_TILE, &map_lo, 0, y0 + kb * 128, fb);
+                }
+            }
+            if (!ok) {
+                abort_s = 1;
+                for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // copies in flight land before the CTA ends
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {  // MMA issue for the pair
+            constexpr uint32_t IDESC0 = (1u << 4) | ((256u >> 4) << 24);
+            long st = 0;
+            int n = 0;
+            bool ok = true;
+            for (int u = cluster; u < nunits && ok; u += nclusters) {
+                const int chunk = u / npt;
+                const uint32_t idesc = IDESC0 | ((uint32_t)(width(chunks[3 * chunk + 2]) >> 3) << 17);
+                const int slot = n & 1;
+                if (n >= 2) ok = mbar_wait(smem_u32(&acc_empty[slot]), (uint32_t)(((n >> 1) - 1) & 1));
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t d = tmem_d + (uint32_t)(slot * HP_N);
+                for (int kb = 0; kb < nkb && ok; ++kb, ++st) {
+                    const int buf = (int)(st % HP_NST);
+                    ok = mbar_wait(smem_u32(&full[buf]), (uint32_t)((st / HP_NST) & 1)) && !abort_s;
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    const uint32_t base = smem + (uint32_t)buf * HP_STAGE;
+                    const int steps = min(4, nst16 - 4 * kb);
+                    for (int j = 0; j < steps; ++j) {
+                        const uint64_t ah = make_desc(base + j * TC_TILE_BYTES, 128, 256);
+                        const uint64_t al = make_desc(base + HP_TILE + j * TC_TILE_BYTES, 128, 256);
+                        const uint64_t bh = make_desc_sw128(base + 2 * HP_TILE + 32 * j);
+                        const uint64_t bl = make_desc_sw128(base + 3 * HP_TILE + 32 * j);
+                        mma_f16_pair(d, ah, bh, idesc, kb + j > 0 ? 1u : 0u);
+                        mma_f16_pair(d, ah, bl, idesc, 1u);
+                        mma_f16_pair(d, al, bh, idesc, 1u);
+                    }
+                    commit_pair(smem_u32(&empty[buf]));
+                }
+                commit_pair(smem_u32(&acc_full[slot]));  // on every path: the last MMAs are waited for
+                ++n;
+            }
+            if (!ok) abort_s = 1;
+        }
+        __syncwarp();
+    } else if (warp < 2 + HP_GATHER) {
+        // this CTA's half of the multipole rows: eight lanes a row of 128 bytes, four rows a warp
+        // instruction; warp g takes rows 32 g .. + 31.  A stage is signalled once the next one is issued
+        const int g = warp - 2, c = lane & 7;
+        uint32_t dst[2];  // rows 4 i + lane / 8 of i even, odd: the 128-byte swizzle of the 16-byte pieces
+        for (int i = 0; i < 2; ++i) {
+            const int r = 4 * i + (lane >> 3);
+            dst[i] = (uint32_t)(2 * HP_TILE + (32 * g + r) * 128 + ((c ^ r) << 4));
+        }
+        long st = 0;
+        bool ok = true;
+        auto signal = [&](long s2) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)  // relaxed: the data lies in this CTA's shared memory, read there by its tensor core
+                asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                                 cluster_addr(smem_u32(&full[(int)(s2 % HP_NST)]), 0))
+                             : "memory");
+        };
+        for (int u = cluster; u < nunits && ok; u += nclusters) {
+            const int chunk = u / npt;
+            const int b = chunks[3 * chunk + 1], cnt = chunks[3 * chunk + 2];
+            const int half = width(cnt) >> 1, e = b + cnt - 1;
+            long src[8];  // byte offset of this lane's piece in rows 4 i + lane / 8; past the end the last pair again
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                src[i] = (long)vsrc[min(b + (int)rank * half + 32 * g + 4 * i + (lane >> 3), e)] * kpad * 2 + 16 * c;
+            const int nr = max(0, min(8, (half - 32 * g + 3) >> 2));  // four-row groups of this warp (half: a multiple of 8)
+            for (int kb = 0; kb < nkb; ++kb, ++st) {
+                const int buf = (int)(st % HP_NST);
+                if (st >= HP_NST) ok = mbar_wait(smem_u32(&empty[buf]), (uint32_t)(((st / HP_NST) - 1) & 1));
+                ok = __all_sync(0xffffffffu, ok && !abort_s);
+                if (!ok) break;
+                const uint32_t base = smem + (uint32_t)buf * HP_STAGE;
+                if (kb * HP_KB + 8 * c < kpad) {  // the last stage of an order may end early
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < nr) {
+                            const uint32_t d = base + dst[i & 1] + (i >> 1) * 1024;
+                            cp_async16(d, b_hi + src[i] + kb * HP_KB * 2, 16u);
+                            cp_async16(d + HP_TILE, b_lo + src[i] + kb * HP_KB * 2, 16u);
+                        }
+                }
+                asm volatile("cp.async.commit_group;");
+                if (st > 0) {
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    signal(st - 1);
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (ok && st > 0) signal(st - 1);
+        if (!ok) abort_s = 1;
+    } else {  // warp w reads TMEM lanes 32 (w % 4) .. + 31, its rows of this CTA's tile; two warps share them
+        const int lg = warp & 3, et = tid - 32 * (2 + HP_GATHER), part = (warp - 2 - HP_GATHER) >> 2;
+        int n = 0;
+        bool ok = true;
+        for (int u = cluster; u < nunits; u += nclusters) {
+            const int chunk = u / npt;
+            const int op = chunks[3 * chunk], b = chunks[3 * chunk + 1], cnt = chunks[3 * chunk + 2];
+            const int slot = n & 1;
+            const int tile = 2 * (u - chunk * npt) + (int)rank;
+            // every warp is done with this slot's list; all go on, or none
+            uint32_t go;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\t"
+                "setp.ne.u32 p, %1, 0;\n\t"
+                "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+                "selp.u32 %0, 1, 0, q;\n\t}"
+                : "=r"(go)
+                : "r"(ok && !abort_s ? 1u : 0u), "n"(32 * HP_DRAIN)
+                : "memory");
+            if (!go) break;
+            static_assert(32 * HP_DRAIN == HP_N, "one thread a pair");
+            pair_s[slot][et] = et < cnt ? make_int2(vtgt[b + et], __float_as_int(cscale[vsrc[b + et]])) : make_int2(-1, 0);
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * HP_DRAIN) : "memory");
+            const int row = tile * TC_M + 32 * lg + lane;
+            const float rs = tile < mtiles ? rscale[(long)op * mtiles * TC_M + row] : 0.f;
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[slot]), (uint32_t)((n >> 1) & 1)));
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            if (!ok) {
+                abort_s = 1;
+            } else if (tile < mtiles) {
+                const uint32_t taddr = tmem_d + ((uint32_t)(32 * lg) << 16) + (uint32_t)(slot * HP_N);
+                float *dst = local + row;
+#pragma unroll 1
+                for (int c0 = 32 * part; c0 < cnt; c0 += 64) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + (uint32_t)c0, v);
+                    if (row < n4) {
+#pragma unroll
+                        for (int q = 0; q < 32; ++q) {
+                            const int2 pr = pair_s[slot][c0 + q];
+                            if (pr.x >= 0)
+                                atomicAdd(dst + (long)pr.x * n4, __uint_as_float(v[q]) * rs * __int_as_float(pr.y));
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0 && ok)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                                 cluster_addr(smem_u32(&acc_empty[slot]), 0))
+                             : "memory");
+            ++n;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (abort_s && tid == 0) atomicExch(err, 1);
+    cluster_sync_all();  // neither CTA leaves while the other may still use the pair's TMEM and barriers
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(2 * HP_N));
+    __syncwarp();
+    // the pair's columns are free on both SMs before either CTA's place is: a kernel of another stream
+    // that took the place of a CTA whose peer had yet to deallocate could wait for its own columns for good
+    cluster_sync_all();
 }
 
 // hi = x rounded to TF32 (10 explicit mantissa bits, to nearest even), lo = x - hi.
@@ -1955,13 +2246,63 @@ static bool tc_fp16() {
 
 bool m2l_tc_fp16_form() { return tc_fp16(); }
 
-// Launch form of the contraction (the plan's tuning, tuning.cpp): two CTAs of two row tiles per SM
-// (2: one CTA's prologue and epilogue overlap the other's MMAs; 2.32 ms a launch on the 2,000-atom
-// protein), one CTA of four row tiles per SM (4; 2.50 ms) or, FP16 form only, persistent (0: one
+// Launch form of the contraction (the plan's tuning, tuning.cpp): the default 2, CTA pairs (k_m2l_pair)
+// in the FP16 form from order 4 and else two CTAs of two row tiles per SM (one CTA's prologue and epilogue
+// overlap the other's MMAs; 2.32 ms a launch on the 2,000-atom protein), one CTA of four row tiles per SM (4; 2.50 ms) or, FP16 form only, persistent (0: one
 // CTA per SM walking units of two row tiles with double-buffered accumulators; 2.94 ms).
+
+// The pair kernel's tensor maps: operator hi and lo images.
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        IBIM_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q));
+        if (q != cudaDriverEntryPointSuccess || !p) throw Error(IBIM_ERR_CUDA, "no cuTensorMapEncodeTiled in the driver");
+        return (EncodeTiled)p;
+    }();
+    return fn;
+}
+
+// rows x cols FP16, boxes of box_rows x 64.
+static CUtensorMap map_2d(const void *base, long rows, long cols, int box_rows, CUtensorMapSwizzle sw) {
+    CUtensorMap m;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {HP_KB, (cuuint32_t)box_rows}, es[2] = {1, 1};
+    const CUresult r = encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box,
+                                      es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw Error(IBIM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+    return m;
+}
+
+// Order 4 up: below, one row tile would leave the pair's odd CTA without work.  Not for merged plans: several
+// waves and preparations share the device there, and CTAs that come and go fit between each other
+// better than a persistent one that takes each SM (eight molecules of 50 to 400 atoms: 171 against 199 ms).
+static bool tc_pair_form(const Plan &P) { return P.tc_h16 && P.tune.tc_form == 2 && P.p >= 4 && !P.batched; }
+
+// From 64 pairs an operator: with few, a unit is the copy of its operator and the one-CTA form's smaller
+// units overlap better (20 pairs an operator, 60 atoms: 0.18 ms against 0.16; 100 at order 6, 200 atoms:
+// 1.13 against 1.21).
+bool m2l_tc_pairs(const Plan &P, const TargetSet &S) { return tc_pair_form(P) && S.nvpairs >= 64L * P.nops; }
+
+static void tc_maps(Plan &P) {
+    if (!tc_pair_form(P)) return;
+    // 32 rows of 128 bytes a 4 KB tile
+    const long rows = (long)std::max(1, P.nops) * (P.tc_mpad / TC_M) * (P.tc_kpad / TC_KS16) * 32;
+    P.tc_map[0] = map_2d(P.tc_a_hi.ptr, rows, HP_KB, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
+    P.tc_map[1] = map_2d(P.tc_a_lo.ptr, rows, HP_KB, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
+    IBIM_CUDA(cudaFuncSetAttribute(k_m2l_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, HP_SMEM));
+}
 
 // Shapes and device buffers of the contraction's images (operators, multipoles, scales).
 static void tc_alloc(Plan &P) {
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_m2l_pair, (const void *)k_split_mult_h16,
+                         (const void *)k_m2l_tc<M2L_CHTC, true, 2, 2>});
     P.tc_h16 = tc_fp16();
     cudaStream_t s = P.ctx->stream;
     const int n4 = 4 * P.R;
@@ -1983,6 +2324,7 @@ static void tc_alloc(Plan &P) {
         P.tc_err.alloc(1, s);
         P.tc_err.zero();
     }
+    tc_maps(P);
     // the contraction kernels' shared memory (above the 48 KB default)
     IBIM_CUDA(cudaFuncSetAttribute(k_m2l_tc<M2L_CHTC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    TcShape<M2L_CHTC>::SMEM));
@@ -2031,7 +2373,7 @@ void m2l_tc_pack(Plan &P, const float2 *ff) {
 // V-list M2L on the tensor cores; mult32 -> local32 (accumulating): chunks of 128 pairs against
 // two row tiles per CTA, two CTAs per SM (or four row tiles, one CTA per SM).  (Chunks of 256 pairs against two row tiles, k_m2l_tc<256>, measured 5.0 ms
 // against 3.9 ms on the 2,000-atom protein: the operator traffic falls but the chunks fill worse.)
-void m2l_tc_run(Plan &P, TargetSet &S) {
+void m2l_tc_run(Plan &P, TargetSet &S, const std::function<void()> &beside) {
     constexpr int N = M2L_CHTC;
     if (S.nchunks_tc == 0) return;
     cudaStream_t s = P.ctx->stream;
@@ -2043,6 +2385,7 @@ void m2l_tc_run(Plan &P, TargetSet &S) {
     else
         (count_launch(), k_split_mult_tc<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, P.tc_kpad, P.mult32.ptr,
                                                                             P.tc_b_hi.ptr, P.tc_b_lo.ptr));
+    if (beside) beside();
     const int mt = P.tc_mpad / TC_M;
     IBIM_REQUIRE(!S.chunk_mol_tc.ptr || (P.mol_img.ptr && P.mol_active.ptr), "merged plan without its image table");
     ProfScope ps_(PROF_M2L_V, 2.0 * n4 * (double)n4 * S.nvpairs,
@@ -2053,6 +2396,18 @@ void m2l_tc_run(Plan &P, TargetSet &S) {
         (count_launch(), k_m2l_tc2<<<grid2, TC_THREADS, TC2_SMEM, s>>>(
                              n4, P.tc_kpad, mt, S.v_chunk_tc2.ptr, S.v_src.ptr, S.v_tgt.ptr, P.tc_a_hi.ptr,
                              P.tc_a_lo.ptr, P.tc_b_hi.ptr, P.tc_b_lo.ptr, P.local32.ptr, P.tc_err.ptr));
+        IBIM_CHECK_LAUNCH();
+        return;
+    }
+    if (m2l_tc_pairs(P, S)) {
+        const int nunits = S.nchunks_tc2 * ((mt + 1) / 2);
+        if (nunits == 0) return;
+        const int grid = 2 * std::min(nunits, P.ctx->num_sms / 2);
+        (count_launch(), k_m2l_pair<<<grid, HP_THREADS, HP_SMEM, s>>>(
+                             n4, P.tc_kpad, mt, nunits, S.v_chunk_tc2.ptr, S.v_src.ptr, S.v_tgt.ptr, P.tc_map[0],
+                             P.tc_map[1], reinterpret_cast<const char *>(P.tc_b_hi.ptr),
+                             reinterpret_cast<const char *>(P.tc_b_lo.ptr), P.tc_rsc.ptr, P.tc_csc.ptr, P.local32.ptr,
+                             P.tc_err.ptr));
         IBIM_CHECK_LAUNCH();
         return;
     }
@@ -2107,6 +2462,9 @@ void m2l_tc_run(Plan &P, TargetSet &S) {
 // bits where K <= 800 (orders up to 5), else 7 of 6 bits.
 // Shapes and device buffers of the digit images (nops > 0).
 static void oz_alloc(Plan &P) {
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_m2l_oz<6>, (const void *)k_m2l_oz<7>, (const void *)k_split_mult_oz<6>,
+                         (const void *)k_split_mult_oz<7>});
     cudaStream_t s = P.ctx->stream;
     const int n4 = 4 * P.R;
     P.oz_kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS;
@@ -2321,9 +2679,9 @@ void m2l_oz64_alloc(Plan &P) {
     }
     IBIM_CUDA(cudaFuncSetAttribute(k_m2l_oz<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzShape<8>::SMEM));
     IBIM_CUDA(cudaFuncSetAttribute(k_m2l_oz<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzShape<9>::SMEM));
-    for (const void *k : {(const void *)k_m2l_oz<8>, (const void *)k_m2l_oz<9>, (const void *)k_split_mult_oz<8>,
-                          (const void *)k_split_mult_oz<9>})
-        side_by_side(k);
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_m2l_oz<8>, (const void *)k_m2l_oz<9>, (const void *)k_split_mult_oz<8>,
+                         (const void *)k_split_mult_oz<9>});
 }
 
 void m2l_oz64_pack(Plan &P, const double *ops, int o, int n) {
@@ -2344,13 +2702,14 @@ void m2l_oz64_pack(Plan &P, const double *ops, int o, int n) {
     IBIM_CHECK_LAUNCH();
 }
 
-void m2l_oz64_run(Plan &P, const TargetSet &S) {
+void m2l_oz64_run(Plan &P, const TargetSet &S, const std::function<void()> &beside) {
     if (S.nchunks_oz64 == 0) return;
     cudaStream_t s = P.ctx->stream;
     auto &Z = P.oz64;
     const int n4 = 4 * P.R;
     ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
                   2.0 * Z.s * Z.kpad * ((double)Z.mtiles * OZ_M * P.nops + (double)S.nvpairs));
+    if (beside) beside();
     auto split = Z.s == 8 ? k_split_mult_oz<8> : k_split_mult_oz<9>;
     (count_launch(), split<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, Z.kpad, P.mult.ptr, Z.b.ptr, Z.tau.ptr));
     auto kern = Z.s == 8 ? k_m2l_oz<8> : k_m2l_oz<9>;

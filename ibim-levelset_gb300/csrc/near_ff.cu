@@ -370,6 +370,8 @@ bool near_ff_enabled() {
 }
 
 int near_ff_occupancy() {
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_near_ff<false>, (const void *)k_near_ff<true>, (const void *)k_pack_src_ff});
     static const int occ = [] {
         int b = 0;
         IBIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_near_ff<false>, NTF, 0));

@@ -417,6 +417,11 @@ void apply_rot(double &dx, double &dy, double cs, double sn) {
 }  // namespace
 
 Krylov::Krylov(Ctx *c, long n_, int m_) : ctx(c), n(n_), m(m_) {
+    // between the matvecs, without a change of the SMs' split of L1 and shared memory
+    static std::atomic<uint64_t> split;
+    side_by_side(split, {(const void *)k_densities, (const void *)k_combine, (const void *)k_dot, (const void *)k_mgs,
+                         (const void *)k_normalize, (const void *)k_update, (const void *)k_sub, (const void *)k_axpy,
+                         (const void *)k_permute});
     cudaStream_t s = c->stream;
     V.alloc((size_t)(m + 1) * n, s);
     w.alloc(n, s);
