@@ -94,7 +94,10 @@ __global__ void k_to_f32(long n, const double *__restrict__ a, float *b) {
 // kernels' common factor q = 1 / (4 pi): {x, y, z, q m_x}, {q m_y, q m_z, q psi, 0}.
 __global__ void k_pack_src32(long ns, const double *__restrict__ dens, const float *__restrict__ sx,
                              const float *__restrict__ sy, const float *__restrict__ sz, float *d32, float4 *src8,
-                             double q) {
+                             double q, int *next, long nout, double *out) {
+    // the near field's work counter, and (nout > 0) its sums, start at zero
+    if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nout; i += (long)gridDim.x * blockDim.x) out[i] = 0.;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < ns; i += (long)gridDim.x * blockDim.x) {
         const double m0 = dens[i], m1 = dens[ns + i], m2 = dens[2 * ns + i], psi = dens[3 * ns + i];
         d32[i] = (float)m0;
@@ -1000,8 +1003,10 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     const KParams kp = make_kparams(kpp, P.tube->h);
     const KParams32 k32 = to32(kp);
     const ChebTables32 *tab = reinterpret_cast<const ChebTables32 *>(P.tables32.ptr);
+    if (!P.near_next.ptr) P.near_next.alloc(1, s);
     (count_launch(), k_pack_src32<<<ew(c, P.ns), 256, 0, s>>>(P.ns, dens, P.sxf.ptr, P.syf.ptr, P.szf.ptr,
-                                                               P.dens32.ptr, P.src8.ptr, kp.q4pi));
+                                                               P.dens32.ptr, P.src8.ptr, kp.q4pi, P.near_next.ptr,
+                                                               S.ntleaves > 0 && S.near32_atomic ? 4 * S.nt : 0, out));
     const float *tx = S.self ? P.sxf.ptr : S.txf.ptr;
     const float *ty = S.self ? P.syf.ptr : S.tyf.ptr;
     const float *tz = S.self ? P.szf.ptr : S.tzf.ptr;
@@ -1037,7 +1042,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     // 7.2 or 13.3 ms a 5,000-atom matvec by chance).  The other forms fill the SM, and the near field runs first.
     // 2,000-atom solve: 138 ms with the near field first, 147, 130 and 142 with one, two and three CTAs an SM.
     const bool with_m2l = tc && m2l_tc_pairs(P, S) && S.nchunks_tc2 > 0;
-    const int ctas = near_side_ctas() > 0 ? near_side_ctas() : (with_m2l ? 2 : 0);
+    const int ctas = near_side_ctas() > 0 ? near_side_ctas() : (tc && !P.batched ? 2 : 0);
     const int full = occ * c->num_sms, side = ctas > 0 ? ctas * c->num_sms : full;
     bool forked = false;
     auto fork = [&] {
@@ -1047,12 +1052,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
         IBIM_CUDA(cudaEventRecord(c->ev_near_join, c->aux));
         forked = true;
     };
-    if (overlap) {
-        if (!P.near_next.ptr) P.near_next.alloc(1, s);
-        IBIM_CUDA(cudaMemsetAsync(P.near_next.ptr, 0, sizeof(int), s));
-        if (S.near32_atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
-        if (!with_m2l) fork();
-    }
+    if (overlap && !with_m2l) fork();
     try {
         if (P.np2m > 0) {
             ProfScope ps_(PROF_P2M, (8.0 * R + 6.0 * P.p * P.p) * P.ns, 28.0 * P.ns);
@@ -1069,7 +1069,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
                                                                                 P.nempty.ptr, P.mult32.ptr));
             }
         }
-        P.local32.zero();
+        if (!(tc && m2l_tc_zeroes(P, S))) P.local32.zero();
         if (tc) {
             m2l_tc_run(P, S, overlap && with_m2l ? std::function<void()>(fork) : nullptr);
         } else if (S.nchunks32 > 0) {
@@ -1102,7 +1102,6 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
         (count_launch(), k_l2p32<<<S.ntleaves, NT32, 0, s>>>(tab, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr, P.nrad32.ptr,
                                                              tx, ty, tz, S.nt, P.local32.ptr, out));
     } else if (S.ntleaves > 0) {
-        if (S.near32_atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
         near(s, 1, div_up(S.nnear32_seg, NW32), nullptr, 70.0 * S.near_pairs);
     }
     IBIM_CHECK_LAUNCH();

@@ -431,6 +431,8 @@ void m2l_tc_pack(Plan &P, const float2 *ff = nullptr);
 bool m2l_tc_fp16_form();
 // beside: called between the multipoles' split and the contraction (work for another stream, to run beside it).
 void m2l_tc_run(Plan &P, TargetSet &S, const std::function<void()> &beside = nullptr);
+// Whether m2l_tc_run sets the locals to zero itself, with the multipoles' split.
+bool m2l_tc_zeroes(const Plan &P, const TargetSet &S);
 // Whether a target set's M2L takes the CTA-pair form that leaves room for the near field beside it.
 bool m2l_tc_pairs(const Plan &P, const TargetSet &S);
 int m2l_tc_error(Plan &P);

@@ -1626,7 +1626,7 @@ __global__ void k_pack_ops_h16(int n4, int mtiles, int kpad, int nops, const OW 
 // Multipoles [node][n4] (FP32) -> scaled FP16 hi / lo [node][kpad] and the column scales t_j.
 // One warp per node.
 __global__ void k_split_mult_h16(long nnodes, int n4, int kpad, const float *__restrict__ m, uint16_t *hi,
-                                 uint16_t *lo, float *cscale) {
+                                 uint16_t *lo, float *cscale, float *local) {
     const int lane = threadIdx.x & 31;
     const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1638,6 +1638,7 @@ __global__ void k_split_mult_h16(long nnodes, int n4, int kpad, const float *__r
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float sc = h16_scale(mx), inv = 1.f / sc;
         if (lane == 0) cscale[node] = sc;
+        for (int k = lane; k < n4; k += 32) local[node * n4 + k] = 0.f;  // the contraction adds into the locals
         for (int k = lane; k < kpad; k += 32) {
             uint16_t h, l;
             split_h16(k < n4 ? x[k] * inv : 0.f, h, l);
@@ -2246,6 +2247,8 @@ static bool tc_fp16() {
 
 bool m2l_tc_fp16_form() { return tc_fp16(); }
 
+bool m2l_tc_zeroes(const Plan &P, const TargetSet &S) { return P.tc_h16 && S.nchunks_tc > 0; }
+
 // Launch form of the contraction (the plan's tuning, tuning.cpp): the default 2, CTA pairs (k_m2l_pair)
 // in the FP16 form from order 4 and else two CTAs of two row tiles per SM (one CTA's prologue and epilogue
 // overlap the other's MMAs; 2.32 ms a launch on the 2,000-atom protein), one CTA of four row tiles per SM (4; 2.50 ms) or, FP16 form only, persistent (0: one
@@ -2381,7 +2384,7 @@ void m2l_tc_run(Plan &P, TargetSet &S, const std::function<void()> &beside) {
     if (P.tc_h16)
         (count_launch(), k_split_mult_h16<<<4 * P.ctx->num_sms, 256, 0, s>>>(
                              P.tree.nnodes, n4, P.tc_kpad, P.mult32.ptr, reinterpret_cast<uint16_t *>(P.tc_b_hi.ptr),
-                             reinterpret_cast<uint16_t *>(P.tc_b_lo.ptr), P.tc_csc.ptr));
+                             reinterpret_cast<uint16_t *>(P.tc_b_lo.ptr), P.tc_csc.ptr, P.local32.ptr));
     else
         (count_launch(), k_split_mult_tc<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, P.tc_kpad, P.mult32.ptr,
                                                                             P.tc_b_hi.ptr, P.tc_b_lo.ptr));

@@ -20,6 +20,8 @@ struct Krylov {
     long n;
     int m;
     DevBuf<double> V, w, r, part, hcol, ydev;
+    DevBuf<unsigned> bar;  // k_arnoldi's barrier: arrivals since the start, and whether a wait ran out
+    unsigned arrived = 0;
     double *hpin = nullptr;
     Krylov(Ctx *c, long n, int m);
     ~Krylov();
