@@ -14,6 +14,7 @@
 // (the mixed-precision path: storage and WENO arithmetic in FP32; tube points are emitted in
 // FP64 from the FP32 values).
 
+#include "f32x2.cuh"
 #include "internal.cuh"
 
 #include <cmath>
@@ -296,6 +297,40 @@ __device__ __forceinline__ T godunov(const T n[3], const T p[3]) {
     return D::root(v);
 }
 
+// Counts and deviations of a block's threads (256 at most) into the grid's.
+__device__ __forceinline__ void count_block(unsigned bad, unsigned tot, double acc, unsigned long long *counts,
+                                            double *accum) {
+    for (int o = 16; o > 0; o >>= 1) {
+        bad += __shfl_down_sync(0xffffffffu, bad, o);
+        tot += __shfl_down_sync(0xffffffffu, tot, o);
+        acc += __shfl_down_sync(0xffffffffu, acc, o);
+    }
+    __shared__ unsigned sb[8], st[8];
+    __shared__ double sa[8];
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    if ((tid & 31) == 0) {
+        sb[tid >> 5] = bad;
+        st[tid >> 5] = tot;
+        sa[tid >> 5] = acc;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        unsigned B = 0, Tt = 0;
+        double A = 0;
+        const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
+        for (int w = 0; w < nw; ++w) {
+            B += sb[w];
+            Tt += st[w];
+            A += sa[w];
+        }
+        if (Tt) {
+            atomicAdd(counts, (unsigned long long)B);
+            atomicAdd(counts + 1, (unsigned long long)Tt);
+            atomicAdd(accum, A);
+        }
+    }
+}
+
 // One TVD-RK3 stage over the whole grid.  MODE 0: evolve (phi_t + vel|grad phi| = 0);
 // MODE 1: reinitialize (phi_t + S(phi0)(|grad phi| - 1) = 0, S = phi0/sqrt(phi0^2 + dx^2)).
 // STAGE 0: u1 = g - L(g); 1: u2 = (3g + u1 - L(u1))/4; 2: g = (g + 2(u2 - L(u2)))/3.
@@ -307,28 +342,20 @@ __global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, 
                                                     T *u2, const T *__restrict__ phi0, T band = (T)0,
                                                     T thres = (T)0, unsigned long long *counts = nullptr,
                                                     double *accum = nullptr) {
+    // consecutive cells to consecutive threads: the FP64 pipe takes as long for a warp at a row's end
+    // with few cells as for a full one (a fifth of the warps of a 105^3 grid)
     int i, j, k;
-    bool in;
-    if constexpr (sizeof(T) == 8) {
-        // consecutive cells to consecutive threads: the FP64 pipe takes as long for a warp at a
-        // row's end with few cells as for a full one (a fifth of the warps of a 105^3 grid)
-        const long I = blockIdx.x * 256L + threadIdx.x;
-        in = I < (long)dm.nx * dm.ny * dm.nz;
-        if (I < (1L << 32)) {
-            const unsigned row = (unsigned)I / (unsigned)dm.nz;
-            k = (int)((unsigned)I - row * (unsigned)dm.nz);
-            i = (int)(row / (unsigned)dm.ny);
-            j = (int)(row - (unsigned)i * (unsigned)dm.ny);
-        } else {
-            k = (int)(I % dm.nz);
-            j = (int)(I / dm.nz % dm.ny);
-            i = (int)(I / dm.nz / dm.ny);
-        }
+    const long I0 = blockIdx.x * 256L + threadIdx.x;
+    const bool in = I0 < (long)dm.nx * dm.ny * dm.nz;
+    if (I0 < (1L << 32)) {
+        const unsigned row = (unsigned)I0 / (unsigned)dm.nz;
+        k = (int)((unsigned)I0 - row * (unsigned)dm.nz);
+        i = (int)(row / (unsigned)dm.ny);
+        j = (int)(row - (unsigned)i * (unsigned)dm.ny);
     } else {
-        k = blockIdx.x * blockDim.x + threadIdx.x;
-        j = blockIdx.y * blockDim.y + threadIdx.y;
-        i = blockIdx.z * blockDim.z + threadIdx.z;
-        in = i < dm.nx && j < dm.ny && k < dm.nz;
+        k = (int)(I0 % dm.nz);
+        j = (int)(I0 / dm.nz % dm.ny);
+        i = (int)(I0 / dm.nz / dm.ny);
     }
     if (!COUNT && !in) return;
     unsigned bad = 0, tot = 0;
@@ -360,37 +387,141 @@ __global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, 
         else
             g[I] = D::third(g[I] + 2 * (u2[I] - L));
     }
-    if (COUNT) {
-        for (int o = 16; o > 0; o >>= 1) {
-            bad += __shfl_down_sync(0xffffffffu, bad, o);
-            tot += __shfl_down_sync(0xffffffffu, tot, o);
-            acc += __shfl_down_sync(0xffffffffu, acc, o);
-        }
-        __shared__ unsigned sb[8], st[8];
-        __shared__ double sa[8];
-        const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-        if ((tid & 31) == 0) {
-            sb[tid >> 5] = bad;
-            st[tid >> 5] = tot;
-            sa[tid >> 5] = acc;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            unsigned B = 0, Tt = 0;
-            double A = 0;
-            const int nw = (blockDim.x * blockDim.y * blockDim.z + 31) >> 5;
-            for (int w = 0; w < nw; ++w) {
-                B += sb[w];
-                Tt += st[w];
-                A += sa[w];
+    if (COUNT) count_block(bad, tot, acc, counts, accum);
+}
+
+// weno5<float> for two cells at once: the same operations, in the order and with the contractions into
+// fused multiply-adds that the scalar form compiles to, so both give the same bits.
+struct Weno2 {
+    f2 r12, r3, r6, mr3, mr6, rh;
+    __device__ explicit Weno2(float h) {
+        const float q3 = __fdividef(1.0f, 3.0f), q6 = __fdividef(1.0f, 6.0f);
+        r12 = k2(__fdividef(1.0f, 12.0f));
+        r3 = k2(q3);
+        r6 = k2(q6);
+        mr3 = k2(-q3);
+        mr6 = k2(-q6);
+        rh = k2(__fdividef(1.0f, h));
+    }
+    __device__ static f2 k2(float v) { return pk2(v, v); }
+    __device__ static f2 sub(f2 a, f2 b) { return fma2(b, k2(-1.0f), a); }  // one rounding, as a - b
+    __device__ static f2 rcp(f2 v) {
+        // __fdividef(1, x)'s value (both are 0 from 2^126 up; the operands are 1e-12 and more) without its scaling
+        const float2 x = up2(v);
+        float2 y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(x.x));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(x.y));
+        return pk2(y.x, y.y);
+    }
+    // 13 u u + 3 v v; the signs of u and v do not matter
+    __device__ static f2 ind(f2 u, f2 v) { return fma2(mul2(k2(13.0f), u), u, mul2(mul2(k2(3.0f), v), v)); }
+    // one side: p3 = w_0 X and p6 = (w_2 - 1/2) Y, to be added to df over 3 and 6
+    __device__ static void side(f2 s0, f2 s1, f2 s2, f2 X, f2 Y, f2 &p3, f2 &p6) {
+        const f2 e = k2(1e-6f);
+        const f2 t0 = add2(e, s0), t1 = add2(e, s1), t2 = add2(e, s2);
+        const f2 a0 = rcp(mul2(t0, t0)), r1 = rcp(mul2(t1, t1)), r2 = rcp(mul2(t2, t2));
+        const f2 a2 = mul2(k2(3.0f), r2), w1 = rcp(add2(a2, fma2(k2(6.0f), r1, a0)));
+        p3 = mul2(mul2(a0, w1), X);
+        p6 = mul2(fma2(a2, w1, k2(-0.5f)), Y);
+    }
+    __device__ void operator()(const f2 w[7], f2 &up, f2 &un) const {
+        const f2 mb = sub(w[1], w[2]), c1 = sub(w[3], w[2]), d1 = sub(w[4], w[3]), e1 = sub(w[5], w[4]);
+        const f2 df = mul2(sub(fma2(k2(7.0f), add2(c1, d1), mb), e1), r12);
+        const f2 b1 = sub(w[2], w[1]);
+        const f2 a = sub(b1, sub(w[1], w[0])), b = sub(c1, b1), c = sub(d1, c1), d = sub(e1, d1),
+                 e = sub(sub(w[6], w[5]), e1);
+        const f2 m3 = k2(-3.0f), m2 = k2(-2.0f);
+        const f2 dc = sub(d, c), cb = sub(c, b);
+        f2 q3, q6;
+        side(ind(sub(e, d), fma2(m3, d, e)), ind(dc, add2(d, c)), ind(cb, fma2(m3, c, b)), add2(fma2(m2, d, e), c),
+             add2(fma2(m2, c, d), b), q3, q6);
+        up = mul2(fma2(q6, r6, fma2(q3, r3, df)), rh);
+        side(ind(sub(a, b), fma2(m3, b, a)), ind(cb, add2(b, c)), ind(dc, fma2(m3, c, d)), add2(fma2(m2, b, a), c),
+             add2(fma2(m2, c, b), d), q3, q6);
+        un = mul2(fma2(q6, mr6, fma2(q3, mr3, df)), rh);
+    }
+};
+
+// k_weno_stage for FP32 grids: a thread takes two cells along k as register pairs (half the instructions
+// of the WENO arithmetic, one set of row addresses for both).  The scalar stage issued 870 instructions a cell at
+// 76 % of the issue slots: 93 -> 64 us a stage on a 158^3 grid (3.9 M cells).
+template <int MODE, int STAGE, bool COUNT = false>
+__global__ void __launch_bounds__(256) k_weno_stage32(Dims dm, float h, float dtv, float eps,
+                                                      const float *__restrict__ src, float *g, float *u1, float *u2,
+                                                      const float *__restrict__ phi0, float band = 0.f,
+                                                      float thres = 0.f, unsigned long long *counts = nullptr,
+                                                      double *accum = nullptr) {
+    using T = float;
+    using D = Div32;
+    const int k0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.z * blockDim.z + threadIdx.z;
+    const bool in = i < dm.nx && j < dm.ny && k0 < dm.nz;
+    if (!COUNT && !in) return;
+    unsigned bad = 0, tot = 0;
+    double acc = 0.;
+    if (in) {
+        const int k1 = min(k0 + 1, dm.nz - 1);
+        const Weno2 weno(h);
+        f2 w[7], up2_[3], un2_[3];
+        const float *row = src + dm.idx(i, j, 0);
+        float v[8];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) v[l] = __ldg(row + min(max(k0 - 3 + l, 0), dm.nz - 1));
+        const f2 mid = pk2(v[3], v[4]);
+#pragma unroll
+        for (int l = 0; l < 7; ++l) w[l] = pk2(v[l], v[l + 1]);
+        weno(w, up2_[2], un2_[2]);
+#pragma unroll
+        for (int ax = 0; ax < 2; ++ax) {
+#pragma unroll
+            for (int l = 0; l < 7; ++l) {
+                if (l == 3) {
+                    w[l] = mid;
+                    continue;
+                }
+                const float *r = src + (ax == 0 ? dm.idx(min(max(i - 3 + l, 0), dm.nx - 1), j, 0)
+                                                : dm.idx(i, min(max(j - 3 + l, 0), dm.ny - 1), 0));
+                w[l] = pk2(__ldg(r + k0), __ldg(r + k1));
             }
-            if (Tt) {
-                atomicAdd(counts, (unsigned long long)B);
-                atomicAdd(counts + 1, (unsigned long long)Tt);
-                atomicAdd(accum, A);
+            weno(w, up2_[ax], un2_[ax]);
+        }
+        const long I0 = dm.idx(i, j, k0);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (k0 + c >= dm.nz) break;
+            T up[3], un[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float2 p = up2(up2_[a]), n = up2(un2_[a]);
+                up[a] = c ? p.y : p.x;
+                un[a] = c ? n.y : n.x;
             }
+            const long I = I0 + c;
+            T L;
+            if (MODE == 0) {
+                L = dtv * godunov(un, up);
+            } else {
+                const T p0 = phi0[I];
+                const T sign = D::over_sqrt(p0, p0 * p0 + eps);
+                const T nd = sign > (T)0 ? godunov(un, up) : godunov(up, un);
+                L = dtv * sign * (nd - (T)1.0);
+            }
+            if (COUNT && fabs(src[I]) < band) {
+                const T nr = godunov(un, up);
+                tot += 1;
+                bad += fabs(nr - (T)1.0) > thres ? 1u : 0u;
+                acc += fabs((double)nr - 1.0);
+            }
+            if (STAGE == 0)
+                u1[I] = g[I] - L;
+            else if (STAGE == 1)
+                u2[I] = (3 * g[I] + u1[I] - L) * (T)0.25;
+            else
+                g[I] = D::third(g[I] + 2 * (u2[I] - L));
         }
     }
+    if (COUNT) count_block(bad, tot, acc, counts, accum);
 }
 
 // levelset::countGradient: among cells with |g| < thickness*dx, count | |grad g| - 1 | > thres.
@@ -769,11 +900,17 @@ inline dim3 stencil_grid(const Grid &g) {
     dim3 b = stencil_block();
     return dim3(div_up(g.nz, b.x), div_up(g.ny, b.y), div_up(g.nx, b.z));
 }
-// Launch shape of k_weno_stage<T> over nx x ny x nz cells.
+// Launch shape of a stage over nx x ny x nz cells (FP32: 32 cells along k a block row).
 template <class T> inline void stage_shape(int nx, int ny, int nz, dim3 &gr, dim3 &bl) {
-    bl = sizeof(T) == 8 ? dim3(256) : stencil_block();
+    bl = sizeof(T) == 8 ? dim3(256) : dim3(16, 4, 4);
     gr = sizeof(T) == 8 ? dim3((unsigned)(((long)nx * ny * nz + 255) / 256))
-                        : dim3(div_up(nz, bl.x), div_up(ny, bl.y), div_up(nx, bl.z));
+                        : dim3(div_up(nz, 2 * bl.x), div_up(ny, bl.y), div_up(nx, bl.z));
+}
+template <int MODE, int STAGE, class T, bool COUNT = false> auto stage_kernel() {
+    if constexpr (sizeof(T) == 8)
+        return k_weno_stage<MODE, STAGE, T, COUNT>;
+    else
+        return k_weno_stage32<MODE, STAGE, COUNT>;
 }
 inline Dims dims_of(const Grid &g) { return Dims{g.nx, g.ny, g.nz}; }
 
@@ -816,9 +953,9 @@ void evolve_t(Grid &g, double final_t, double vel, double cfl) {
     T *G = gdata<T>(g);
     const double fl = 350.0 * g.cells(), by = 3.0 * sizeof(T) * g.cells();
     for (int st = 0; st < steps; ++st) {
-        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), k_weno_stage<0, 0, T><<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, G, G, u1.ptr, u2.ptr, nullptr)); }
-        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), k_weno_stage<0, 1, T><<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, u1.ptr, G, u1.ptr, u2.ptr, nullptr)); }
-        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), k_weno_stage<0, 2, T><<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, u2.ptr, G, u1.ptr, u2.ptr, nullptr)); }
+        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), stage_kernel<0, 0, T>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, G, G, u1.ptr, u2.ptr, nullptr, (T)0, (T)0, nullptr, nullptr)); }
+        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), stage_kernel<0, 1, T>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, u1.ptr, G, u1.ptr, u2.ptr, nullptr, (T)0, (T)0, nullptr, nullptr)); }
+        { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), stage_kernel<0, 2, T>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)0, u2.ptr, G, u1.ptr, u2.ptr, nullptr, (T)0, (T)0, nullptr, nullptr)); }
     }
     IBIM_CHECK_LAUNCH();
 }
@@ -864,7 +1001,7 @@ int reinit_t(Grid &g, const Grid &phi0, double final_t, double vel, double cfl, 
             acc.zero();
             {
                 ProfScope ps_(PROF_WENO, fl, by);
-                (count_launch(), k_weno_stage<1, 0, T, true><<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, G, G, u1.ptr, u2.ptr,
+                (count_launch(), stage_kernel<1, 0, T, true>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, G, G, u1.ptr, u2.ptr,
                                                                               P0, band, th, cnt.ptr, acc.ptr));
             }
             IBIM_CHECK_LAUNCH();
@@ -872,8 +1009,8 @@ int reinit_t(Grid &g, const Grid &phi0, double final_t, double vel, double cfl, 
             IBIM_CUDA(cudaStreamSynchronize(s));
             if (hcnt[0] == 0 || step >= steps) break;
             step++;
-            { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), k_weno_stage<1, 1, T><<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, u1.ptr, G, u1.ptr, u2.ptr, P0)); }
-            { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), k_weno_stage<1, 2, T><<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, u2.ptr, G, u1.ptr, u2.ptr, P0)); }
+            { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), stage_kernel<1, 1, T>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, u1.ptr, G, u1.ptr, u2.ptr, P0, (T)0, (T)0, nullptr, nullptr)); }
+            { ProfScope ps_(PROF_WENO, fl, by); (count_launch(), stage_kernel<1, 2, T>()<<<gr, bl, 0, s>>>(dm, h, dtv, (T)eps, u2.ptr, G, u1.ptr, u2.ptr, P0, (T)0, (T)0, nullptr, nullptr)); }
         }
     } catch (...) {
         cudaFreeHost(hcnt);
