@@ -859,19 +859,24 @@ int ibim_fmm_apply(ibim_plan p, int kernel, const ibim_kernel_params *kp, const 
         DevBuf<double> hin;
         hin.alloc((size_t)rows * ns, s);
         hin.upload(in, (size_t)rows * ns);
-        P.dens4.zero();
+        const bool one = rows == 1 && fmm_one_entry(P);  // the kernel's own entry of the block alone
+        if (!one) P.dens4.zero();
         if (rows == 4) {
             for (int d = 0; d < 4; ++d) permute(c, ns, P.src_perm.ptr, hin.ptr + d * ns, P.dens4.ptr + d * ns, false);
         } else {
-            permute(c, ns, P.src_perm.ptr, hin.ptr, P.dens4.ptr + kKernelMap[kernel].slot * ns, false);
+            permute(c, ns, P.src_perm.ptr, hin.ptr, P.dens4.ptr + (one ? 0 : kKernelMap[kernel].slot * ns),
+                    false);
         }
-        fmm_run(P, 0, *kp, P.dens4.ptr, S.out4.ptr, P.precision);
+        if (one)
+            fmm_run_entry(P, 0, *kp, P.dens4.ptr, S.out4.ptr, 4 * kKernelMap[kernel].field + kKernelMap[kernel].slot);
+        else
+            fmm_run(P, 0, *kp, P.dens4.ptr, S.out4.ptr, P.precision);
         DevBuf<double> hout;
         hout.alloc((size_t)rows * nt, s);
         if (rows == 4) {
             for (int d = 0; d < 4; ++d) permute(c, nt, S.perm_d.ptr, S.out4.ptr + d * nt, hout.ptr + d * nt, true);
         } else {
-            permute(c, nt, S.perm_d.ptr, S.out4.ptr + kKernelMap[kernel].field * nt, hout.ptr, true);
+            permute(c, nt, S.perm_d.ptr, S.out4.ptr + (one ? 0 : kKernelMap[kernel].field * nt), hout.ptr, true);
         }
         hout.download(out, (size_t)rows * nt);
         sync_checked(P);

@@ -67,13 +67,15 @@ void cheb_tables_host(int p, ChebTables &T) {
 
 namespace {
 
+// The translations take nc components a node: 4 for the fused block, 1 for one scalar kernel.
+
 // P2M (upPass leaf, bbfmm.h:507-519): mult[leaf][d][c] = sum_pts S(pt, c) dens[d][pt].
 __global__ void __launch_bounds__(128) k_p2m64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
                                                const int *__restrict__ sb, const int *__restrict__ se,
                                                const double *__restrict__ ctr, const double *__restrict__ rad,
                                                const double *__restrict__ x, const double *__restrict__ y,
                                                const double *__restrict__ z, const double *__restrict__ dens, long ns,
-                                               double *mult) {
+                                               int nc, double *mult) {
     __shared__ ChebTables T;
     __shared__ double Sp[32][3][MAXP];
     __shared__ double D[4][32];
@@ -100,12 +102,12 @@ __global__ void __launch_bounds__(128) k_p2m64(const ChebTables *__restrict__ ta
         } else if (threadIdx.x < 128) {
             const int pt = threadIdx.x - 96;
             if (pt < cnt)
-                for (int d = 0; d < 4; ++d) D[d][pt] = dens[d * ns + base + pt];
+                for (int d = 0; d < nc; ++d) D[d][pt] = dens[d * ns + base + pt];
         }
         __syncthreads();
         for (int q = 0; q < 16; ++q) {
             const int o = threadIdx.x + 128 * q;
-            if (o >= 4 * R) break;
+            if (o >= nc * R) break;
             const int d = o / R, cc = o % R;
             const int i = cc % p, j = (cc / p) % p, l = cc / (p * p);
             double s = acc[q];
@@ -116,14 +118,14 @@ __global__ void __launch_bounds__(128) k_p2m64(const ChebTables *__restrict__ ta
     }
     for (int q = 0; q < 16; ++q) {
         const int o = threadIdx.x + 128 * q;
-        if (o >= 4 * R) break;
-        mult[(long)node * 4 * R + o] = acc[q];
+        if (o >= nc * R) break;
+        mult[(long)node * nc * R + o] = acc[q];
     }
 }
 
 // One separable Kronecker transfer (R[id] = S[b2] (x) S[b1] (x) S[b0], bbfmm.h:345-366) on a
-// [4][p^3] block in shared memory.  up = true: child -> parent (R^T), else parent -> child (R).
-__device__ void kron_apply(const ChebTables &T, int id, bool up, double *buf, double *tmp, int nthreads) {
+// [nc][p^3] block in shared memory.  up = true: child -> parent (R^T), else parent -> child (R).
+__device__ void kron_apply(const ChebTables &T, int nc, int id, bool up, double *buf, double *tmp, int nthreads) {
     const int p = T.p, R = T.R;
     const int b[3] = {id & 1, (id >> 1) & 1, (id >> 2) & 1};
     // axis 0 (x, stride 1), axis 1 (y, stride p), axis 2 (z, stride p^2)
@@ -131,7 +133,7 @@ __device__ void kron_apply(const ChebTables &T, int id, bool up, double *buf, do
         const int stride = ax == 0 ? 1 : (ax == 1 ? p : p * p);
         double *src = (ax & 1) ? tmp : buf;
         double *dst = (ax & 1) ? buf : tmp;
-        for (int o = threadIdx.x; o < 4 * R; o += nthreads) {
+        for (int o = threadIdx.x; o < nc * R; o += nthreads) {
             const int d = o / R, cc = o % R;
             const int idx = (cc / stride) % p;
             const int base = d * R + cc - idx * stride;
@@ -151,13 +153,13 @@ __device__ void kron_apply(const ChebTables &T, int id, bool up, double *buf, do
 // M2M (upPass, bbfmm.h:530-534): parent = sum over non-empty children R[i]^T child.
 __global__ void __launch_bounds__(128) k_m2m64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
                                                const int *__restrict__ child_first, const int *__restrict__ empty,
-                                               double *mult) {
+                                               int nc, double *mult) {
     extern __shared__ double sm[];
     __shared__ ChebTables T;
     for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
         reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
     __syncthreads();
-    const int R = T.R, n4 = 4 * R;
+    const int R = T.R, n4 = nc * R;
     double *buf = sm, *tmp = sm + n4, *acc = sm + 2 * n4;
     const int node = nodes[blockIdx.x];
     for (int o = threadIdx.x; o < n4; o += blockDim.x) acc[o] = 0.;
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(128) k_m2m64(const ChebTables *__restrict__ ta
         __syncthreads();
         for (int o = threadIdx.x; o < n4; o += blockDim.x) buf[o] = mult[(long)ch * n4 + o];
         __syncthreads();
-        kron_apply(T, c8, true, buf, tmp, blockDim.x);
+        kron_apply(T, nc, c8, true, buf, tmp, blockDim.x);
         for (int o = threadIdx.x; o < n4; o += blockDim.x) acc[o] += tmp[o];
     }
     __syncthreads();
@@ -178,19 +180,19 @@ __global__ void __launch_bounds__(128) k_m2m64(const ChebTables *__restrict__ ta
 // L2L (downPass, bbfmm.h:566-567): child += R[index8] parent.
 __global__ void __launch_bounds__(128) k_l2l64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
                                                const int *__restrict__ parent, const int *__restrict__ index8,
-                                               double *local) {
+                                               int nc, double *local) {
     extern __shared__ double sm[];
     __shared__ ChebTables T;
     for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
         reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
     __syncthreads();
-    const int R = T.R, n4 = 4 * R;
+    const int R = T.R, n4 = nc * R;
     double *buf = sm, *tmp = sm + n4;
     const int node = nodes[blockIdx.x];
     const int par = parent[node];
     for (int o = threadIdx.x; o < n4; o += blockDim.x) buf[o] = local[(long)par * n4 + o];
     __syncthreads();
-    kron_apply(T, index8[node], false, buf, tmp, blockDim.x);
+    kron_apply(T, nc, index8[node], false, buf, tmp, blockDim.x);
     for (int o = threadIdx.x; o < n4; o += blockDim.x) local[(long)node * n4 + o] += tmp[o];
 }
 
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(128) k_l2l64(const ChebTables *__restrict__ ta
 // -> K[col * 4R + row], row = out * R + ct, col = in * R + cs,
 // entry = block(src_cheb(cs) - tgt_cheb(ct))[out][in], node positions D r_t + r_s cheb - r_t cheb.
 // V operators (same level, D = 2 o) and X operators (coarser source leaf) share the layout.
+// One entry of the block (entry = 4 out + in) gives R x R operators K[cs * R + ct].
 __device__ __forceinline__ void op_geometry(const int *keys, int op, const double *root_r, double rt[3], double rs[3],
                                             int D[3]) {
     const int lt = keys[5 * op], ls = keys[5 * op + 1];
@@ -212,7 +215,7 @@ __device__ __forceinline__ void op_geometry(const int *keys, int op, const doubl
 }
 
 __global__ void k_make_ops64(const ChebTables *__restrict__ tab, const int *__restrict__ keys,
-                             const double *__restrict__ root_r, KParams kp, double *ops) {
+                             const double *__restrict__ root_r, KParams kp, int entry, double *ops) {
     const ChebTables &T = *tab;
     const int op = blockIdx.y;
     const int p = T.p, R = T.R, n4 = 4 * R;
@@ -230,6 +233,13 @@ __global__ void k_make_ops64(const ChebTables *__restrict__ tab, const int *__re
     for (int a = 0; a < 3; ++a) d[a] = (D[a] * rt[a] + rs[a] * T.cheb[si[a]]) - rt[a] * T.cheb[ti[a]];
     double b[16];
     kblock64(kp, d[0], d[1], d[2], b);
+    if (entry != ENTRY_BLOCK) {
+        double v = b[0];
+#pragma unroll
+        for (int i = 1; i < 16; ++i) v = i == entry ? b[i] : v;
+        ops[(long)op * R * R + pair] = v;
+        return;
+    }
     double *K = ops + (long)op * n4 * n4;
     for (int o = 0; o < 4; ++o)
         for (int in = 0; in < 4; ++in) K[(long)(in * R + cs) * n4 + (o * R + ct)] = b[o * 4 + in];
@@ -365,11 +375,27 @@ __device__ __forceinline__ double near64_f64(float v) {
     return __hiloint2double((b >> 3) + 0x38000000, b << 29);
 }
 
+// t = kappa r and e = e^-t = 2^{-n/128} 2^{-g}: n from the FP32 r, g exact, |g| < 2^-7.8, Taylor to degree 5
+// (below 2^-58).
+__device__ __forceinline__ void near64_exp(const Near64K &k, const double2 *__restrict__ e2, double r, float rf, double &t,
+                                           double &e) {
+    t = k.kappa * r;
+    const float xm = fminf(rf * k.klt, 128000.f) + 12582912.f;  // n in the low bits
+    const int n = __float_as_int(xm) - 0x4b400000;
+    const double g = fma(k.kl, r, -near64_f64((xm - 12582912.f) * (1.f / NEAR_EXP)));
+    double q = fma(g, -1.3333558146428443e-3, 9.6181291076284772e-3);
+    q = fma(g, q, -5.5504108664821580e-2);
+    q = fma(g, q, 2.4022650695910072e-1);
+    q = fma(g, q, -6.9314718055994531e-1) * g;
+    const double2 tb = e2[n & (NEAR_EXP - 1)];
+    const double ef = tb.x + fma(tb.x, q, tb.y);
+    e = n >= 128000 ? 0.0 : __hiloint2double(__double2hiint(ef) - ((n / NEAR_EXP) << 20), __double2loint(ef));
+}
+
 // One source -> target update of the fused block (kblock64's formulas) for d2 >= vr2, with
 // M = d.m / r^3 shared by K1 and K3, psi staged times q4pi / k3f, and the factors q4pi (F) and
 // k3f (G) left to the caller.  1 / r: FP32 seed y (relative error below 2^-22), then
 // y (1 + e/2 + 3 e^2/8) with e = 1 - d2 y^2, whose error is about 5/16 e^3 < 2^-64.
-// e^{-kappa r} = 2^{-n/128} 2^{-g}: n from FP32, g exact, |g| < 2^-7.8, Taylor to degree 5 (below 2^-58).
 template <int MODE>
 __device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__restrict__ e2, double dx, double dy,
                                             double dz, double m0, double m1, double m2, double psi, double acc[4]) {
@@ -395,18 +421,8 @@ __device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__r
         acc[3] = fma(dz, w, acc[3]);
         return;
     }
-    const double r = d2 * ir, t = k.kappa * r;
-    const float xm = fminf(d2f * yf * k.klt, 128000.f) + 12582912.f;  // n in the low bits
-    const int n = __float_as_int(xm) - 0x4b400000;
-    const double g = fma(k.kl, r, -near64_f64((xm - 12582912.f) * (1.f / NEAR_EXP)));
-    double q = fma(g, -1.3333558146428443e-3, 9.6181291076284772e-3);
-    q = fma(g, q, -5.5504108664821580e-2);
-    q = fma(g, q, 2.4022650695910072e-1);
-    q = fma(g, q, -6.9314718055994531e-1) * g;
-    const double2 tb = e2[n & (NEAR_EXP - 1)];
-    const double ef = tb.x + fma(tb.x, q, tb.y);
-    const double e = n >= 128000 ? 0.0
-                                 : __hiloint2double(__double2hiint(ef) - ((n / NEAR_EXP) << 20), __double2loint(ef));
+    double t, e;
+    near64_exp(k, e2, d2 * ir, d2f * yf, t, e);
     const double et1 = fma(e, t, e);
     acc[0] = fma(fma(k.eps, et1, -1.0), M, acc[0]);
     acc[0] = fma(-(fma(-k.sk, e, k.sk) * ir), psi, acc[0]);
@@ -418,19 +434,59 @@ __device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__r
     acc[3] = fma(dz, cm, fma(hd, m2, acc[3]));
 }
 
-template <int MODE>
+// One scalar kernel's update, an entry of the block above by the same steps (26 to 31 FP64 instructions
+// screened, 12 not): a and b are the axes of the dipole (K1, K3) and of the gradient (K3, K4).
+enum { NEAR_BLOCK = 0, NEAR_K1 = 1, NEAR_K2 = 2, NEAR_K3 = 3, NEAR_K4 = 4 };
+template <int MODE, int KIND>
+__device__ __forceinline__ double near64_one(const Near64K &k, const double2 *__restrict__ e2, double dx, double dy,
+                                             double dz, int a, int b, double m, double acc) {
+    const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const double da = a == 0 ? dx : (a == 1 ? dy : dz), db = b == 0 ? dx : (b == 1 ? dy : dz);
+    if (MODE == NEAR_GENERAL) {
+        if (d2 < k.vr2) return KIND == NEAR_K2 ? fma(-k.kp.k2in, m, acc) : acc;
+        double c1, c4, k2, hd, ho;
+        radial64(k.kp, d2, c1, c4, k2, hd, ho);
+        if (KIND == NEAR_K1) return fma(c1, da * m, acc);
+        if (KIND == NEAR_K2) return fma(-k2, m, acc);
+        if (KIND == NEAR_K3) return fma(db, ho * (da * m), a == b ? fma(hd, m, acc) : acc);
+        return fma(db, -c4 * m, acc);
+    }
+    if (MODE == NEAR_LAPLACE && (KIND == NEAR_K2 || KIND == NEAR_K3)) return acc;
+    if (__double_as_longlong(d2) < __double_as_longlong(k.vr2)) return KIND == NEAR_K2 ? fma(-k.k2c, m, acc) : acc;
+    const float d2f = near64_f32(d2);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(d2f));
+    const double y = near64_f64(yf);
+    const double e0 = fma(-(d2 * y), y, 1.0);
+    const double ir = fma(y, fma(e0, 0.375, 0.5) * e0, y);
+    const double ir2 = ir * ir, ir3 = ir2 * ir;
+    if (MODE == NEAR_LAPLACE) return fma((KIND == NEAR_K1 ? da : db) * m, ir3, acc);
+    double t, e;
+    near64_exp(k, e2, d2 * ir, d2f * yf, t, e);
+    if (KIND == NEAR_K2) return fma(-(fma(-k.sk, e, k.sk) * ir), m, acc);
+    const double et1 = fma(e, t, e);
+    if (KIND == NEAR_K1) return fma(fma(k.eps, et1, -1.0), (da * m) * ir3, acc);
+    if (KIND == NEAR_K4) return fma(db, -fma(-k.ieps, et1, 1.0) * (ir3 * m), acc);
+    const double ho = fma(e, fma(t + 3.0, t, 3.0), -3.0);
+    if (a == b) acc = fma((1.0 - et1) * ir3, m, acc);
+    return fma(db, ho * (ir2 * ((da * m) * ir3)), acc);
+}
+
+template <int MODE, int KIND>
 __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave the M2L its own
     k_near64(const ChebTables *__restrict__ tab, const double2 *__restrict__ etab, Near64K kp, const int4 *__restrict__ segs,
              const int *__restrict__ near_range, const int *__restrict__ tb_, const int *__restrict__ te_,
              const double *__restrict__ ctr, const double *__restrict__ rad, const double *__restrict__ sx,
              const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ dens, long ns,
              const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz, long nt,
-             const double *__restrict__ local, double *out, int l2p_mask, int nseg, int *next) {
-    __shared__ double2 S[NEAR_TILE][4];  // x y | z m_x | m_y m_z | psi -
+             const double *__restrict__ local, double *out, int l2p_mask, int nseg, int *next, int ax_in, int ax_out) {
+    constexpr int NC = KIND == NEAR_BLOCK ? 4 : 1;
+    constexpr bool FG = KIND == NEAR_K1 || KIND == NEAR_K2;  // the one output is F
+    __shared__ double2 S[NEAR_TILE][NC == 4 ? 4 : 2];  // x y | z m_x | m_y m_z | psi - , one kernel: x y | z m
     __shared__ double2 e2[MODE == NEAR_YUKAWA ? NEAR_EXP : 1];  // 2^(-j / 128), high and low word
     __shared__ int cur;
-    double(*red)[4] = reinterpret_cast<double(*)[4]>(S);  // [NEAR_T][4], once the tiles are done
-    static_assert(sizeof(S) >= sizeof(double) * 4 * NEAR_T, "reduction scratch");
+    double(*red)[NC] = reinterpret_cast<double(*)[NC]>(S);  // [NEAR_T][NC], once the tiles are done
+    static_assert(sizeof(S) >= sizeof(double) * NC * NEAR_T, "reduction scratch");
     if (MODE == NEAR_YUKAWA && threadIdx.x < NEAR_EXP) e2[threadIdx.x] = etab[threadIdx.x];
     const double psi_f = MODE == NEAR_GENERAL ? 1.0 : kp.psi_f;
     // with a work counter the CTA takes segments until none is left; without one it does segment blockIdx.x
@@ -457,7 +513,7 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
             const bool active = ph < nph;
             double X = 0, Y = 0, Z = 0;
             if (active) { X = tx[t0 + my_t]; Y = ty[t0 + my_t]; Z = tz[t0 + my_t]; }
-            double acc[4] = {0., 0., 0., 0.};
+            double acc[NC] = {};
             for (int rr = r0; rr < r1; ++rr) {
                 const int b = near_range[2 * rr], e = near_range[2 * rr + 1];
                 for (int s0 = b; s0 < e; s0 += NEAR_TILE) {
@@ -467,7 +523,12 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                     const int q = threadIdx.x >> 1;
                     if (q < cnt) {
                         const long i = s0 + q;
-                        if (threadIdx.x & 1) {
+                        if constexpr (NC == 1) {
+                            if (threadIdx.x & 1)
+                                S[q][1] = make_double2(sz[i], KIND == NEAR_K2 || KIND == NEAR_K4 ? dens[i] * psi_f : dens[i]);
+                            else
+                                S[q][0] = make_double2(sx[i], sy[i]);
+                        } else if (threadIdx.x & 1) {
                             S[q][2] = make_double2(dens[ns + i], dens[2 * ns + i]);
                             S[q][3] = make_double2(dens[3 * ns + i] * psi_f, 0.);
                         } else {
@@ -478,42 +539,49 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                     __syncthreads();
                     if (active)
                         for (int q2 = ph; q2 < cnt; q2 += nph) {
-                            const double2 a0 = S[q2][0], a1 = S[q2][1], a2 = S[q2][2];
+                            const double2 a0 = S[q2][0], a1 = S[q2][1];
+                            if constexpr (NC == 1) {
+                                acc[0] = near64_one<MODE, KIND>(kp, e2, a0.x - X, a0.y - Y, a1.x - Z, ax_in, ax_out, a1.y,
+                                                                acc[0]);
+                                continue;
+                            } else {
+                            const double2 a2 = S[q2][2];
                             const double psi = S[q2][3].x;
                             if (MODE == NEAR_GENERAL)
                                 near_pair64(kp.kp, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
                             else
                                 near64_pair<MODE>(kp, e2, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
+                            }
                         }
                 }
             }
             if (MODE != NEAR_GENERAL) {
                 // without screening the pairs carry c1 = eps - 1 and -c4 = 1/eps - 1 here
-                acc[0] *= MODE == NEAR_LAPLACE ? kp.f0 * (kp.eps - 1.0) : kp.f0;
-                for (int o = 1; o < 4; ++o) acc[o] *= MODE == NEAR_LAPLACE ? kp.fg * (kp.ieps - 1.0) : kp.fg;
+                if (NC == 4 || FG) acc[0] *= MODE == NEAR_LAPLACE ? kp.f0 * (kp.eps - 1.0) : kp.f0;
+                for (int o = NC == 4 || FG ? 1 : 0; o < NC; ++o) acc[o] *= MODE == NEAR_LAPLACE ? kp.fg * (kp.ieps - 1.0) : kp.fg;
             }
             __syncthreads();  // every thread is done with the last tile
-            for (int o = 0; o < 4; ++o) red[threadIdx.x][o] = acc[o];
+            for (int o = 0; o < NC; ++o) red[threadIdx.x][o] = acc[o];
             __syncthreads();
             if (threadIdx.x < nT) {
-                double f[4] = {0., 0., 0., 0.};
+                double f[NC] = {};
                 for (int q = 0; q < nph; ++q)
-                    for (int o = 0; o < 4; ++o) f[o] += red[threadIdx.x + q * nT][o];
+                    for (int o = 0; o < NC; ++o) f[o] += red[threadIdx.x + q * nT][o];
                 // L2P (bbfmm.h:600): local expansion at the target, by the leaf's first segment
-                double l2p[4] = {0., 0., 0., 0.};
+                double l2p[NC] = {};
                 if (mode & l2p_mask & 1) {
                     const ChebTables &T = *tab;
                     double Sp[3][MAXP];
                     const double xyz[3] = {X, Y, Z};
                     for (int a = 0; a < 3; ++a) interp1(T, (xyz[a] - ctr[3 * leaf + a]) / rad[3 * leaf + a], Sp[a]);
                     const int p = T.p, R = T.R;
-                    const double *L = local + (long)leaf * 4 * R;
+                    const double *L = local + (long)leaf * NC * R;
                     for (int c = 0; c < R; ++c) {
                         const double w = Sp[0][c % p] * Sp[1][(c / p) % p] * Sp[2][c / (p * p)];
-                        for (int o = 0; o < 4; ++o) l2p[o] += w * L[o * R + c];
+                        for (int o = 0; o < NC; ++o) l2p[o] += w * L[o * R + c];
                     }
                 }
-                for (int o = 0; o < 4; ++o) {
+                for (int o = 0; o < NC; ++o) {
                     double *dst = out + o * nt + t0 + threadIdx.x;
                     if (mode & 2) atomicAdd(dst, f[o] + l2p[o]);
                     else *dst = f[o] + l2p[o];
@@ -524,9 +592,35 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
     }
 }
 
+using Near64Fn = decltype(&k_near64<NEAR_YUKAWA, NEAR_BLOCK>);
+template <int KIND> Near64Fn near64_mode(int mode) {
+    return mode == NEAR_YUKAWA ? k_near64<NEAR_YUKAWA, KIND>
+                               : (mode == NEAR_LAPLACE ? k_near64<NEAR_LAPLACE, KIND> : k_near64<NEAR_GENERAL, KIND>);
+}
+Near64Fn near64_kernel(int mode, int kind) {
+    switch (kind) {
+        case NEAR_K1: return near64_mode<NEAR_K1>(mode);
+        case NEAR_K2: return near64_mode<NEAR_K2>(mode);
+        case NEAR_K3: return near64_mode<NEAR_K3>(mode);
+        case NEAR_K4: return near64_mode<NEAR_K4>(mode);
+        default: return near64_mode<NEAR_BLOCK>(mode);
+    }
+}
+
+void near64_side_by_side(std::atomic<uint64_t> &done) {
+    side_by_side(done, {
+#define NEAR64_MODES(K) \
+    (const void *)k_near64<NEAR_GENERAL, K>, (const void *)k_near64<NEAR_YUKAWA, K>, (const void *)k_near64<NEAR_LAPLACE, K>
+                           NEAR64_MODES(NEAR_BLOCK), NEAR64_MODES(NEAR_K1), NEAR64_MODES(NEAR_K2), NEAR64_MODES(NEAR_K3),
+                           NEAR64_MODES(NEAR_K4)
+#undef NEAR64_MODES
+                       });
+}
+
 // L2P alone (bbfmm.h:600), one target leaf per block, added to the near-field sums already in
 // `out`: the form used when the near field runs beside the far field.
 constexpr int L2P_T = 128;
+template <int NC>
 __global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ tab, const int *__restrict__ tleaf,
                                                   const int *__restrict__ tb_, const int *__restrict__ te_,
                                                   const double *__restrict__ ctr, const double *__restrict__ rad,
@@ -534,7 +628,7 @@ __global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ 
                                                   const double *__restrict__ tz, long nt,
                                                   const double *__restrict__ local, double *out) {
     __shared__ ChebTables T;
-    __shared__ double Ls[4 * MAXR];                // the leaf's local expansion
+    __shared__ double Ls[NC * MAXR];               // the leaf's local expansion
     __shared__ double W[3][L2P_T][MAXP + 1];      // per-thread interpolation weights (odd stride)
     for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
         reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
@@ -542,14 +636,14 @@ __global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ 
     const int tb = tb_[leaf], te = te_[leaf];
     __syncthreads();
     const int p = T.p, R = p * p * p;
-    for (int i = threadIdx.x; i < 4 * R; i += blockDim.x) Ls[i] = local[(long)leaf * 4 * R + i];
+    for (int i = threadIdx.x; i < NC * R; i += blockDim.x) Ls[i] = local[(long)leaf * NC * R + i];
     __syncthreads();
     double *w0 = W[0][threadIdx.x], *w1 = W[1][threadIdx.x], *w2 = W[2][threadIdx.x];
     for (int t = tb + threadIdx.x; t < te; t += blockDim.x) {
         interp1(T, (tx[t] - ctr[3 * leaf]) / rad[3 * leaf], w0);
         interp1(T, (ty[t] - ctr[3 * leaf + 1]) / rad[3 * leaf + 1], w1);
         interp1(T, (tz[t] - ctr[3 * leaf + 2]) / rad[3 * leaf + 2], w2);
-        double l2p[4] = {0., 0., 0., 0.};
+        double l2p[NC] = {};
         int c = 0;
         for (int c2 = 0; c2 < p; ++c2) {
             const double s2 = w2[c2];
@@ -558,11 +652,11 @@ __global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ 
                 for (int c0 = 0; c0 < p; ++c0, ++c) {
                     const double w = w0[c0] * s1 * s2;
 #pragma unroll
-                    for (int o = 0; o < 4; ++o) l2p[o] += w * Ls[o * R + c];
+                    for (int o = 0; o < NC; ++o) l2p[o] += w * Ls[o * R + c];
                 }
             }
         }
-        for (int o = 0; o < 4; ++o) out[o * nt + t] += l2p[o];
+        for (int o = 0; o < NC; ++o) out[o * nt + t] += l2p[o];
     }
 }
 
@@ -1189,10 +1283,10 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
             IBIM_CUDA(cudaFuncSetAttribute(k_m2m64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
             IBIM_CUDA(cudaFuncSetAttribute(k_l2l64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
         }
-        static std::atomic<uint64_t> split;
-        side_by_side(split, {(const void *)k_near64<NEAR_GENERAL>, (const void *)k_near64<NEAR_YUKAWA>,
-                             (const void *)k_near64<NEAR_LAPLACE>, (const void *)k_p2m64, (const void *)k_m2m64,
-                             (const void *)k_l2l64, (const void *)k_l2p64, (const void *)k_gather});
+        static std::atomic<uint64_t> split, split_near;
+        near64_side_by_side(split_near);
+        side_by_side(split, {(const void *)k_p2m64, (const void *)k_m2m64, (const void *)k_l2l64,
+                             (const void *)k_l2p64<4>, (const void *)k_l2p64<1>, (const void *)k_gather});
         const size_t sm = sizeof(double) * M2L_CH * n4;
         if (sm > 48 * 1024)
             IBIM_CUDA(cudaFuncSetAttribute(k_m2l_v64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1217,7 +1311,7 @@ void fmm_prepare_operators(Plan &P, const ibim_kernel_params &kp, int precision)
     if (precision == IBIM_PRECISION_FP64) {
         P.ops64.alloc((size_t)P.nops * n4 * n4, s);
         dim3 g(div_up((long)R * R, 256), P.nops);
-        { ProfScope ps_(PROF_OPS); (count_launch(), k_make_ops64<<<g, 256, 0, s>>>(P.tables.ptr, P.op_key.ptr, P.root_r.ptr, k, P.ops64.ptr)); }
+        { ProfScope ps_(PROF_OPS); (count_launch(), k_make_ops64<<<g, 256, 0, s>>>(P.tables.ptr, P.op_key.ptr, P.root_r.ptr, k, ENTRY_BLOCK, P.ops64.ptr)); }
         IBIM_CHECK_LAUNCH();
     } else {
         bool have64 = P.ops64_ready;
@@ -1345,54 +1439,70 @@ void near64_lists(Plan &P, TargetSet &S) {
     S.near64_ready = true;
 }
 
-// The FP64 operator's digit images: the operators in blocks of at most 1 GB, each cut and dropped.
-bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp) {
+// The FP64 operator's digit images, whole or of one entry of the block: the operators in blocks of at most
+// 1 GB, each cut and dropped.
+bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry) {
     if (!P.oz64_ok) return false;
     double key[5];
     kp_key(kp, key);
-    if (P.oz64.ready && same_key(P.oz64.key, key)) return true;
-    P.oz64.ready = false;
+    auto &Z = P.oz64[entry];
+    if (Z.ready && same_key(Z.key, key)) return true;
+    Z.ready = false;
     cudaStream_t s = P.ctx->stream;
-    const int R = P.R, n4 = 4 * R;
+    const int R = P.R, n = entry == ENTRY_BLOCK ? 4 * R : R;
     const KParams k = make_kparams(kp, P.tube->h);
-    const size_t per = (size_t)n4 * n4;
+    const size_t per = (size_t)n * n;
     const int block = (int)std::max<size_t>(1, std::min<size_t>(std::max(1, P.nops), (1UL << 30) / (8 * per)));
-    m2l_oz64_alloc(P);
+    m2l_oz64_alloc(P, entry);
     DevBuf<double> ops;
     ops.alloc(per * block, s);
     ProfScope ps_(PROF_OPS);
-    for (int o = 0; o < P.nops; o += block) {
-        const int nb = std::min(block, P.nops - o);
-        (count_launch(), k_make_ops64<<<dim3(div_up((long)R * R, 256), nb), 256, 0, s>>>(P.tables.ptr, P.op_key.ptr + 5 * o,
-                                                                                       P.root_r.ptr, k, ops.ptr));
+    // operators are blockIdx.y
+    for (int o = 0; o < P.nops; o += std::min(block, 65535)) {
+        const int nb = std::min({block, 65535, P.nops - o});
+        (count_launch(), k_make_ops64<<<dim3(div_up((long)R * R, 256), nb), 256, 0, s>>>(
+            P.tables.ptr, P.op_key.ptr + 5 * o, P.root_r.ptr, k, entry, ops.ptr));
         IBIM_CHECK_LAUNCH();
-        m2l_oz64_pack(P, ops.ptr, o, nb);
+        m2l_oz64_pack(P, entry, ops.ptr, o, nb);
     }
-    for (int i = 0; i < 5; ++i) P.oz64.key[i] = key[i];
-    P.oz64.ready = true;
+    for (int i = 0; i < 5; ++i) Z.key[i] = key[i];
+    Z.ready = true;
     return true;
 }
 
 void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp) {
-    if (!fmm_ensure_oz64_images(P, kp)) fmm_prepare_operators(P, kp, IBIM_PRECISION_FP64);
+    if (!fmm_ensure_oz64_images(P, kp, ENTRY_BLOCK)) fmm_prepare_operators(P, kp, IBIM_PRECISION_FP64);
 }
 
-// One FP64 FMM: dens (4 x ns, tree order) -> out (4 x nt of target set ts, tree order).
-void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *dens, double *out, bool m2l_sliced) {
+// A scalar kernel's FMM as its entry of the block: one component a node, R x R operators instead of 4R x 4R
+// (a sixteenth of the products, images of their own built on the first call of each kernel and kept), half
+// the near field's instructions.  150 atoms at order 6: 16.5 -> 3.3 ms a product, 40 -> 18 ms the first one.
+// Plans without room for all 16 entries' images beside the block's, without digit images, or with X pairs
+// evaluated on the fly run the block with the other densities zero.
+bool fmm_one_entry(const Plan &P) {
+    return P.precision == IBIM_PRECISION_FP64 && P.oz64_ok && P.x_as_ops && m2l_oz64_fits(P.p, P.nops, true);
+}
+
+// One FP64 FMM: dens (nc x ns, tree order) -> out (nc x nt of target set ts, tree order), nc = 4 for the block,
+// 1 for one entry of it.  m2l_sliced: the V-list M2L by exact BF16 slices and the near field in float-float (FP64-class
+// accuracy), the mixed path's refinement residual.
+static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *dens, double *out, bool m2l_sliced,
+                         int entry = ENTRY_BLOCK) {
     IBIM_REQUIRE(ts >= 0 && ts < (int)P.targets.size(), "no such target set");
     const bool use_oz = m2l_sliced && (4 * P.R + 15) / 16 * 16 <= M2L_OZ_MAXK;
     const bool use_oz64 = !m2l_sliced && P.oz64_ok;
     if (use_oz)
         fmm_ensure_oz_images(P, kpp);
     else if (use_oz64)
-        fmm_ensure_oz64_images(P, kpp);
+        fmm_ensure_oz64_images(P, kpp, entry);
     else
         fmm_prepare_operators(P, kpp, IBIM_PRECISION_FP64);
     const TargetSet &S = *P.targets[ts];
     Ctx *c = P.ctx;
     cudaStream_t s = c->stream;
     const TreeHost &T = P.tree;
-    const int R = P.R, n4 = 4 * R;
+    const int nc = entry == ENTRY_BLOCK ? 4 : 1;
+    const int R = P.R, n4 = nc * R;
     const KParams kp = make_kparams(kpp, P.tube->h);
     const size_t smem_k = sizeof(double) * 3 * n4;
     const double *tx = S.self ? P.sx.ptr : S.tx.ptr;
@@ -1425,12 +1535,16 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
         // the fast forms take FP32 seeds of d2 >= (tau h)^2 and n >= 0 of 2^-n/128
         const int mode = !(kp.vr2 >= 1e-30) ? NEAR_GENERAL
                                             : (kp.kappa > 0. ? NEAR_YUKAWA : (kp.kappa == 0. ? NEAR_LAPLACE : NEAR_GENERAL));
-        auto kern = mode == NEAR_YUKAWA ? k_near64<NEAR_YUKAWA>
-                                        : (mode == NEAR_LAPLACE ? k_near64<NEAR_LAPLACE> : k_near64<NEAR_GENERAL>);
+        const int slot = entry & 3, field = entry >> 2;
+        const int kind = entry == ENTRY_BLOCK ? NEAR_BLOCK
+                         : field == 0         ? (slot == 3 ? NEAR_K2 : NEAR_K1)
+                                              : (slot == 3 ? NEAR_K4 : NEAR_K3);
+        auto kern = near64_kernel(mode, kind);
         (count_launch(), kern<<<grid, NEAR_T, 0, st>>>(P.tables.ptr, P.exp_tab.ptr, nk, reinterpret_cast<const int4 *>(S.near_seg.ptr),
                                                        S.near_range.ptr, S.tbeg.ptr, S.tend.ptr, P.ncenter.ptr,
                                                        P.nradius.ptr, P.sx.ptr, P.sy.ptr, P.sz.ptr, dens, P.ns, tx, ty,
-                                                       tz, S.nt, P.local.ptr, out, l2p_mask, S.nnear_seg, next));
+                                                       tz, S.nt, P.local.ptr, out, l2p_mask, S.nnear_seg, next, slot,
+                                                       field - 1));
     };
     const bool overlap = near_overlap() && S.ntleaves > 0;
     if (!P.exp_tab.ptr) {
@@ -1464,7 +1578,7 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
     if (overlap) {
         if (!P.near_next.ptr) P.near_next.alloc(1, s);
         IBIM_CUDA(cudaMemsetAsync(P.near_next.ptr, 0, sizeof(int), s));
-        if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
+        if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * nc * S.nt, s));
         if (!with_m2l) fork();
     }
     try {
@@ -1472,21 +1586,21 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
             ProfScope ps_(PROF_P2M, (8.0 * R + 6.0 * P.p * P.p) * P.ns, 56.0 * P.ns);
             (count_launch(), k_p2m64<<<P.np2m, 128, 0, s>>>(P.tables.ptr, P.p2m_nodes.ptr, P.nsrc_begin.ptr,
                                                             P.nsrc_end.ptr, P.ncenter.ptr, P.nradius.ptr, P.sx.ptr,
-                                                            P.sy.ptr, P.sz.ptr, dens, P.ns, P.mult.ptr));
+                                                            P.sy.ptr, P.sz.ptr, dens, P.ns, nc, P.mult.ptr));
         }
         for (int l = T.nlevels - 1; l >= 0; --l) {
             const int b = P.m2m_level_begin[l], e = P.m2m_level_begin[l + 1];
             if (e > b) {
                 ProfScope ps_(PROF_M2M);
                 (count_launch(), k_m2m64<<<e - b, 128, smem_k, s>>>(P.tables.ptr, P.m2m_nodes.ptr + b,
-                                                                    P.nchild_first.ptr, P.nempty.ptr, P.mult.ptr));
+                                                                    P.nchild_first.ptr, P.nempty.ptr, nc, P.mult.ptr));
             }
         }
         P.local.zero();
         if (use_oz) {
             m2l_oz_run(P, S);
         } else if (use_oz64) {
-            m2l_oz64_run(P, S, beside);
+            m2l_oz64_run(P, S, entry, beside);
         } else if (S.nchunks > 0) {
             ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
                           8.0 * n4 * (2.0 * S.nvpairs + (double)n4 * P.nops));
@@ -1504,7 +1618,7 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
             if (e > b) {
                 ProfScope ps_(PROF_L2L);
                 (count_launch(), k_l2l64<<<e - b, 128, smem_k, s>>>(P.tables.ptr, S.l2l_nodes.ptr + b, P.nparent.ptr,
-                                                                    P.nindex8.ptr, P.local.ptr));
+                                                                    P.nindex8.ptr, nc, P.local.ptr));
             }
         }
     } catch (...) {
@@ -1516,17 +1630,23 @@ void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const double *
             if (side < std::min(nseg, full)) near(s, 0, std::min(nseg, full), P.near_next.ptr, false);
             IBIM_CUDA(cudaStreamWaitEvent(s, c->ev_near_join, 0));
         } else {
-            if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * 4 * S.nt, s));
+            if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * nc * S.nt, s));
             near(s, 1, nseg, nullptr, true);
         }
         if (overlap || ff) {  // the L2P runs on its own after the near field
             ProfScope ps_(PROF_L2P64, (10.0 * R + 6.0 * P.p * P.p) * S.nt, 32.0 * n4 * S.ntleaves + 88.0 * S.nt);
-            (count_launch(), k_l2p64<<<S.ntleaves, L2P_T, 0, s>>>(P.tables.ptr, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr,
+            auto kern = nc == 4 ? k_l2p64<4> : k_l2p64<1>;
+            (count_launch(), kern<<<S.ntleaves, L2P_T, 0, s>>>(P.tables.ptr, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr,
                                                                    P.ncenter.ptr, P.nradius.ptr, tx, ty, tz, S.nt,
                                                                    P.local.ptr, out));
         }
     }
     IBIM_CHECK_LAUNCH();
+}
+
+void fmm_run_entry(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int entry) {
+    IBIM_REQUIRE(fmm_one_entry(P), "the plan has no images of single kernels");
+    fmm_run_fp64(P, ts, kp, dens, out, false, entry);
 }
 
 void fmm_run(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int precision) {

@@ -315,6 +315,9 @@ Tuning tuning_for(int order, long npoints);
 // Plans made on this thread while t is set use it instead of the table; nullptr restores the table.
 void tuning_override(const Tuning *t);
 
+// The fused operator's block: entry 4 out + in of F, Gx, Gy, Gz by m_x, m_y, m_z, psi, or all of it.
+constexpr int ENTRY_BLOCK = 16;
+
 // Tree over the sources + operators + target sets.
 struct Plan {
     Ctx *ctx;
@@ -377,13 +380,16 @@ struct Plan {
     DevBuf<double> oz_sig, oz_tau;
     // the FP64 operator's own digit images (m2l_oz64_run), on FP64 plans whose images fit (oz64_ok)
     bool oz64_ok = false;
-    struct {
+    struct Oz64 {
         bool ready = false;
         double key[5] = {-1, -1, -1, -1, -1};
-        int kpad = 0, mtiles = 0, s = 8;
-        DevBuf<uint16_t> a, b;
-        DevBuf<double> sig, tau;
-    } oz64;
+        int n = 0, kpad = 0, mtiles = 0;  // rows and columns, K padded, row tiles
+        DevBuf<uint16_t> a;
+        DevBuf<double> sig;
+    } oz64[ENTRY_BLOCK + 1];               // of the block's entries (built when asked for) and of the whole block
+    int oz64_s = 8;                        // digits
+    DevBuf<uint16_t> oz64_b;               // the multipoles' digits and scales
+    DevBuf<double> oz64_tau;
     double kp64[5] = {-1, -1, -1, -1, -1}, kp32[5] = {-1, -1, -1, -1, -1};  // kernel parameters of the cached operators
     bool ops64_ready = false, ops32_ready = false;
     // a plan merged over several molecules (batch.cu): the molecule of every node and each
@@ -416,10 +422,10 @@ struct Plan {
 
 // FMM engine.  dens: 4 x ns (tree order), out: 4 x nt of target set `ts` (tree order).
 void fmm_prepare_operators(Plan &P, const ibim_kernel_params &kp, int precision);
-// m2l_sliced: the V-list M2L on the tensor cores by exact BF16 slicing (FP64-class accuracy),
-// as used for the mixed path's refinement residual; false = FP64 pipe, the reference-exact path.
-void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out,
-                  bool m2l_sliced = false);
+// One scalar kernel's FMM in FP64, an entry of the block: dens ns, out nt.  Only where fmm_one_entry: FP64 plans with
+// digit images, whose 16 entries' images fit too (else the block runs with the other densities zero).
+bool fmm_one_entry(const Plan &P);
+void fmm_run_entry(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int entry);
 void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out);
 void fmm_run(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int precision);
 
@@ -447,18 +453,18 @@ void m2l_oz_run(Plan &P, const TargetSet &S);
 // has none), whether nops of them may be kept on this device, the buffers, the cut of operators
 // [o, o + n) from FP64 ones, one contraction.
 double m2l_oz64_op_bytes(int p);
-bool m2l_oz64_fits(int p, double nops);
-void m2l_oz64_alloc(Plan &P);
-void m2l_oz64_pack(Plan &P, const double *ops, int o, int n);
+bool m2l_oz64_fits(int p, double nops, bool entries = false);  // entries: all the block's, one by one
+void m2l_oz64_alloc(Plan &P, int entry);
+void m2l_oz64_pack(Plan &P, int entry, const double *ops, int o, int n);
 // beside: called before the multipoles' split (work for another stream that has to be on the SMs before the
 // contraction's many CTAs queue for them).
-void m2l_oz64_run(Plan &P, const TargetSet &S, const std::function<void()> &beside = nullptr);
+void m2l_oz64_run(Plan &P, const TargetSet &S, int entry, const std::function<void()> &beside = nullptr);
 // Operator images for kernel parameters kp, built when missing or stale: the TF32 images (from
 // FP32 operators, which are then released) and the digit images (from the FP64 operators).
 void fmm_ensure_tc_images(Plan &P, const ibim_kernel_params &kp);
 void fmm_ensure_oz_images(Plan &P, const ibim_kernel_params &kp);
 // The FP64 operator's digit images; false when the plan has none.
-bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp);
+bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry);
 // What an FP64 matvec needs: its digit images, or the FP64 operators.
 void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp);
 // The mixed path's FP16 images and the FP64-class digit images together, from one set of

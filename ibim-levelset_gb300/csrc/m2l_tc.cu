@@ -2640,14 +2640,14 @@ void m2l_oz_run(Plan &P, const TargetSet &S) {
 // ---------------------------------------------------------------------------------------------
 static int oz64_digits(int p) { return p <= 5 ? 8 : 9; }
 
-double m2l_oz64_op_bytes(int p) {
-    if (p > 7) return 0.;
-    const int n4 = 4 * p * p * p;
+static double oz64_image_bytes(int p, int n4) {
     const double kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS, mpad = (n4 + OZ_M - 1) / OZ_M * OZ_M;
     return 2.0 * oz64_digits(p) * kpad * mpad;
 }
 
-bool m2l_oz64_fits(int p, double nops) {
+double m2l_oz64_op_bytes(int p) { return p > 7 ? 0. : oz64_image_bytes(p, 4 * p * p * p); }
+
+bool m2l_oz64_fits(int p, double nops, bool entries) {
     if (p > 7 || !m2l_tc_supported()) return false;
     if (nops <= 0.) return true;
     static std::atomic<size_t> total[64];  // each device's memory, asked for once
@@ -2659,23 +2659,24 @@ bool m2l_oz64_fits(int p, double nops) {
         IBIM_CUDA(cudaMemGetInfo(&free_b, &t));
         if (dev < 64) total[dev].store(t);
     }
-    return m2l_oz64_op_bytes(p) * nops <= t / 3.0;
+    return (entries ? ENTRY_BLOCK * oz64_image_bytes(p, p * p * p) : m2l_oz64_op_bytes(p)) * nops <= t / 3.0;
 }
 
-void m2l_oz64_alloc(Plan &P) {
+void m2l_oz64_alloc(Plan &P, int entry) {
     cudaStream_t s = P.ctx->stream;
-    auto &Z = P.oz64;
-    const int n4 = 4 * P.R;
-    Z.kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS;
-    Z.mtiles = (n4 + OZ_M - 1) / OZ_M;
-    Z.s = oz64_digits(P.p);
+    auto &Z = P.oz64[entry];
+    Z.n = entry == ENTRY_BLOCK ? 4 * P.R : P.R;
+    Z.kpad = (Z.n + OZ_KS - 1) / OZ_KS * OZ_KS;
+    Z.mtiles = (Z.n + OZ_M - 1) / OZ_M;
+    P.oz64_s = oz64_digits(P.p);
     const size_t stages = Z.kpad / OZ_KS, rows = (size_t)P.nops * Z.mtiles;
-    if (Z.a.n != rows * stages * Z.s * (OZ_ATILE / 2)) {
-        Z.a.alloc(rows * stages * Z.s * (OZ_ATILE / 2), s);
+    if (Z.a.n != rows * stages * P.oz64_s * (OZ_ATILE / 2)) {
+        Z.a.alloc(rows * stages * P.oz64_s * (OZ_ATILE / 2), s);
         Z.sig.alloc(rows * OZ_M, s);
-        Z.b.alloc((size_t)P.tree.nnodes * stages * Z.s * OZ_KS, s);
-        Z.tau.alloc((size_t)P.tree.nnodes, s);
     }
+    const size_t nb = (size_t)P.tree.nnodes * stages * P.oz64_s * OZ_KS;
+    if (P.oz64_b.n < nb) P.oz64_b.alloc(nb, s);
+    if (P.oz64_tau.n < (size_t)P.tree.nnodes) P.oz64_tau.alloc((size_t)P.tree.nnodes, s);
     if (!P.tc_err.ptr) {
         P.tc_err.alloc(1, s);
         P.tc_err.zero();
@@ -2687,10 +2688,10 @@ void m2l_oz64_alloc(Plan &P) {
                          (const void *)k_split_mult_oz<9>});
 }
 
-void m2l_oz64_pack(Plan &P, const double *ops, int o, int n) {
+void m2l_oz64_pack(Plan &P, int entry, const double *ops, int o, int n) {
     cudaStream_t s = P.ctx->stream;
-    auto &Z = P.oz64;
-    const int n4 = 4 * P.R, D = Z.s == 8 ? OzShape<8>::D : OzShape<9>::D;
+    auto &Z = P.oz64[entry];
+    const int n4 = Z.n, D = P.oz64_s == 8 ? OzShape<8>::D : OzShape<9>::D;
     const long rows = (long)n * Z.mtiles * OZ_M;
     DevBuf<int> sexp;
     sexp.alloc((size_t)rows, s);
@@ -2699,27 +2700,28 @@ void m2l_oz64_pack(Plan &P, const double *ops, int o, int n) {
     const size_t row0 = (size_t)o * Z.mtiles;
     (count_launch(), k_scale_ops_oz<double><<<gs, 256, 0, s>>>(n4, Z.mtiles, n, 2 * D, ops, Z.sig.ptr + row0 * OZ_M,
                                                                sexp.ptr));
-    uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr + row0 * (Z.kpad / OZ_KS) * Z.s * (OZ_ATILE / 2));
-    auto kern = Z.s == 8 ? k_pack_ops_oz<8, double> : k_pack_ops_oz<9, double>;
+    uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr + row0 * (Z.kpad / OZ_KS) * P.oz64_s * (OZ_ATILE / 2));
+    auto kern = P.oz64_s == 8 ? k_pack_ops_oz<8, double> : k_pack_ops_oz<9, double>;
     (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr));
     IBIM_CHECK_LAUNCH();
 }
 
-void m2l_oz64_run(Plan &P, const TargetSet &S, const std::function<void()> &beside) {
+void m2l_oz64_run(Plan &P, const TargetSet &S, int entry, const std::function<void()> &beside) {
     if (S.nchunks_oz64 == 0) return;
     cudaStream_t s = P.ctx->stream;
-    auto &Z = P.oz64;
-    const int n4 = 4 * P.R;
+    auto &Z = P.oz64[entry];
+    const int n4 = Z.n, ns = P.oz64_s;
     ProfScope ps_(PROF_M2L_V64, 2.0 * n4 * (double)n4 * S.nvpairs,
-                  2.0 * Z.s * Z.kpad * ((double)Z.mtiles * OZ_M * P.nops + (double)S.nvpairs));
+                  2.0 * ns * Z.kpad * ((double)Z.mtiles * OZ_M * P.nops + (double)S.nvpairs));
     if (beside) beside();
-    auto split = Z.s == 8 ? k_split_mult_oz<8> : k_split_mult_oz<9>;
-    (count_launch(), split<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, Z.kpad, P.mult.ptr, Z.b.ptr, Z.tau.ptr));
-    auto kern = Z.s == 8 ? k_m2l_oz<8> : k_m2l_oz<9>;
-    const int smem = Z.s == 8 ? OzShape<8>::SMEM : OzShape<9>::SMEM;
+    auto split = ns == 8 ? k_split_mult_oz<8> : k_split_mult_oz<9>;
+    (count_launch(), split<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, Z.kpad, P.mult.ptr, P.oz64_b.ptr,
+                                                                P.oz64_tau.ptr));
+    auto kern = ns == 8 ? k_m2l_oz<8> : k_m2l_oz<9>;
+    const int smem = ns == 8 ? OzShape<8>::SMEM : OzShape<9>::SMEM;
     (count_launch(), kern<<<dim3(S.nchunks_oz64, Z.mtiles), OZ_THREADS, smem, s>>>(
-        n4, Z.kpad, Z.mtiles, S.v_chunk_oz64.ptr, S.v_src.ptr, S.v_tgt.ptr, Z.a.ptr, Z.sig.ptr, Z.b.ptr, Z.tau.ptr,
-        P.local.ptr, P.tc_err.ptr, nullptr, nullptr, nullptr));
+        n4, Z.kpad, Z.mtiles, S.v_chunk_oz64.ptr, S.v_src.ptr, S.v_tgt.ptr, Z.a.ptr, Z.sig.ptr, P.oz64_b.ptr,
+        P.oz64_tau.ptr, P.local.ptr, P.tc_err.ptr, nullptr, nullptr, nullptr));
     IBIM_CHECK_LAUNCH();
 }
 
