@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libibim_gb300.so")
-SOURCES = ["levelset.cu", "tree.cpp", "fmm.cu", "fmm_mixed.cu", "near_ff.cu", "m2l_tc.cu", "solve.cu", "capi.cu",
+SOURCES = ["levelset.cu", "tree.cpp", "fmm.cu", "fmm_mixed.cu", "near_ff.cu", "translate.cu", "m2l_tc.cu", "solve.cu", "capi.cu",
            "server.cpp", "batch.cu", "tuning.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 OPENMP_CU = {"fmm.cu", "fmm_mixed.cu"}  # CUDA files whose host code (plan building) uses OpenMP

@@ -388,15 +388,14 @@ Plan *merge_wave(Ctx *c, Tube *mtube, const std::vector<Plan *> &mols, const std
     cat_shift(B->nsrc_end, M, 1, 0, [&](int m) { return P_(m).nsrc_end.ptr; }, nodes, add_src, sms, s);
     cat_shift(B->nparent, M, 1, 1, [&](int m) { return P_(m).nparent.ptr; }, nodes, add_node, sms, s);
     cat_shift(B->nchild_first, M, 1, 1, [&](int m) { return P_(m).nchild_first.ptr; }, nodes, add_node, sms, s);
-    cat_shift(B->nindex8, M, 1, 0, [&](int m) { return P_(m).nindex8.ptr; }, nodes, zero4, sms, s);
+    cat_shift(B->up_need, M, 1, 0, [&](int m) { return P_(m).up_need.ptr; }, nodes, zero4, sms, s);
     cat_shift(B->nempty, M, 1, 0, [&](int m) { return P_(m).nempty.ptr; }, nodes, zero4, sms, s);
     cat_shift(B->p2m_nodes, M, 1, 0, [&](int m) { return P_(m).p2m_nodes.ptr; },
               [&](int m) { return (long)P_(m).np2m; }, add_node, sms, s);
     B->np2m = 0;
     for (int m = 0; m < M; ++m) B->np2m += P_(m).np2m;
-    B->m2m_level_begin = cat_levels(
-        B->m2m_nodes, M, nlev, [&](int m) { return P_(m).m2m_nodes.ptr; },
-        [&](int m) { return P_(m).m2m_level_begin.data(); }, [&](int m) { return P_(m).tree.nlevels; }, node_off, sms, s);
+    B->up_count.alloc((size_t)nn, s);
+    B->up_count.zero();
     // image shapes per operator and per node, from a molecule with operators
     int ref = -1;
     for (int m = 0; m < M && ref < 0; ++m)
@@ -526,7 +525,7 @@ Plan *merge_wave(Ctx *c, Tube *mtube, const std::vector<Plan *> &mols, const std
         cat_shift(T->tbeg, M, 1, 0, [&](int m) { return S_(m).tbeg.ptr; }, nodes, add_tgt, sms, s);
         cat_shift(T->tend, M, 1, 0, [&](int m) { return S_(m).tend.ptr; }, nodes, add_tgt, sms, s);
         T->l2l_level_begin = cat_levels(
-            T->l2l_nodes, M, nlev, [&](int m) { return S_(m).l2l_nodes.ptr; },
+            T->l2l_parents, M, nlev, [&](int m) { return S_(m).l2l_parents.ptr; },
             [&](int m) { return S_(m).l2l_level_begin.data(); }, [&](int m) { return P_(m).tree.nlevels; }, node_off,
             sms, s);
         auto npair = [&](int m) { return (long)S_(m).nvpairs; };

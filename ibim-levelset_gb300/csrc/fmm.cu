@@ -67,135 +67,6 @@ void cheb_tables_host(int p, ChebTables &T) {
 
 namespace {
 
-// The translations take nc components a node: 4 for the fused block, 1 for one scalar kernel.
-
-// P2M (upPass leaf, bbfmm.h:507-519): mult[leaf][d][c] = sum_pts S(pt, c) dens[d][pt].
-__global__ void __launch_bounds__(128) k_p2m64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
-                                               const int *__restrict__ sb, const int *__restrict__ se,
-                                               const double *__restrict__ ctr, const double *__restrict__ rad,
-                                               const double *__restrict__ x, const double *__restrict__ y,
-                                               const double *__restrict__ z, const double *__restrict__ dens, long ns,
-                                               int nc, double *mult) {
-    __shared__ ChebTables T;
-    __shared__ double Sp[32][3][MAXP];
-    __shared__ double D[4][32];
-    if (threadIdx.x < sizeof(ChebTables) / 8) reinterpret_cast<double *>(&T)[threadIdx.x] = reinterpret_cast<const double *>(tab)[threadIdx.x];
-    for (int t = threadIdx.x + 128; t < (int)(sizeof(ChebTables) / 8); t += 128)
-        reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
-    const int node = nodes[blockIdx.x];
-    const int b = sb[node], e = se[node];
-    const double c[3] = {ctr[3 * node], ctr[3 * node + 1], ctr[3 * node + 2]};
-    const double r[3] = {rad[3 * node], rad[3 * node + 1], rad[3 * node + 2]};
-    __syncthreads();
-    const int p = T.p, R = T.R;
-    double acc[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) acc[q] = 0.;
-    for (int base = b; base < e; base += 32) {
-        const int cnt = min(32, e - base);
-        if (threadIdx.x < 96) {
-            const int pt = threadIdx.x / 3, ax = threadIdx.x % 3;
-            if (pt < cnt) {
-                const double *X = ax == 0 ? x : (ax == 1 ? y : z);
-                interp1(T, (X[base + pt] - c[ax]) / r[ax], Sp[pt][ax]);
-            }
-        } else if (threadIdx.x < 128) {
-            const int pt = threadIdx.x - 96;
-            if (pt < cnt)
-                for (int d = 0; d < nc; ++d) D[d][pt] = dens[d * ns + base + pt];
-        }
-        __syncthreads();
-        for (int q = 0; q < 16; ++q) {
-            const int o = threadIdx.x + 128 * q;
-            if (o >= nc * R) break;
-            const int d = o / R, cc = o % R;
-            const int i = cc % p, j = (cc / p) % p, l = cc / (p * p);
-            double s = acc[q];
-            for (int pt = 0; pt < cnt; ++pt) s += Sp[pt][0][i] * Sp[pt][1][j] * Sp[pt][2][l] * D[d][pt];
-            acc[q] = s;
-        }
-        __syncthreads();
-    }
-    for (int q = 0; q < 16; ++q) {
-        const int o = threadIdx.x + 128 * q;
-        if (o >= nc * R) break;
-        mult[(long)node * nc * R + o] = acc[q];
-    }
-}
-
-// One separable Kronecker transfer (R[id] = S[b2] (x) S[b1] (x) S[b0], bbfmm.h:345-366) on a
-// [nc][p^3] block in shared memory.  up = true: child -> parent (R^T), else parent -> child (R).
-__device__ void kron_apply(const ChebTables &T, int nc, int id, bool up, double *buf, double *tmp, int nthreads) {
-    const int p = T.p, R = T.R;
-    const int b[3] = {id & 1, (id >> 1) & 1, (id >> 2) & 1};
-    // axis 0 (x, stride 1), axis 1 (y, stride p), axis 2 (z, stride p^2)
-    for (int ax = 0; ax < 3; ++ax) {
-        const int stride = ax == 0 ? 1 : (ax == 1 ? p : p * p);
-        double *src = (ax & 1) ? tmp : buf;
-        double *dst = (ax & 1) ? buf : tmp;
-        for (int o = threadIdx.x; o < nc * R; o += nthreads) {
-            const int d = o / R, cc = o % R;
-            const int idx = (cc / stride) % p;
-            const int base = d * R + cc - idx * stride;
-            double s = 0.;
-            for (int k = 0; k < p; ++k) {
-                // up:   out[n] = sum_k S[b][k][n] in[k];   down: out[k] = sum_n S[b][k][n] in[n]
-                const double w = up ? T.S[b[ax]][k][idx] : T.S[b[ax]][idx][k];
-                s += w * src[base + k * stride];
-            }
-            dst[o] = s;
-        }
-        __syncthreads();
-    }
-    // after 3 passes the result is in tmp (passes wrote tmp, buf, tmp)
-}
-
-// M2M (upPass, bbfmm.h:530-534): parent = sum over non-empty children R[i]^T child.
-__global__ void __launch_bounds__(128) k_m2m64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
-                                               const int *__restrict__ child_first, const int *__restrict__ empty,
-                                               int nc, double *mult) {
-    extern __shared__ double sm[];
-    __shared__ ChebTables T;
-    for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
-        reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
-    __syncthreads();
-    const int R = T.R, n4 = nc * R;
-    double *buf = sm, *tmp = sm + n4, *acc = sm + 2 * n4;
-    const int node = nodes[blockIdx.x];
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) acc[o] = 0.;
-    const int c0 = child_first[node];
-    for (int c8 = 0; c8 < 8; ++c8) {
-        const int ch = c0 + c8;
-        if (empty[ch]) continue;
-        __syncthreads();
-        for (int o = threadIdx.x; o < n4; o += blockDim.x) buf[o] = mult[(long)ch * n4 + o];
-        __syncthreads();
-        kron_apply(T, nc, c8, true, buf, tmp, blockDim.x);
-        for (int o = threadIdx.x; o < n4; o += blockDim.x) acc[o] += tmp[o];
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) mult[(long)node * n4 + o] = acc[o];
-}
-
-// L2L (downPass, bbfmm.h:566-567): child += R[index8] parent.
-__global__ void __launch_bounds__(128) k_l2l64(const ChebTables *__restrict__ tab, const int *__restrict__ nodes,
-                                               const int *__restrict__ parent, const int *__restrict__ index8,
-                                               int nc, double *local) {
-    extern __shared__ double sm[];
-    __shared__ ChebTables T;
-    for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
-        reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
-    __syncthreads();
-    const int R = T.R, n4 = nc * R;
-    double *buf = sm, *tmp = sm + n4;
-    const int node = nodes[blockIdx.x];
-    const int par = parent[node];
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) buf[o] = local[(long)par * n4 + o];
-    __syncthreads();
-    kron_apply(T, nc, index8[node], false, buf, tmp, blockDim.x);
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) local[(long)node * n4 + o] += tmp[o];
-}
-
 // Build the M2L operators: op (target level, source level, centre offset D in target half-widths)
 // -> K[col * 4R + row], row = out * R + ct, col = in * R + cs,
 // entry = block(src_cheb(cs) - tgt_cheb(ct))[out][in], node positions D r_t + r_s cheb - r_t cheb.
@@ -617,49 +488,6 @@ void near64_side_by_side(std::atomic<uint64_t> &done) {
                        });
 }
 
-// L2P alone (bbfmm.h:600), one target leaf per block, added to the near-field sums already in
-// `out`: the form used when the near field runs beside the far field.
-constexpr int L2P_T = 128;
-template <int NC>
-__global__ void __launch_bounds__(L2P_T) k_l2p64(const ChebTables *__restrict__ tab, const int *__restrict__ tleaf,
-                                                  const int *__restrict__ tb_, const int *__restrict__ te_,
-                                                  const double *__restrict__ ctr, const double *__restrict__ rad,
-                                                  const double *__restrict__ tx, const double *__restrict__ ty,
-                                                  const double *__restrict__ tz, long nt,
-                                                  const double *__restrict__ local, double *out) {
-    __shared__ ChebTables T;
-    __shared__ double Ls[NC * MAXR];               // the leaf's local expansion
-    __shared__ double W[3][L2P_T][MAXP + 1];      // per-thread interpolation weights (odd stride)
-    for (int t = threadIdx.x; t < (int)(sizeof(ChebTables) / 8); t += blockDim.x)
-        reinterpret_cast<double *>(&T)[t] = reinterpret_cast<const double *>(tab)[t];
-    const int leaf = tleaf[blockIdx.x];
-    const int tb = tb_[leaf], te = te_[leaf];
-    __syncthreads();
-    const int p = T.p, R = p * p * p;
-    for (int i = threadIdx.x; i < NC * R; i += blockDim.x) Ls[i] = local[(long)leaf * NC * R + i];
-    __syncthreads();
-    double *w0 = W[0][threadIdx.x], *w1 = W[1][threadIdx.x], *w2 = W[2][threadIdx.x];
-    for (int t = tb + threadIdx.x; t < te; t += blockDim.x) {
-        interp1(T, (tx[t] - ctr[3 * leaf]) / rad[3 * leaf], w0);
-        interp1(T, (ty[t] - ctr[3 * leaf + 1]) / rad[3 * leaf + 1], w1);
-        interp1(T, (tz[t] - ctr[3 * leaf + 2]) / rad[3 * leaf + 2], w2);
-        double l2p[NC] = {};
-        int c = 0;
-        for (int c2 = 0; c2 < p; ++c2) {
-            const double s2 = w2[c2];
-            for (int c1 = 0; c1 < p; ++c1) {
-                const double s1 = w1[c1];
-                for (int c0 = 0; c0 < p; ++c0, ++c) {
-                    const double w = w0[c0] * s1 * s2;
-#pragma unroll
-                    for (int o = 0; o < NC; ++o) l2p[o] += w * Ls[o * R + c];
-                }
-            }
-        }
-        for (int o = 0; o < NC; ++o) out[o * nt + t] += l2p[o];
-    }
-}
-
 }  // namespace
 
 // ----------------------------------------------------------------------------------------
@@ -826,15 +654,17 @@ static void build_target_lists(Plan &P, TargetSet &S, OpIndex &opid) {
     const int nn = T.nnodes;
     auto has_t = [&](int i) { return S.end[i] > S.begin[i]; };
     auto has_s = [&](int i) { return T.src_end[i] > T.src_begin[i]; };
+    // parents by their children's level; levels 0 and 1 have no locals
     std::vector<int> l2l, lb(T.nlevels + 1, 0);
     for (int l = 0; l < T.nlevels; ++l) {
         lb[l] = (int)l2l.size();
-        for (int i = T.level_begin[l]; i < T.level_begin[l + 1]; ++i)
-            if (l >= 3 && has_t(i)) l2l.push_back(i);
+        if (l < 3) continue;
+        for (int i = T.level_begin[l - 1]; i < T.level_begin[l]; ++i)
+            if (!T.leaf[i] && has_t(i)) l2l.push_back(i);
     }
     lb[T.nlevels] = (int)l2l.size();
     S.l2l_level_begin = lb;
-    up_int(S.l2l_nodes, l2l, s);
+    up_int(S.l2l_parents, l2l, s);
     // V and X pairs grouped by operator with counting sorts: pairs are generated per target node
     // in parallel, new operator keys get ids in key order (V: dense index, X: sorted keys), and
     // each thread scatters its own contiguous node range, so the grouping is deterministic
@@ -1210,25 +1040,26 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
         up_int(P->nsrc_begin, T.src_begin, s);
         up_int(P->nsrc_end, T.src_end, s);
         up_int(P->nparent, T.parent, s);
-        up_int(P->nindex8, T.index8, s);
         up_int(P->nempty, T.empty, s);
         std::vector<int> child_first(nn, -1);
         for (int i = nn - 1; i >= 0; --i)
             if (T.parent[i] >= 0) child_first[T.parent[i]] = i - T.index8[i];
         up_int(P->nchild_first, child_first, s);
         auto has_s = [&](int i) { return T.src_end[i] > T.src_begin[i]; };
-        std::vector<int> p2m, m2m, m2m_lb(T.nlevels + 1, 0);
+        std::vector<int> p2m, need(nn, 0);
         for (int i = 0; i < nn; ++i)
             if (T.leaf[i] && has_s(i)) p2m.push_back(i);
-        for (int l = 0; l < T.nlevels; ++l) {
-            m2m_lb[l] = (int)m2m.size();
-            for (int i = T.level_begin[l]; i < T.level_begin[l + 1]; ++i)
-                if (!T.leaf[i] && has_s(i)) m2m.push_back(i);
-        }
-        m2m_lb[T.nlevels] = (int)m2m.size();
+        // no list holds a multipole of levels 0 and 1 but a leaf's own: the upward pass ends at level 2
+        for (int l = 3; l < T.nlevels; ++l)
+            for (int i = T.level_begin[l]; i < T.level_begin[l + 1]; i += 8) {
+                int k = 0;
+                for (int c = 0; c < 8; ++c) k += has_s(i + c);
+                for (int c = 0; c < 8; ++c) need[i + c] = k;
+            }
         up_int(P->p2m_nodes, p2m, s);
-        up_int(P->m2m_nodes, m2m, s);
-        P->m2m_level_begin = m2m_lb;
+        up_int(P->up_need, need, s);
+        P->up_count.alloc(nn, s);
+        P->up_count.zero();
         P->np2m = (int)p2m.size();
         OpIndex opid(T.nlevels);
         trace_mark("plan: node arrays enqueued");
@@ -1278,15 +1109,9 @@ Plan *make_plan(Tube *t, bool with_self, const double *extra, long n_extra, int 
         P->mult.alloc((size_t)nn * n4, s);
         P->local.alloc((size_t)nn * n4, s);
         P->dens4.alloc((size_t)4 * ns, s);
-        const size_t smem_k = sizeof(double) * 3 * n4;
-        if (smem_k + sizeof(ChebTables) > 48 * 1024) {  // the kernels' own tables count too (order 8)
-            IBIM_CUDA(cudaFuncSetAttribute(k_m2m64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
-            IBIM_CUDA(cudaFuncSetAttribute(k_l2l64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_k));
-        }
         static std::atomic<uint64_t> split, split_near;
         near64_side_by_side(split_near);
-        side_by_side(split, {(const void *)k_p2m64, (const void *)k_m2m64, (const void *)k_l2l64,
-                             (const void *)k_l2p64<4>, (const void *)k_l2p64<1>, (const void *)k_gather});
+        side_by_side(split, {(const void *)k_gather});
         const size_t sm = sizeof(double) * M2L_CH * n4;
         if (sm > 48 * 1024)
             IBIM_CUDA(cudaFuncSetAttribute(k_m2l_v64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1500,11 +1325,9 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
     const TargetSet &S = *P.targets[ts];
     Ctx *c = P.ctx;
     cudaStream_t s = c->stream;
-    const TreeHost &T = P.tree;
     const int nc = entry == ENTRY_BLOCK ? 4 : 1;
     const int R = P.R, n4 = nc * R;
     const KParams kp = make_kparams(kpp, P.tube->h);
-    const size_t smem_k = sizeof(double) * 3 * n4;
     const double *tx = S.self ? P.sx.ptr : S.tx.ptr;
     const double *ty = S.self ? P.sy.ptr : S.ty.ptr;
     const double *tz = S.self ? P.sz.ptr : S.tz.ptr;
@@ -1582,20 +1405,7 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
         if (!with_m2l) fork();
     }
     try {
-        if (P.np2m > 0) {
-            ProfScope ps_(PROF_P2M, (8.0 * R + 6.0 * P.p * P.p) * P.ns, 56.0 * P.ns);
-            (count_launch(), k_p2m64<<<P.np2m, 128, 0, s>>>(P.tables.ptr, P.p2m_nodes.ptr, P.nsrc_begin.ptr,
-                                                            P.nsrc_end.ptr, P.ncenter.ptr, P.nradius.ptr, P.sx.ptr,
-                                                            P.sy.ptr, P.sz.ptr, dens, P.ns, nc, P.mult.ptr));
-        }
-        for (int l = T.nlevels - 1; l >= 0; --l) {
-            const int b = P.m2m_level_begin[l], e = P.m2m_level_begin[l + 1];
-            if (e > b) {
-                ProfScope ps_(PROF_M2M);
-                (count_launch(), k_m2m64<<<e - b, 128, smem_k, s>>>(P.tables.ptr, P.m2m_nodes.ptr + b,
-                                                                    P.nchild_first.ptr, P.nempty.ptr, nc, P.mult.ptr));
-            }
-        }
+        translate_up(P, nc, dens, P.mult.ptr);
         P.local.zero();
         if (use_oz) {
             m2l_oz_run(P, S);
@@ -1613,14 +1423,7 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
                                                                       P.ncenter.ptr, P.nradius.ptr, P.mult.ptr,
                                                                       P.local.ptr));
         }
-        for (int l = 3; l < T.nlevels; ++l) {
-            const int b = S.l2l_level_begin[l], e = S.l2l_level_begin[l + 1];
-            if (e > b) {
-                ProfScope ps_(PROF_L2L);
-                (count_launch(), k_l2l64<<<e - b, 128, smem_k, s>>>(P.tables.ptr, S.l2l_nodes.ptr + b, P.nparent.ptr,
-                                                                    P.nindex8.ptr, nc, P.local.ptr));
-            }
-        }
+        translate_down(P, S, nc, P.local.ptr);
     } catch (...) {
         if (forked) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
         throw;
@@ -1633,13 +1436,8 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
             if (atomic) IBIM_CUDA(cudaMemsetAsync(out, 0, sizeof(double) * nc * S.nt, s));
             near(s, 1, nseg, nullptr, true);
         }
-        if (overlap || ff) {  // the L2P runs on its own after the near field
-            ProfScope ps_(PROF_L2P64, (10.0 * R + 6.0 * P.p * P.p) * S.nt, 32.0 * n4 * S.ntleaves + 88.0 * S.nt);
-            auto kern = nc == 4 ? k_l2p64<4> : k_l2p64<1>;
-            (count_launch(), kern<<<S.ntleaves, L2P_T, 0, s>>>(P.tables.ptr, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr,
-                                                                   P.ncenter.ptr, P.nradius.ptr, tx, ty, tz, S.nt,
-                                                                   P.local.ptr, out));
-        }
+        // the L2P runs on its own after the near field
+        if (overlap || ff) translate_l2p(P, S, nc, tx, ty, tz, P.local.ptr, out);
     }
     IBIM_CHECK_LAUNCH();
 }

@@ -110,147 +110,6 @@ __global__ void k_pack_src32(long ns, const double *__restrict__ dens, const flo
     }
 }
 
-// P2M in FP32 (bbfmm.h:507-519); coordinates relative to the leaf centre.
-__global__ void __launch_bounds__(128) k_p2m32(const ChebTables32 *__restrict__ tab, const int *__restrict__ nodes,
-                                               const int *__restrict__ sb, const int *__restrict__ se,
-                                               const float *__restrict__ rad, const float *__restrict__ x,
-                                               const float *__restrict__ y, const float *__restrict__ z,
-                                               const float *__restrict__ dens, long ns, float *mult) {
-    __shared__ ChebTables32 T;
-    __shared__ float Sp[32][3][MAXP];
-    __shared__ float D[4][32];
-    load_tables(T, tab);
-    const int node = nodes[blockIdx.x];
-    const int b = sb[node], e = se[node];
-    const float ir[3] = {1.f / rad[3 * node], 1.f / rad[3 * node + 1], 1.f / rad[3 * node + 2]};
-    __syncthreads();
-    const int p = T.p, R = T.R;
-    float acc[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) acc[q] = 0.f;
-    for (int base = b; base < e; base += 32) {
-        const int cnt = min(32, e - base);
-        if (threadIdx.x < 96) {
-            const int pt = threadIdx.x / 3, ax = threadIdx.x % 3;
-            if (pt < cnt) {
-                const float *X = ax == 0 ? x : (ax == 1 ? y : z);
-                interp1f(T, X[base + pt] * ir[ax], Sp[pt][ax]);
-            }
-        } else {
-            const int pt = threadIdx.x - 96;
-            if (pt < cnt)
-                for (int d = 0; d < 4; ++d) D[d][pt] = dens[d * ns + base + pt];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int o = threadIdx.x + 128 * q;
-            if (o < 4 * R) {
-                const int d = o / R, cc = o % R;
-                const int i = cc % p, j = (cc / p) % p, l = cc / (p * p);
-                float s = acc[q];
-                for (int pt = 0; pt < cnt; ++pt) s = fmaf(Sp[pt][0][i] * Sp[pt][1][j] * Sp[pt][2][l], D[d][pt], s);
-                acc[q] = s;
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        const int o = threadIdx.x + 128 * q;
-        if (o < 4 * R) mult[(long)node * 4 * R + o] = acc[q];
-    }
-}
-
-__device__ void kron_apply32(const ChebTables32 &T, int id, bool up, float *buf, float *tmp) {
-    const int p = T.p, R = T.R;
-    const int b[3] = {id & 1, (id >> 1) & 1, (id >> 2) & 1};
-    for (int ax = 0; ax < 3; ++ax) {
-        const int stride = ax == 0 ? 1 : (ax == 1 ? p : p * p);
-        float *src = (ax & 1) ? tmp : buf;
-        float *dst = (ax & 1) ? buf : tmp;
-        for (int o = threadIdx.x; o < 4 * R; o += blockDim.x) {
-            const int d = o / R, cc = o % R;
-            const int idx = (cc / stride) % p;
-            const int base = d * R + cc - idx * stride;
-            float s = 0.f;
-            for (int k = 0; k < p; ++k) s = fmaf(up ? T.S[b[ax]][k][idx] : T.S[b[ax]][idx][k], src[base + k * stride], s);
-            dst[o] = s;
-        }
-        __syncthreads();
-    }
-}
-
-// One warp's separable transfer (the 3 passes of kron_apply32) on its own buffers.
-__device__ void kron_apply32_warp(const ChebTables32 &T, int id, bool up, float *buf, float *tmp) {
-    const int p = T.p, R = T.R, lane = threadIdx.x & 31;
-    const int b[3] = {id & 1, (id >> 1) & 1, (id >> 2) & 1};
-    for (int ax = 0; ax < 3; ++ax) {
-        const int stride = ax == 0 ? 1 : (ax == 1 ? p : p * p);
-        float *src = (ax & 1) ? tmp : buf;
-        float *dst = (ax & 1) ? buf : tmp;
-        for (int o = lane; o < 4 * R; o += 32) {
-            const int d = o / R, cc = o % R;
-            const int idx = (cc / stride) % p;
-            const int base = d * R + cc - idx * stride;
-            float s = 0.f;
-            for (int k = 0; k < p; ++k) s = fmaf(up ? T.S[b[ax]][k][idx] : T.S[b[ax]][idx][k], src[base + k * stride], s);
-            dst[o] = s;
-        }
-        __syncwarp();
-    }
-}
-
-// M2M in FP32 (bbfmm.h:521-533): one parent per block, warp c transfers child c (its three
-// separable passes need no block barrier), then the block sums the eight results.
-constexpr int M2M32_THREADS = 256;
-__global__ void __launch_bounds__(M2M32_THREADS) k_m2m32(const ChebTables32 *__restrict__ tab,
-                                                         const int *__restrict__ nodes,
-                                                         const int *__restrict__ child_first,
-                                                         const int *__restrict__ empty, float *mult) {
-    extern __shared__ float smf[];  // [8 children][2][4R]
-    __shared__ ChebTables32 T;
-    load_tables(T, tab);
-    __syncthreads();
-    const int n4 = 4 * T.R;
-    const int node = nodes[blockIdx.x];
-    const int c8 = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ch = child_first[node] + c8;
-    float *buf = smf + (size_t)c8 * 2 * n4, *tmp = buf + n4;
-    // after three passes the result is in tmp (odd pass count)
-    if (empty[ch]) {
-        for (int o = lane; o < n4; o += 32) tmp[o] = 0.f;
-    } else {
-        for (int o = lane; o < n4; o += 32) buf[o] = mult[(long)ch * n4 + o];
-        __syncwarp();
-        kron_apply32_warp(T, c8, true, buf, tmp);
-    }
-    __syncthreads();
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) {
-        float a = 0.f;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) a += smf[(size_t)c * 2 * n4 + n4 + o];
-        mult[(long)node * n4 + o] = a;
-    }
-}
-
-__global__ void __launch_bounds__(128) k_l2l32(const ChebTables32 *__restrict__ tab, const int *__restrict__ nodes,
-                                               const int *__restrict__ parent, const int *__restrict__ index8,
-                                               float *local) {
-    extern __shared__ float smf[];
-    __shared__ ChebTables32 T;
-    load_tables(T, tab);
-    __syncthreads();
-    const int n4 = 4 * T.R;
-    float *buf = smf, *tmp = smf + n4;
-    const int node = nodes[blockIdx.x];
-    const int par = parent[node];
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) buf[o] = local[(long)par * n4 + o];
-    __syncthreads();
-    kron_apply32(T, index8[node], false, buf, tmp);
-    for (int o = threadIdx.x; o < n4; o += blockDim.x) local[(long)node * n4 + o] += tmp[o];
-}
-
 // FP32 M2L operators (V and X keys), evaluated in FP64 and rounded (same layout as the FP64
 // operators).
 __global__ void k_make_ops32(const ChebTables *__restrict__ tab, const int *__restrict__ keys,
@@ -677,45 +536,6 @@ __global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restri
     }
 }
 
-// L2P alone (downPass leaf, bbfmm.h:600), one target leaf per block, added to the near-field
-// sums already in `out`: the form used when the near field runs beside the far field.
-__global__ void __launch_bounds__(NT32) k_l2p32(const ChebTables32 *__restrict__ tab, const int *__restrict__ tleaf,
-                                                const int *__restrict__ tb_, const int *__restrict__ te_,
-                                                const float *__restrict__ rad, const float *__restrict__ tx,
-                                                const float *__restrict__ ty, const float *__restrict__ tz, long nt,
-                                                const float *__restrict__ local, double *out) {
-    __shared__ ChebTables32 T;
-    __shared__ float Ls[4 * MAXR];                 // the leaf's local expansion
-    __shared__ float W[3][NT32][MAXP + 1];         // per-thread interpolation weights (odd stride)
-    load_tables(T, tab);
-    const int leaf = tleaf[blockIdx.x];
-    const int tb = tb_[leaf], te = te_[leaf];
-    __syncthreads();  // the tables are loaded
-    const int p = T.p, R = p * p * p;
-    for (int i = threadIdx.x; i < 4 * R; i += blockDim.x) Ls[i] = local[(long)leaf * 4 * R + i];
-    __syncthreads();
-    float *w0 = W[0][threadIdx.x], *w1 = W[1][threadIdx.x], *w2 = W[2][threadIdx.x];
-    for (int t = tb + threadIdx.x; t < te; t += blockDim.x) {
-        interp1f(T, tx[t] / rad[3 * leaf], w0);
-        interp1f(T, ty[t] / rad[3 * leaf + 1], w1);
-        interp1f(T, tz[t] / rad[3 * leaf + 2], w2);
-        float l2p[4] = {0.f, 0.f, 0.f, 0.f};
-        int c = 0;
-        for (int c2 = 0; c2 < p; ++c2) {
-            const float s2 = w2[c2];
-            for (int c1 = 0; c1 < p; ++c1) {
-                const float s1 = w1[c1];
-                for (int c0 = 0; c0 < p; ++c0, ++c) {
-                    const float w = w0[c0] * s1 * s2;
-#pragma unroll
-                    for (int o = 0; o < 4; ++o) l2p[o] = fmaf(w, Ls[o * R + c], l2p[o]);
-                }
-            }
-        }
-        for (int o = 0; o < 4; ++o) out[o * nt + t] += (double)l2p[o];
-    }
-}
-
 inline int ew(Ctx *c, long n) { return (int)std::max<long>(1, std::min<long>(8L * c->num_sms, div_up(n, 256))); }
 
 void up_i(DevBuf<int> &b, const std::vector<int> &v, cudaStream_t s) {
@@ -859,11 +679,6 @@ void prepare_mixed(Plan &P, TargetSet &S) {
         P.local32.alloc((size_t)nn * n4, s);
         P.dens32.alloc((size_t)4 * P.ns, s);
         P.src8.alloc((size_t)2 * P.ns, s);
-        const size_t smk = sizeof(float) * 3 * n4, smk_m2m = sizeof(float) * 16 * n4;
-        if (smk_m2m > 48 * 1024)
-            IBIM_CUDA(cudaFuncSetAttribute(k_m2m32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smk_m2m));
-        if (smk > 48 * 1024)
-            IBIM_CUDA(cudaFuncSetAttribute(k_l2l32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smk));
         IBIM_CUDA(cudaStreamSynchronize(s));
         P.mixed_ready = true;
     }
@@ -1002,8 +817,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     };
     const bool overlap = near_overlap() && S.ntleaves > 0;
     static std::atomic<uint64_t> split;
-    side_by_side(split, {(const void *)k_near32<false>, (const void *)k_near32<true>, (const void *)k_pack_src32,
-                         (const void *)k_p2m32, (const void *)k_m2m32, (const void *)k_l2l32, (const void *)k_l2p32});
+    side_by_side(split, {(const void *)k_near32<false>, (const void *)k_near32<true>, (const void *)k_pack_src32});
     static const int occ = [] {
         int b = 0;
         IBIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_near32<false>, NT32, 0));
@@ -1027,21 +841,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     };
     if (overlap && !with_m2l) fork();
     try {
-        if (P.np2m > 0) {
-            ProfScope ps_(PROF_P2M, (8.0 * R + 6.0 * P.p * P.p) * P.ns, 28.0 * P.ns);
-            (count_launch(), k_p2m32<<<P.np2m, 128, 0, s>>>(tab, P.p2m_nodes.ptr, P.nsrc_begin.ptr, P.nsrc_end.ptr,
-                                                            P.nrad32.ptr, P.sxf.ptr, P.syf.ptr, P.szf.ptr, P.dens32.ptr,
-                                                            P.ns, P.mult32.ptr));
-        }
-        const size_t smk = sizeof(float) * 3 * n4, smk_m2m = sizeof(float) * 16 * n4;
-        for (int l = T.nlevels - 1; l >= 0; --l) {
-            const int b = P.m2m_level_begin[l], e = P.m2m_level_begin[l + 1];
-            if (e > b) {
-                ProfScope ps_(PROF_M2M);
-                (count_launch(), k_m2m32<<<e - b, M2M32_THREADS, smk_m2m, s>>>(tab, P.m2m_nodes.ptr + b, P.nchild_first.ptr,
-                                                                                P.nempty.ptr, P.mult32.ptr));
-            }
-        }
+        translate_up(P, P.dens32.ptr, P.mult32.ptr);
         if (!(tc && m2l_tc_zeroes(P, S))) P.local32.zero();
         if (tc) {
             m2l_tc_run(P, S, overlap && with_m2l ? std::function<void()>(fork) : nullptr);
@@ -1056,14 +856,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
             (count_launch(), k_m2l_x32<<<(int)S.nxpairs, 128, 0, s>>>(tab, k32, S.x_src.ptr, S.x_tgt.ptr, S.x_off32.ptr,
                                                                       P.nrad32.ptr, P.mult32.ptr, P.local32.ptr));
         }
-        for (int l = 3; l < T.nlevels; ++l) {
-            const int b = S.l2l_level_begin[l], e = S.l2l_level_begin[l + 1];
-            if (e > b) {
-                ProfScope ps_(PROF_L2L);
-                (count_launch(), k_l2l32<<<e - b, 128, smk, s>>>(tab, S.l2l_nodes.ptr + b, P.nparent.ptr, P.nindex8.ptr,
-                                                                 P.local32.ptr));
-            }
-        }
+        translate_down(P, S, P.local32.ptr);
     } catch (...) {
         if (forked) cudaStreamSynchronize(c->aux);  // the near field still reads dens and writes out
         throw;
@@ -1071,9 +864,7 @@ void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kpp, const double 
     if (overlap) {
         if (side < std::min(div_up(S.nnear32_seg, NW32), full)) near(s, 0, std::min(div_up(S.nnear32_seg, NW32), full), P.near_next.ptr, 0.);
         IBIM_CUDA(cudaStreamWaitEvent(s, c->ev_near_join, 0));
-        ProfScope ps_(PROF_L2P, (10.0 * R + 6.0 * P.p * P.p) * S.nt, 16.0 * n4 * S.ntleaves + 44.0 * S.nt);
-        (count_launch(), k_l2p32<<<S.ntleaves, NT32, 0, s>>>(tab, S.tleaf.ptr, S.tbeg.ptr, S.tend.ptr, P.nrad32.ptr,
-                                                             tx, ty, tz, S.nt, P.local32.ptr, out));
+        translate_l2p(P, S, tx, ty, tz, P.local32.ptr, out);
     } else if (S.ntleaves > 0) {
         near(s, 1, div_up(S.nnear32_seg, NW32), nullptr, 70.0 * S.near_pairs);
     }

@@ -250,7 +250,7 @@ struct TargetSet {
     DevBuf<double> tx, ty, tz;         // tree order (self: unused, the source arrays are used)
     DevBuf<int> perm_d, tbeg, tend;
     std::vector<int> l2l_level_begin;
-    DevBuf<int> l2l_nodes;
+    DevBuf<int> l2l_parents;           // nodes with children to translate to, by the children's level
     DevBuf<int> v_src, v_tgt, v_chunk; // contraction pairs sorted by operator; chunks (op, begin, count)
     int nchunks = 0;
     DevBuf<int> v_chunk32;             // chunks of the FP32 contraction (larger)
@@ -331,11 +331,10 @@ struct Plan {
     DevBuf<int> src_perm;       // tree pos -> tube index
     // nodes
     DevBuf<double> ncenter, nradius;  // 3 per node
-    DevBuf<int> nsrc_begin, nsrc_end, nparent, nindex8, nempty, nchild_first;
+    DevBuf<int> nsrc_begin, nsrc_end, nparent, nempty, nchild_first;
     int np2m = 0;
     DevBuf<int> p2m_nodes;
-    std::vector<int> m2m_level_begin;
-    DevBuf<int> m2m_nodes;
+    DevBuf<int> up_need, up_count;  // per node: its parent's children with sources (0: the parent is not needed); children done
     DevBuf<int> near_next;      // work counter shared by the near-field launches of one matvec
     // M2L operators keyed by (target level, source level, centre offset), union over target sets:
     // the V list's, and (x_as_ops) the X list's, whose pairs then join the V contraction
@@ -428,6 +427,16 @@ bool fmm_one_entry(const Plan &P);
 void fmm_run_entry(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int entry);
 void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out);
 void fmm_run(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int precision);
+
+// Translations (translate.cu), nc components a node: P2M and M2M, L2L, L2P added to out.  FP32: 4 components.
+void translate_up(Plan &P, int nc, const double *dens, double *mult);
+void translate_up(Plan &P, const float *dens, float *mult);
+void translate_down(Plan &P, const TargetSet &S, int nc, double *local);
+void translate_down(Plan &P, const TargetSet &S, float *local);
+void translate_l2p(Plan &P, const TargetSet &S, int nc, const double *tx, const double *ty, const double *tz,
+                   const double *local, double *out);
+void translate_l2p(Plan &P, const TargetSet &S, const float *tx, const float *ty, const float *tz, const float *local,
+                   double *out);
 
 // Tensor-core V-list M2L (m2l_tc.cu)
 bool m2l_tc_supported();
