@@ -129,6 +129,31 @@ __device__ __forceinline__ void near_pair64(const KParams &k, double dx, double 
     acc[3] += hd * m2 + dz * cm;
 }
 
+// Operators whose centre offsets differ in signs only are one operator with nodes mirrored and the odd components'
+// signs turned (F and psi are even, the gradient and the dipole odd along their axis): each class is evaluated
+// once, at the offsets' magnitudes, and written to all its members.
+struct Mirror {
+    int ct, cs;     // the member's nodes
+    int odd;        // bit c: component c (x, y, z) changes sign
+    __device__ __forceinline__ Mirror(const int *__restrict__ key, int p, const int ti[3], const int si[3])
+        : ct(0), cs(0), odd(0) {
+        int f = 1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const bool m = key[2 + a] < 0;
+            ct += (m ? p - 1 - ti[a] : ti[a]) * f;
+            cs += (m ? p - 1 - si[a] : si[a]) * f;
+            odd |= (int)m << a;
+            f *= p;
+        }
+    }
+    // whether entry (out, in) of the block changes sign: F, Gx, Gy, Gz by m_x, m_y, m_z, psi
+    __device__ __forceinline__ bool flip(int out, int in) const {
+        const int o = out > 0 ? odd >> (out - 1) : 0, i = in < 3 ? odd >> in : 0;
+        return (o ^ i) & 1;
+    }
+};
+
 // Kernel parameters of the float-float near field (hi, lo word pairs) with the tables of its
 // exponential: e0[j] = e^{-j/64}, e1[j] = e^{-j}.
 struct KParamsFF {

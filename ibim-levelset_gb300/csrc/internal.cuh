@@ -342,6 +342,10 @@ struct Plan {
     int nops = 0;
     std::vector<int> op_key_h;
     DevBuf<int> op_key;
+    // operators that are mirror images of one another (centre offsets equal but for signs): classes of up to eight,
+    // op_ord[op_cls[c] .. op_cls[c + 1])
+    std::vector<int> op_cls_h;
+    DevBuf<int> op_ord, op_cls;
     DevBuf<double> ops64;          // nops * (4R)^2, column-major per operator
     DevBuf<float> ops32;
     std::vector<TargetSet *> targets;
@@ -459,12 +463,12 @@ void m2l_pack_images_ff(Plan &P, const float2 *ff);
 void m2l_check_images_ff(Plan &P, const float2 *ff);
 void m2l_oz_run(Plan &P, const TargetSet &S);
 // The FP64 operator's M2L as digit products: bytes of one operator's images at order p (0: the order
-// has none), whether nops of them may be kept on this device, the buffers, the cut of operators
-// [o, o + n) from FP64 ones, one contraction.
+// has none), whether nops of them may be kept on this device, the buffers, the cut of n operators
+// (of places ids) from FP64 ones, one contraction.
 double m2l_oz64_op_bytes(int p);
 bool m2l_oz64_fits(int p, double nops, bool entries = false);  // entries: all the block's, one by one
 void m2l_oz64_alloc(Plan &P, int entry);
-void m2l_oz64_pack(Plan &P, int entry, const double *ops, int o, int n);
+void m2l_oz64_pack(Plan &P, int entry, const double *ops, const int *ids, int n);
 // beside: called before the multipoles' split (work for another stream that has to be on the SMs before the
 // contraction's many CTAs queue for them).
 void m2l_oz64_run(Plan &P, const TargetSet &S, int entry, const std::function<void()> &beside = nullptr);

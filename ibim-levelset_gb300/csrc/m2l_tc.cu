@@ -1747,17 +1747,23 @@ __device__ __forceinline__ long long scaled_rint_bits(double v, int s) {
 // Balanced base-2^D digits of m = rint(x 2^(S D)), |x| <= 1, stored scaled: dig[i] = a_i 2^(-D i)
 // with x = sum_i a_i 2^(-D(i+1)) up to 2^-(S D + 1) (a_i in [-2^(D-1), 2^(D-1)) for i >= 1,
 // |a_0| <= 2^D).
+// All at once: with H = 2^(D-1) added to every digit but the first, the digits are the bit fields of the sum
+// (no carry runs from one to the next), and a field q becomes (q - H) 2^(-D i) by one exact multiply-add on the
+// float 2^23 + q.  Digit by digit, each with a carry in 64 bits, took four times the instructions.
 template <int S>
 __device__ __forceinline__ void oz_digits_of(long long m, uint16_t *dig) {
     constexpr int D = OzShape<S>::D;
-    constexpr long long H = 1LL << (D - 1), MASK = (1LL << D) - 1;
+    constexpr long long H = 1LL << (D - 1);
+    constexpr long long BIAS = H * (((1LL << (D * (S - 1))) - 1) / ((1LL << D) - 1));  // sum_i H 2^(D i), i < S - 1
+    const unsigned long long t = (unsigned long long)(m + BIAS);
 #pragma unroll
     for (int i = S - 1; i > 0; --i) {
-        const long long a = ((m + H) & MASK) - H;
-        dig[i] = bf16_bits_exact((float)(int)a * __int_as_float((127 - D * i) << 23));  // a 2^(-D i)
-        m = (m - a) >> D;  // exact: m - a is a multiple of 2^D
+        const unsigned q = (unsigned)(t >> (D * (S - 1 - i))) & ((1u << D) - 1);
+        const float s = 1.f / (float)(1ULL << (D * i));  // a power of two
+        dig[i] = bf16_bits_exact(fmaf(__uint_as_float(0x4b000000u | q), s, -(8388608.f + (float)H) * s));
     }
-    dig[0] = bf16_bits_exact((float)(int)m);
+    const int top = (int)((long long)t >> (D * (S - 1)));  // |a_0| <= 2^D
+    dig[0] = bf16_bits_exact(__int_as_float(0x4b400000 + top) - 12582912.f);
 }
 
 // Digits of ldexp(v, -e) (|v| < 2^e): the cut of the operator or multipole value v under its
@@ -1823,16 +1829,16 @@ __device__ __forceinline__ int row_scale_exp(const float2 *__restrict__ col0, in
 
 // Row scales of the operators (FP64 or float-float, column-major n4 x n4 per op):
 // sig[op][mtiles * 128] = s_r 2^(-2D) with s_r the power of two >= max_k |A_rk|, and the exponent
-// of s_r.  One thread per (op, row); neighbouring threads read neighbouring rows of a column.
+// of s_r.  ids: the operators' places among the scales, else their own order.  One thread per (op, row); neighbouring threads read neighbouring rows of a column.
 template <class OW>
 __global__ void k_scale_ops_oz(int n4, int mtiles, int nops, int scale_exp, const OW *__restrict__ ops, double *sig,
-                               int *sexp) {
+                               int *sexp, const int *__restrict__ ids = nullptr) {
     const int mpad = mtiles * OZ_M;
     const long total = (long)nops * mpad;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
         const int r = (int)(i % mpad), op = (int)(i / mpad);
         const int e = r < n4 ? row_scale_exp(ops + (long)op * n4 * n4 + r, n4) : 0;
-        sig[i] = ldexp(1.0, e - scale_exp);
+        sig[ids ? (long)ids[op] * mpad + r : i] = ldexp(1.0, e - scale_exp);
         sexp[i] = e;
     }
 }
@@ -1846,7 +1852,7 @@ __global__ void k_scale_ops_oz(int n4, int mtiles, int nops, int scale_exp, cons
 template <int S, class OW, bool H16 = false>
 __global__ void k_pack_ops_oz(int n4, int mtiles, int kpad, int nops, const OW *__restrict__ ops,
                               const int *__restrict__ sexp, uint4 *a, const float *__restrict__ rscale = nullptr,
-                              uint4 *a_hi = nullptr, uint4 *a_lo = nullptr) {
+                              uint4 *a_hi = nullptr, uint4 *a_lo = nullptr, const int *__restrict__ ids = nullptr) {
     static_assert(!H16 || std::is_same<OW, float2>::value, "FP16 images from float-float operators");
     static_assert(OZ_M == TC_M && OZ_KS == TC_KS16 && OZ_ATILE == TC_TILE_BYTES, "one tile layout");
     const int nstage = kpad / OZ_KS, mpad = mtiles * OZ_M, ngrp = kpad / 8;
@@ -1886,7 +1892,7 @@ __global__ void k_pack_ops_oz(int n4, int mtiles, int kpad, int nops, const OW *
             }
         }
         const int t = r / OZ_M, row = r % OZ_M, st = grp / 2, half = grp & 1;
-        const long tile = ((long)op * mtiles + t) * nstage + st, tbase = tile * S;
+        const long tile = ((long)(ids ? ids[op] : op) * mtiles + t) * nstage + st, tbase = tile * S;
         const uint32_t off = tile_off(row, half);  // byte offset of the 16-byte piece
 #pragma unroll
         for (int d = 0; d < S; ++d)
@@ -2510,10 +2516,10 @@ void m2l_oz_pack(Plan &P, const float2 *ff) {
     auto pack = [&](auto kf, auto kd) {
         if (ff)
             (count_launch(), kf<<<gp, 256, 0, s>>>(n4, P.oz_mtiles, P.oz_kpad, P.nops, ff, sexp.ptr, a, nullptr,
-                                                   nullptr, nullptr));
+                                                   nullptr, nullptr, nullptr));
         else
             (count_launch(), kd<<<gp, 256, 0, s>>>(n4, P.oz_mtiles, P.oz_kpad, P.nops, P.ops64.ptr, sexp.ptr, a,
-                                                   nullptr, nullptr, nullptr));
+                                                   nullptr, nullptr, nullptr, nullptr));
     };
     if (S == 6)
         pack(k_pack_ops_oz<6, float2>, k_pack_ops_oz<6, double>);
@@ -2688,7 +2694,7 @@ void m2l_oz64_alloc(Plan &P, int entry) {
                          (const void *)k_split_mult_oz<9>});
 }
 
-void m2l_oz64_pack(Plan &P, int entry, const double *ops, int o, int n) {
+void m2l_oz64_pack(Plan &P, int entry, const double *ops, const int *ids, int n) {
     cudaStream_t s = P.ctx->stream;
     auto &Z = P.oz64[entry];
     const int n4 = Z.n, D = P.oz64_s == 8 ? OzShape<8>::D : OzShape<9>::D;
@@ -2697,12 +2703,11 @@ void m2l_oz64_pack(Plan &P, int entry, const double *ops, int o, int n) {
     sexp.alloc((size_t)rows, s);
     const int gs = (int)std::min<long>((rows + 255) / 256, 32L * P.ctx->num_sms);
     const int gp = (int)std::min<long>((rows * (Z.kpad / 8) + 255) / 256, 64L * P.ctx->num_sms);
-    const size_t row0 = (size_t)o * Z.mtiles;
-    (count_launch(), k_scale_ops_oz<double><<<gs, 256, 0, s>>>(n4, Z.mtiles, n, 2 * D, ops, Z.sig.ptr + row0 * OZ_M,
-                                                               sexp.ptr));
-    uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr + row0 * (Z.kpad / OZ_KS) * P.oz64_s * (OZ_ATILE / 2));
+    (count_launch(), k_scale_ops_oz<double><<<gs, 256, 0, s>>>(n4, Z.mtiles, n, 2 * D, ops, Z.sig.ptr,
+                                                               sexp.ptr, ids));
+    uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr);
     auto kern = P.oz64_s == 8 ? k_pack_ops_oz<8, double> : k_pack_ops_oz<9, double>;
-    (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr));
+    (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr, ids));
     IBIM_CHECK_LAUNCH();
 }
 

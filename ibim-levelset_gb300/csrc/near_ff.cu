@@ -280,11 +280,12 @@ __global__ void __launch_bounds__(NTF) k_near_ff(KParamsFF kp, const int4 *__res
 // root / 2^level, lattice offset, Chebyshev nodes) is split once per block from FP64.
 __global__ void __launch_bounds__(256) k_make_ops_ff(KParamsFF kp, const ChebTables *__restrict__ tab,
                                                      const int *__restrict__ keys, const double *__restrict__ root_r,
+                                                     const int *__restrict__ cls, const int *__restrict__ ord,
                                                      float2 *ops) {
     __shared__ float2 E0[64], E1[64];
     __shared__ f2 rt_s[3], rs_s[3], ch_s[MAXP];
     __shared__ float D_s[3];
-    const int op = blockIdx.y;
+    const int m0 = cls[blockIdx.y], m1 = cls[blockIdx.y + 1], op = ord[m0];
     if (threadIdx.x < 64) {
         E0[threadIdx.x] = kp.e0[threadIdx.x];
         E1[threadIdx.x] = kp.e1[threadIdx.x];
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(256) k_make_ops_ff(KParamsFF kp, const ChebTab
         for (int a = 0; a < 3; ++a) {
             rt_s[a] = split_d(ldexp(root_r[a], -lt));
             rs_s[a] = split_d(ldexp(root_r[a], -ls));
-            D_s[a] = (float)keys[5 * op + 2 + a];
+            D_s[a] = (float)abs(keys[5 * op + 2 + a]);
         }
         for (int m = 0; m < tab->p; ++m) ch_s[m] = split_d(tab->cheb[m]);
     }
@@ -328,12 +329,17 @@ __global__ void __launch_bounds__(256) k_make_ops_ff(KParamsFF kp, const ChebTab
     } else {
         b[3] = neg(ld(kp.k2in));
     }
-    float2 *K = ops + (long)op * n4 * n4;
+    for (int m = m0; m < m1; ++m) {
+        const Mirror M(keys + 5 * ord[m], p, ti, si);
+        float2 *K = ops + (long)ord[m] * n4 * n4;
 #pragma unroll
-    for (int o = 0; o < 4; ++o)
+        for (int o = 0; o < 4; ++o)
 #pragma unroll
-        for (int in = 0; in < 4; ++in)
-            K[(long)(in * R + cs) * n4 + (o * R + ct)] = make_float2(b[o * 4 + in].h, b[o * 4 + in].l);
+            for (int in = 0; in < 4; ++in) {
+                const f2 v = M.flip(o, in) ? neg(b[o * 4 + in]) : b[o * 4 + in];
+                K[(long)(in * R + M.cs) * n4 + (o * R + M.ct)] = make_float2(v.h, v.l);
+            }
+    }
 }
 
 float2 split_h(double x) {
@@ -389,10 +395,11 @@ void fmm_prepare_operators_ff(Plan &P, const ibim_kernel_params &kpp) {
     const int R = P.R, n4 = 4 * R;
     P.opsff.alloc((size_t)P.nops * n4 * n4, s);
     const KParamsFF kff = make_kparams_ff(make_kparams(kpp, P.tube->h));
-    dim3 g((unsigned)div_up((long)R * R, 256), P.nops);
+    dim3 g((unsigned)div_up((long)R * R, 256), (unsigned)P.op_cls_h.size() - 1);
     {
         ProfScope ps_(PROF_OPS);
-        (count_launch(), k_make_ops_ff<<<g, 256, 0, s>>>(kff, P.tables.ptr, P.op_key.ptr, P.root_r.ptr, P.opsff.ptr));
+        (count_launch(), k_make_ops_ff<<<g, 256, 0, s>>>(kff, P.tables.ptr, P.op_key.ptr, P.root_r.ptr,
+                                                           P.op_cls.ptr, P.op_ord.ptr, P.opsff.ptr));
     }
     IBIM_CHECK_LAUNCH();
     for (int i = 0; i < 5; ++i) P.kpff[i] = key[i];
