@@ -211,18 +211,19 @@ __global__ void __launch_bounds__(128) k_m2l_x64(const ChebTables *__restrict__ 
 //
 // Bound by GB300's narrow FP64 pipe (2 lanes a cycle per SM: 16 cycles a warp instruction, whatever
 // else the SM does), so the count of FP64 instructions a pair is the kernel's time.  near64_pair
-// takes 51 (22 without screening) where the formulas as written took about 103: seeds, rounding
-// and comparisons on the integer and FP32 pipes, one cubic step for 1 / r, a 128-entry table and a
-// degree-5 polynomial for the exponential, and the constant factors applied once per target instead of
-// once per pair.  16 warps a SM keep the pipe busy; two CTAs of 11 KB leave the rest of the SM to
-// the tensor-core M2L that runs beside it.  On a 2,000-atom protein (5.2e8 pairs): 82 -> 49 ms alone
-// (51 instructions take 41 ms), 55 ms beside the M2L.
+// takes 42 (20 without screening) where the formulas as written took about 103: seeds, their refinement,
+// rounding and comparisons on the integer and FP32 pipes, a 512-entry table and a polynomial of degree 4, half of
+// it in FP32, for the exponential, and the constant factors applied once per target instead of
+// once per pair.  16 warps a SM keep the pipe busy; two CTAs of 14 KB leave the rest of the SM to
+// the tensor-core M2L that runs beside it.  On a 2,000-atom protein (5.2e8 pairs): 82 -> 43 ms alone
+// (42 instructions take 35 ms; 51, with a cubic step for 1 / r and all of the polynomial in FP64, 49 ms), 46 ms
+// beside the M2L.
 constexpr int NEAR_T = 256, NEAR_TILE = 128, NEAR_CPS = 2;  // threads, sources a tile, CTAs a SM
-constexpr int NEAR_EXP = 128;                               // steps of 2^-x in the table
+constexpr int NEAR_EXP = 512;                               // steps of 2^-x in the table
 enum { NEAR_GENERAL = 0, NEAR_YUKAWA = 1, NEAR_LAPLACE = 2 };
 
 struct Near64K {
-    double vr2, eps, ieps, kappa, kl;  // kl = kappa log2 e
+    double vr2, eps, ieps, kappa, kappa2, kl;  // kl = kappa log2 e
     double sk, k2c;                    // k3f / q4pi; k2in k3f / q4pi^2 (the cutoff's K2 in A0's units)
     double psi_f, f0, fg;              // staged psi = psi psi_f; F = f0 A0, G = fg A
     float klt;                         // kl NEAR_EXP
@@ -236,6 +237,7 @@ Near64K make_near64(const KParams &k) {
     n.eps = k.eps;
     n.ieps = k.ieps;
     n.kappa = k.kappa;
+    n.kappa2 = k.kappa * k.kappa;
     n.kl = k.kappa * 1.4426950408889634074;
     n.sk = k.k3f / k.q4pi;
     n.psi_f = k.q4pi / k.k3f;
@@ -246,10 +248,11 @@ Near64K make_near64(const KParams &k) {
     return n;
 }
 
-// FP32 value of a positive double by its bits (truncated; 2^127 and above, 2^-126 and below clamp).
+// FP32 value of a double below 2^127 in magnitude by its bits (truncated; below 2^-126: 0).
 __device__ __forceinline__ float near64_f32(double v) {
-    const int hi = min(max(__double2hiint(v), 0x38000000), 0x47dfffff);
-    return __int_as_float(((hi - 0x38000000) << 3) | ((unsigned)__double2loint(v) >> 29));
+    const unsigned hi = __double2hiint(v), mag = hi & 0x7fffffff;
+    if (mag < 0x38100000) return 0.f;
+    return __uint_as_float((hi & 0x80000000) | ((mag - 0x38000000) << 3) | ((unsigned)__double2loint(v) >> 29));
 }
 // The double equal to a non-negative normal float (0 becomes 2^-127).
 __device__ __forceinline__ double near64_f64(float v) {
@@ -257,42 +260,63 @@ __device__ __forceinline__ double near64_f64(float v) {
     return __hiloint2double((b >> 3) + 0x38000000, b << 29);
 }
 
-// t = kappa r and e = e^-t = 2^{-n/128} 2^{-g}: n from the FP32 r, g exact, |g| < 2^-7.8, Taylor to degree 5
-// (below 2^-58).
-__device__ __forceinline__ void near64_exp(const Near64K &k, const double2 *__restrict__ e2, double r, float rf, double &t,
+// 1 / sqrt(d2) for normal d2 > 0 in three FP64 instructions, and sqrt(d2) to FP32 (at most 2^121).  The seed is
+// refined to 2^-44 on the FP32 and integer pipes, which are nearly idle here: d2 = 4^E2 (a + rho) with a the FP32
+// head in [1, 4); y = rsqrt(a) from FP32; the residual 1 - (a + rho) y^2 by FP32 multiply-adds (y^2 as head and
+// tail); y (1 + residual / 2) assembled in units of 2^-53.  Then y + y e, e = (1 - d2 y^2) / 2 of 2^-45.
+__device__ __forceinline__ double near64_rsqrt(double d2, float &rf) {
+    const int hi = __double2hiint(d2);
+    const unsigned lo = __double2loint(d2);
+    const int E = (hi >> 20) - 1023, odd = E & 1, E2 = E >> 1;
+    const float a = __uint_as_float(((127u + odd) << 23) | (((unsigned)hi & 0xfffffu) << 3) | (lo >> 29));
+    const float rho = (float)(lo & 0x1fffffffu) * __int_as_float((127 - 52 + odd) << 23);
+    float yf;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(a));
+    rf = __int_as_float(__float_as_int(a * yf) + (min(E2, 120) << 23));
+    const float ph = yf * yf, pl = fmaf(yf, yf, -ph);
+    const float res = fmaf(-rho, ph, fmaf(-a, pl, fmaf(-a, ph, 1.f)));
+    const int inc = __float2int_rn(yf * res * 0x1p49f);  // half the residual in units of 2^-50: below 2^29
+    const int yb = __float_as_int(yf);
+    const long long Y = ((long long)((yb & 0x7fffff) | 0x800000) << ((yb >> 23) - 97)) + ((long long)inc << 3);
+    const int c = (int)(Y >> 53) & 1;  // y >= 1
+    const double y = __longlong_as_double((Y >> c) + ((long long)(1021 + c - E2) << 52));
+    const double mh = __hiloint2double((__double2hiint(y) - 0x00100000) ^ 0x80000000, __double2loint(y));  // -y / 2
+    return fma(y, fma(d2 * y, mh, 0.5), y);
+}
+
+// t = kappa r and e = e^-t = 2^{-n/512} 2^{-g}: n from the FP32 r, g exact, |g| <= 2^-10 (2^-9.7 where e is below
+// 2^-900); Taylor to degree 4 (below 2^-59), the two highest coefficients, 2^-34 of the whole, in FP32.
+__device__ __forceinline__ void near64_exp(const Near64K &k, const double *__restrict__ e2, double r, float rf, double &t,
                                            double &e) {
     t = k.kappa * r;
-    const float xm = fminf(rf * k.klt, 128000.f) + 12582912.f;  // n in the low bits
+    const float xm = fminf(rf * k.klt, 1000.f * NEAR_EXP) + 12582912.f;  // n in the low bits
     const int n = __float_as_int(xm) - 0x4b400000;
     const double g = fma(k.kl, r, -near64_f64((xm - 12582912.f) * (1.f / NEAR_EXP)));
-    double q = fma(g, -1.3333558146428443e-3, 9.6181291076284772e-3);
-    q = fma(g, q, -5.5504108664821580e-2);
-    q = fma(g, q, 2.4022650695910072e-1);
+    const float h = fmaf(near64_f32(g), -9.6181291e-3f, 5.5504109e-2f);
+    double q = fma(-near64_f64(h), g, 2.4022650695910072e-1);
     q = fma(g, q, -6.9314718055994531e-1) * g;
-    const double2 tb = e2[n & (NEAR_EXP - 1)];
-    const double ef = tb.x + fma(tb.x, q, tb.y);
-    e = n >= 128000 ? 0.0 : __hiloint2double(__double2hiint(ef) - ((n / NEAR_EXP) << 20), __double2loint(ef));
+    const double tb = e2[n & (NEAR_EXP - 1)];
+    const double ef = fma(tb, q, tb);
+    e = n >= 1000 * NEAR_EXP ? 0.0
+                             : __hiloint2double(__double2hiint(ef) - ((n / NEAR_EXP) << 20), __double2loint(ef));
 }
 
 // One source -> target update of the fused block (kblock64's formulas) for d2 >= vr2, with
 // M = d.m / r^3 shared by K1 and K3, psi staged times q4pi / k3f, and the factors q4pi (F) and
-// k3f (G) left to the caller.  1 / r: FP32 seed y (relative error below 2^-22), then
-// y (1 + e/2 + 3 e^2/8) with e = 1 - d2 y^2, whose error is about 5/16 e^3 < 2^-64.
+// k3f (G) left to the caller.  With u = 1 - e^-t (1 + t): ho / r^2 = kappa^2 e^-t - 3 u / r^2 and hd = u / r^3; 3 u
+// serves both, with the dipole also staged a third as large (n).
 template <int MODE>
-__device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__restrict__ e2, double dx, double dy,
-                                            double dz, double m0, double m1, double m2, double psi, double acc[4]) {
+__device__ __forceinline__ void near64_pair(const Near64K &k, const double *__restrict__ e2, double dx, double dy,
+                                            double dz, double m0, double m1, double m2, double psi, double n0, double n1,
+                                            double n2, double acc[4]) {
     const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
     // both non-negative: the order of the bits is the order of the values
     if (__double_as_longlong(d2) < __double_as_longlong(k.vr2)) {
         if (MODE == NEAR_YUKAWA) acc[0] = fma(-k.k2c, psi, acc[0]);
         return;
     }
-    const float d2f = near64_f32(d2);
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(d2f));
-    const double y = near64_f64(yf);
-    const double e0 = fma(-(d2 * y), y, 1.0);
-    const double ir = fma(y, fma(e0, 0.375, 0.5) * e0, y);
+    float rf;
+    const double ir = near64_rsqrt(d2, rf);
     const double ir2 = ir * ir, ir3 = ir2 * ir;
     const double M = fma(dx, m0, fma(dy, m1, dz * m2)) * ir3;
     const double w = ir3 * psi;
@@ -304,23 +328,23 @@ __device__ __forceinline__ void near64_pair(const Near64K &k, const double2 *__r
         return;
     }
     double t, e;
-    near64_exp(k, e2, d2 * ir, d2f * yf, t, e);
+    near64_exp(k, e2, d2 * ir, rf, t, e);
     const double et1 = fma(e, t, e);
     acc[0] = fma(fma(k.eps, et1, -1.0), M, acc[0]);
     acc[0] = fma(-(fma(-k.sk, e, k.sk) * ir), psi, acc[0]);
-    const double ho = fma(e, fma(t + 3.0, t, 3.0), -3.0);
-    const double cm = fma(-fma(-k.ieps, et1, 1.0), w, ho * (ir2 * M));
-    const double hd = (1.0 - et1) * ir3;
-    acc[1] = fma(dx, cm, fma(hd, m0, acc[1]));
-    acc[2] = fma(dy, cm, fma(hd, m1, acc[2]));
-    acc[3] = fma(dz, cm, fma(hd, m2, acc[3]));
+    const double u3 = fma(-3.0, et1, 3.0);
+    const double cm = fma(fma(-u3, ir2, e * k.kappa2), M, -(fma(-k.ieps, et1, 1.0) * w));
+    const double hd3 = u3 * ir3;
+    acc[1] = fma(dx, cm, fma(hd3, n0, acc[1]));
+    acc[2] = fma(dy, cm, fma(hd3, n1, acc[2]));
+    acc[3] = fma(dz, cm, fma(hd3, n2, acc[3]));
 }
 
-// One scalar kernel's update, an entry of the block above by the same steps (26 to 31 FP64 instructions
-// screened, 12 not): a and b are the axes of the dipole (K1, K3) and of the gradient (K3, K4).
+// One scalar kernel's update, an entry of the block above by the same steps (22 to 26 FP64 instructions
+// screened, 14 not): a and b are the axes of the dipole (K1, K3) and of the gradient (K3, K4).
 enum { NEAR_BLOCK = 0, NEAR_K1 = 1, NEAR_K2 = 2, NEAR_K3 = 3, NEAR_K4 = 4 };
 template <int MODE, int KIND>
-__device__ __forceinline__ double near64_one(const Near64K &k, const double2 *__restrict__ e2, double dx, double dy,
+__device__ __forceinline__ double near64_one(const Near64K &k, const double *__restrict__ e2, double dx, double dy,
                                              double dz, int a, int b, double m, double acc) {
     const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
     const double da = a == 0 ? dx : (a == 1 ? dy : dz), db = b == 0 ? dx : (b == 1 ? dy : dz);
@@ -335,28 +359,24 @@ __device__ __forceinline__ double near64_one(const Near64K &k, const double2 *__
     }
     if (MODE == NEAR_LAPLACE && (KIND == NEAR_K2 || KIND == NEAR_K3)) return acc;
     if (__double_as_longlong(d2) < __double_as_longlong(k.vr2)) return KIND == NEAR_K2 ? fma(-k.k2c, m, acc) : acc;
-    const float d2f = near64_f32(d2);
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(d2f));
-    const double y = near64_f64(yf);
-    const double e0 = fma(-(d2 * y), y, 1.0);
-    const double ir = fma(y, fma(e0, 0.375, 0.5) * e0, y);
+    float rf;
+    const double ir = near64_rsqrt(d2, rf);
     const double ir2 = ir * ir, ir3 = ir2 * ir;
     if (MODE == NEAR_LAPLACE) return fma((KIND == NEAR_K1 ? da : db) * m, ir3, acc);
     double t, e;
-    near64_exp(k, e2, d2 * ir, d2f * yf, t, e);
+    near64_exp(k, e2, d2 * ir, rf, t, e);
     if (KIND == NEAR_K2) return fma(-(fma(-k.sk, e, k.sk) * ir), m, acc);
     const double et1 = fma(e, t, e);
     if (KIND == NEAR_K1) return fma(fma(k.eps, et1, -1.0), (da * m) * ir3, acc);
     if (KIND == NEAR_K4) return fma(db, -fma(-k.ieps, et1, 1.0) * (ir3 * m), acc);
-    const double ho = fma(e, fma(t + 3.0, t, 3.0), -3.0);
-    if (a == b) acc = fma((1.0 - et1) * ir3, m, acc);
-    return fma(db, ho * (ir2 * ((da * m) * ir3)), acc);
+    const double u = 1.0 - et1, mi3 = m * ir3;
+    if (a == b) acc = fma(u, mi3, acc);
+    return fma(db * da, fma(-3.0 * u, ir2, e * k.kappa2) * mi3, acc);
 }
 
 template <int MODE, int KIND>
 __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave the M2L its own
-    k_near64(const ChebTables *__restrict__ tab, const double2 *__restrict__ etab, Near64K kp, const int4 *__restrict__ segs,
+    k_near64(const ChebTables *__restrict__ tab, const double *__restrict__ etab, Near64K kp, const int4 *__restrict__ segs,
              const int *__restrict__ near_range, const int *__restrict__ tb_, const int *__restrict__ te_,
              const double *__restrict__ ctr, const double *__restrict__ rad, const double *__restrict__ sx,
              const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ dens, long ns,
@@ -364,12 +384,14 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
              const double *__restrict__ local, double *out, int l2p_mask, int nseg, int *next, int ax_in, int ax_out) {
     constexpr int NC = KIND == NEAR_BLOCK ? 4 : 1;
     constexpr bool FG = KIND == NEAR_K1 || KIND == NEAR_K2;  // the one output is F
-    __shared__ double2 S[NEAR_TILE][NC == 4 ? 4 : 2];  // x y | z m_x | m_y m_z | psi - , one kernel: x y | z m
-    __shared__ double2 e2[MODE == NEAR_YUKAWA ? NEAR_EXP : 1];  // 2^(-j / 128), high and low word
+    // x y | z m_x | m_y m_z | psi n_x | n_y n_z (n = m / 3), one kernel: x y | z m
+    __shared__ double2 S[NEAR_TILE][NC == 4 ? 5 : 2];
+    __shared__ double e2[MODE == NEAR_YUKAWA ? NEAR_EXP : 1];  // 2^(-j / 512)
     __shared__ int cur;
     double(*red)[NC] = reinterpret_cast<double(*)[NC]>(S);  // [NEAR_T][NC], once the tiles are done
     static_assert(sizeof(S) >= sizeof(double) * NC * NEAR_T, "reduction scratch");
-    if (MODE == NEAR_YUKAWA && threadIdx.x < NEAR_EXP) e2[threadIdx.x] = etab[threadIdx.x];
+    if (MODE == NEAR_YUKAWA)
+        for (int i = threadIdx.x; i < NEAR_EXP; i += NEAR_T) e2[i] = etab[i];
     const double psi_f = MODE == NEAR_GENERAL ? 1.0 : kp.psi_f;
     // with a work counter the CTA takes segments until none is left; without one it does segment blockIdx.x
     for (int it = 0;; ++it) {
@@ -411,11 +433,14 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                             else
                                 S[q][0] = make_double2(sx[i], sy[i]);
                         } else if (threadIdx.x & 1) {
-                            S[q][2] = make_double2(dens[ns + i], dens[2 * ns + i]);
-                            S[q][3] = make_double2(dens[3 * ns + i] * psi_f, 0.);
+                            const double m1 = dens[ns + i], m2 = dens[2 * ns + i];
+                            S[q][2] = make_double2(m1, m2);
+                            S[q][4] = make_double2(m1 * (1.0 / 3.0), m2 * (1.0 / 3.0));
+                            S[q][3].x = dens[3 * ns + i] * psi_f;
                         } else {
                             S[q][0] = make_double2(sx[i], sy[i]);
                             S[q][1] = make_double2(sz[i], dens[i]);
+                            S[q][3].y = dens[i] * (1.0 / 3.0);
                         }
                     }
                     __syncthreads();
@@ -427,12 +452,12 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                                                                 acc[0]);
                                 continue;
                             } else {
-                            const double2 a2 = S[q2][2];
-                            const double psi = S[q2][3].x;
+                            const double2 a2 = S[q2][2], a3 = S[q2][3], a4 = S[q2][4];
                             if (MODE == NEAR_GENERAL)
-                                near_pair64(kp.kp, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
+                                near_pair64(kp.kp, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, a3.x, acc);
                             else
-                                near64_pair<MODE>(kp, e2, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, psi, acc);
+                                near64_pair<MODE>(kp, e2, a0.x - X, a0.y - Y, a1.x - Z, a1.y, a2.x, a2.y, a3.x, a3.y, a4.x,
+                                                  a4.y, acc);
                             }
                         }
                 }
@@ -1403,13 +1428,8 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
     };
     const bool overlap = near_overlap() && S.ntleaves > 0;
     if (!P.exp_tab.ptr) {
-        // 2^(-j / 128) as high and low words, from the host's long double
-        std::vector<double2> h(NEAR_EXP);
-        for (int j = 0; j < NEAR_EXP; ++j) {
-            const long double v = std::exp2(-(long double)j / NEAR_EXP);
-            h[j].x = (double)v;
-            h[j].y = (double)(v - h[j].x);
-        }
+        std::vector<double> h(NEAR_EXP);
+        for (int j = 0; j < NEAR_EXP; ++j) h[j] = std::exp2(-(double)j / NEAR_EXP);
         P.exp_tab.alloc(NEAR_EXP, s);
         P.exp_tab.upload(h.data(), NEAR_EXP);
         IBIM_CUDA(cudaStreamSynchronize(s));

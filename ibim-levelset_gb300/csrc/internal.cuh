@@ -352,7 +352,7 @@ struct Plan {
     // tables and workspaces
     DevBuf<ChebTables> tables;
     DevBuf<double> root_r;
-    DevBuf<double2> exp_tab;  // the FP64 near field's table of powers of two, made on its first use
+    DevBuf<double> exp_tab;  // the FP64 near field's table of powers of two, made on its first use
     DevBuf<double> mult, local, dens4;
     DevBuf<float> mult32, local32, dens32;
     DevBuf<float4> src8;           // near-field source records (mixed): {x, y, z, m_x}, {m_y, m_z, psi, 0}
