@@ -1963,44 +1963,25 @@ __device__ __forceinline__ int exp_of_pow2(double p) {
     return (int)((__double_as_longlong(p) >> 52) & 0x7ff) - 1023;
 }
 
-// The double nearest T 2^e (ties to even) for an integer 0 < |T| < 2^63, assembled from T's bits
-// by integer instructions while the result is a normal number, else by an FP64 multiply.
-__device__ __forceinline__ double pow2_scaled_ll(long long T, const int e0) {
-    unsigned long long a = (unsigned long long)(T < 0 ? -T : T);
-    int e = e0;
-    int msb = 63 - __clzll((long long)a);
-    if (msb > 52) {  // round the low bits away
-        const int sh = msb - 52;
-        const unsigned long long rem = a & ((1ULL << sh) - 1), half = 1ULL << (sh - 1);
-        a >>= sh;
-        if (rem > half || (rem == half && (a & 1ULL))) ++a;
-        e += sh;
-        if (a >> 53) {  // the rounding carried into bit 53: a = 2^53
-            a >>= 1;
-            ++e;
-        }
-        msb = 52;
-    }
-    const int E = msb + e + 1023;  // biased exponent of the result
-    if (E < 1 || E > 2046) return ldexp((double)T, e0);  // subnormal or overflowing result
-    const unsigned long long mant = ((a << (63 - msb)) & 0x7fffffffffffffffULL) >> 11;
-    const unsigned long long bits = ((unsigned long long)(T < 0) << 63) | ((unsigned long long)E << 52) | mant;
-    return __longlong_as_double((long long)bits);
+// The double nearest T 2^e (ties away from zero) for an integer 0 < |T| < 2^63, assembled from T's bits by integer
+// instructions while the result is a normal number, else by an FP64 multiply.
+__device__ __forceinline__ double pow2_scaled_ll(long long T, const int e) {
+    const unsigned long long a = (unsigned long long)(T < 0 ? -T : T);
+    const int lz = __clzll((long long)a), E = 63 - lz + e + 1023;  // biased exponent of the result
+    if (E < 1 || E > 2046) return ldexp((double)T, e);             // subnormal or overflowing result
+    // 53 bits rounded; their leading one (and a carry beyond it) adds to the exponent field
+    const unsigned long long m = ((a << (lz - 1)) + 512) >> 10;
+    const unsigned long long bits = ((unsigned long long)(unsigned)(E - 1) << 52) + m;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)T & 0x8000000000000000ULL)));
 }
 
-// rint(x 2^s) of an FP32 value, |x 2^s| < 2^62, from its bits (ties away from zero; subnormal
-// x, below 2^-126, count as zero).
+// rint(x 2^s) of an FP32 value, |x 2^s| < 2^44, in two parts rounded by 1.5 2^23 (the conversion to 64 bits would
+// take the FP64 pipe from the near field: 57 against 48 ms a product beside it on a 2,000-atom protein).
 __device__ __forceinline__ long long f32_fixed(float x, int s) {
-    const unsigned u = __float_as_uint(x);
-    const int E = (int)((u >> 23) & 0xff);
-    if (E == 0) return 0;
-    const long long m = (long long)((u & 0x7fffffu) | 0x800000u);  // x = m 2^(E - 150)
-    const int sh = E - 150 + s;
-    long long r;
-    if (sh >= 0) r = m << sh;
-    else if (sh < -25) r = 0;
-    else r = (m + (1LL << (-sh - 1))) >> -sh;
-    return (u >> 31) ? -r : r;
+    constexpr float R = 12582912.f;
+    const float h = fmaf(x, __int_as_float((127 + s - 22) << 23), R), hf = h - R;
+    const float l = fmaf(hf, -4194304.f, x * __int_as_float((127 + s) << 23)) + R;
+    return ((long long)(__float_as_int(h) - 0x4b400000) << 22) + (__float_as_int(l) - 0x4b400000);
 }
 
 template <int S>
@@ -2166,6 +2147,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // int64 (|T| < 2^62; M kept to 2^-F of a group-0 unit, below the cut's own error), then
         // the double nearest T 2^(e_r + e_j - 2D - F) is assembled from T's bits; s_r = 2^e_r and
         // t_j = 2^e_j, and sig holds s_r 2^(-2D).
+        // Every output takes some 60 instructions here; with each group shifted and added in 64 bits and ties
+        // rounded to even it was twice that, and the launch 40.2 against 37.4 ms (2,000 atoms, FP64), 14.5
+        // against 13.1 (the residual).
         constexpr int D = SH::D, F = SH::F, CW = SH::CW;
         const int lg = warp & 3, h = warp >> 2;
         const int row = t * OZ_M + 32 * lg + lane;
@@ -2197,12 +2181,18 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 for (int q = 0; q < CW; ++q) {
                     const int tg = tgt_s[c0 + q];
                     constexpr int F0 = D * (OZ_ACC - 2);  // the exact groups' own fraction bits
-                    long long T = 0;
+                    // exact integers below 2^24, folded in pairs: below 2^31, by the groups' bounds K 2^(2D) for the
+                    // first and K 2^(2D) (1 + (k - 1) / 4) for group k with K <= 800 and 500 at D = 7, 1372 at D = 6
+                    int G[OZ_ACC - 1];
 #pragma unroll
-                    for (int g = 0; g < OZ_ACC - 1; ++g)  // exact integers below 2^24
-                        T += (long long)__float2int_rn(__uint_as_float(v[g][q]) *
-                                                       __int_as_float((127 + D * g) << 23))
-                             << (F0 - D * g);
+                    for (int g = 0; g < OZ_ACC - 1; ++g)
+                        G[g] = __float2int_rn(__uint_as_float(v[g][q]) * __int_as_float((127 + D * g) << 23));
+                    long long T = G[0] * (1 << D) + G[1];
+#pragma unroll
+                    for (int g = 2; g < OZ_ACC - 1; g += 2) {
+                        if (g + 1 < OZ_ACC - 1) T = T * (1LL << (2 * D)) + (G[g] * (1 << D) + G[g + 1]);
+                        else T = T * (1LL << D) + G[g];
+                    }
                     // the shared accumulator on F bits, or for the FP64 operator on as many as the
                     // exact sum leaves below bit 62 (entries far below their row's maximum keep theirs)
                     int sh = F - F0;
@@ -2635,8 +2625,8 @@ void m2l_oz_run(Plan &P, const TargetSet &S) {
 // ---------------------------------------------------------------------------------------------
 // M2L of the FP64 operator (IBIM_PRECISION_FP64) as digit products.  GB300 does 1.25 TFLOP/s on the
 // FP64 pipe and 1.9 PFLOP/s of BF16 MMAs, so the 36 (45) digit pairs of a 56-bit (54-bit) cut cost a
-// fifteenth of the FP64 contraction: 744 -> 38 ms a product on a 2,000-atom protein (1.70 M pairs,
-// order 5), 54 ms beside the near field, which has the FP64 pipe to itself.  It is no less exact: with K = 4p^3 terms the FP64 chain of K multiply-adds leaves about
+// fifteenth of the FP64 contraction: 744 -> 37 ms a product on a 2,000-atom protein (1.70 M pairs,
+// order 5), 46 ms beside the near field, which has the FP64 pipe to itself.  It is no less exact: with K = 4p^3 terms the FP64 chain of K multiply-adds leaves about
 // sqrt(K / 2) 2^-53 of its partial sums, the cut 2^-57 (2^-55) of row and column maximum per term,
 // groups 0 .. 5 (0 .. 6) exact in FP32 (|G_k| <= K 2^(2D) (1 + (k - 1) / 4) <= 2^24 for K = 500,
 // D = 7 and K = 1372, D = 6) and the last two, 2^-42 below, sharing one accumulator.
