@@ -30,6 +30,7 @@
 #include <omp.h>
 
 #include "fmm_common.cuh"
+#include "fp64_seed.cuh"
 
 namespace ibim {
 
@@ -260,28 +261,11 @@ __device__ __forceinline__ double near64_f64(float v) {
     return __hiloint2double((b >> 3) + 0x38000000, b << 29);
 }
 
-// 1 / sqrt(d2) for normal d2 > 0 in three FP64 instructions, and sqrt(d2) to FP32 (at most 2^121).  The seed is
-// refined to 2^-44 on the FP32 and integer pipes, which are nearly idle here: d2 = 4^E2 (a + rho) with a the FP32
-// head in [1, 4); y = rsqrt(a) from FP32; the residual 1 - (a + rho) y^2 by FP32 multiply-adds (y^2 as head and
-// tail); y (1 + residual / 2) assembled in units of 2^-53.  Then y + y e, e = (1 - d2 y^2) / 2 of 2^-45.
+// 1 / sqrt(d2) for normal d2 > 0 in three FP64 instructions, and sqrt(d2) to FP32 (at most 2^121): the seed y of
+// 2^-44, y + y e with e = (1 - d2 y^2) / 2.
 __device__ __forceinline__ double near64_rsqrt(double d2, float &rf) {
-    const int hi = __double2hiint(d2);
-    const unsigned lo = __double2loint(d2);
-    const int E = (hi >> 20) - 1023, odd = E & 1, E2 = E >> 1;
-    const float a = __uint_as_float(((127u + odd) << 23) | (((unsigned)hi & 0xfffffu) << 3) | (lo >> 29));
-    const float rho = (float)(lo & 0x1fffffffu) * __int_as_float((127 - 52 + odd) << 23);
-    float yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(a));
-    rf = __int_as_float(__float_as_int(a * yf) + (min(E2, 120) << 23));
-    const float ph = yf * yf, pl = fmaf(yf, yf, -ph);
-    const float res = fmaf(-rho, ph, fmaf(-a, pl, fmaf(-a, ph, 1.f)));
-    const int inc = __float2int_rn(yf * res * 0x1p49f);  // half the residual in units of 2^-50: below 2^29
-    const int yb = __float_as_int(yf);
-    const long long Y = ((long long)((yb & 0x7fffff) | 0x800000) << ((yb >> 23) - 97)) + ((long long)inc << 3);
-    const int c = (int)(Y >> 53) & 1;  // y >= 1
-    const double y = __longlong_as_double((Y >> c) + ((long long)(1021 + c - E2) << 52));
-    const double mh = __hiloint2double((__double2hiint(y) - 0x00100000) ^ 0x80000000, __double2loint(y));  // -y / 2
-    return fma(y, fma(d2 * y, mh, 0.5), y);
+    const double y = rsqrt_seed(d2, rf);
+    return fma(y, fma(d2 * y, -half_of(y), 0.5), y);
 }
 
 // t = kappa r and e = e^-t = 2^{-n/512} 2^{-g}: n from the FP32 r, g exact, |g| <= 2^-10 (2^-9.7 where e is below

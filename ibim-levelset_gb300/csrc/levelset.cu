@@ -15,6 +15,7 @@
 // FP64 from the FP32 values).
 
 #include "f32x2.cuh"
+#include "fp64_seed.cuh"
 #include "internal.cuh"
 
 #include <cmath>
@@ -27,6 +28,7 @@ namespace {
 
 struct Dims {
     int nx, ny, nz;
+    double wg = 0.;  // (12 h)^-2 for the FP64 stages
     __device__ __forceinline__ long idx(int i, int j, int k) const { return ((long)i * ny + j) * nz + k; }
     __device__ __forceinline__ long cidx(int i, int j, int k) const {
         i = min(max(i, 0), nx - 1);
@@ -118,32 +120,18 @@ __global__ void k_expand(typename OrdT<T>::type *g, Dims d, double sx, double sy
 
 // Reciprocal and square root of the FP64 stencils.  A WENO stage as levelset.cpp writes it has 45
 // FP64 divisions a cell, each a dozen instructions of GB300's narrow FP64 pipe, which is what bounds
-// the stage; these take 3 to 6 from an FP32 seed made of the operand's own bits (the exponent is
-// handled apart, so any normal operand will do) and one cubic step, to about an ulp.
+// the stage; these take 2 to 3 from the seeds of 2^-44 (y + y e, e = 1 - x y or (1 - x y^2) / 2), to about an ulp.
 
-// 1 / x for normal x > 0: seed y within 2^-23, e = 1 - x y, y (1 + e + e^2).
-__device__ __forceinline__ double rcp64(double x) {
-    const int hi = __double2hiint(x);
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;"
-        : "=f"(y)
-        : "f"(__int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | ((unsigned)__double2loint(x) >> 29))));
-    const int yb = __float_as_int(y);
-    const double d = __hiloint2double((yb >> 3) + 0x38000000 - ((hi & 0x7ff00000) - 0x3ff00000), yb << 29);
-    const double e = fma(-x, d, 1.0);
-    return fma(d, fma(e, e, e), d);
+// n / x for normal x > 0.
+__device__ __forceinline__ double div64(double n, double x) {
+    const double y = rcp_seed(x);
+    return n * fma(y, fma(-x, y, 1.0), y);
 }
-// 1 / sqrt(x) for normal x > 0: seed of x 2^(-2k) in [1, 4), y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2.
+// 1 / sqrt(x) for normal x > 0.
 __device__ __forceinline__ double rsqrt64n(double x) {
-    const int hi = __double2hiint(x), E = (hi >> 20) - 1023;
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;"
-        : "=f"(y)
-        : "f"(__int_as_float(((127 + (E & 1)) << 23) | ((hi & 0xfffff) << 3) | ((unsigned)__double2loint(x) >> 29))));
-    const int yb = __float_as_int(y);
-    const double d = __hiloint2double((yb >> 3) + 0x38000000 - ((E >> 1) << 20), yb << 29);
-    const double e = fma(-(x * d), d, 1.0);
-    return fma(d * e, fma(e, 0.375, 0.5), d);
+    float r;
+    const double y = rsqrt_seed(x, r);
+    return fma(y, fma(x * y, -half_of(y), 0.5), y);
 }
 __device__ __forceinline__ bool is_normal_pos(double x) {
     return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u;
@@ -161,8 +149,9 @@ struct Div64 {
     __device__ static double over_sqrt(double x, double y) { return is_normal_pos(y) ? x * rsqrt64n(y) : x / sqrt(y); }
     __device__ static double root(double v) {
         if (!is_normal_pos(v)) return sqrt(v);
-        const double y = rsqrt64n(v), r = v * y;
-        return fma(fma(-r, r, v), 0.5 * y, r);
+        float f;
+        const double y = rsqrt_seed(v, f), r = v * y;  // v y = sqrt(v) (1 + 2^-44), squared away by the correction
+        return fma(fma(-r, r, v), half_of(y), r);
     }
     // max(x, 0) and max(-x, 0), 0 for NaN, and the larger of two such values: on the integer pipe
     __device__ static double pos(double x) {
@@ -224,8 +213,10 @@ __device__ __forceinline__ void weno5(const T w[7], T h, T &up, T &un) {
 //   12 h up = -b + 7 (c + d) - e - B + (4 q_1 q_2 A + 6 q_0 q_1 B) / S    (a .. f first differences,
 // A and B the second differences of the second differences), un its mirror image.  The indicators carry
 // 1/3 (13/3 x^2 + y^2; the weights do not change when every q does by the same factor) and
-// share their squares between the sides.  266 FP64 instructions a cell and stage instead of about 1070:
-// 2.0 -> 0.60 ms a stage on a 105^3 grid, the FP64 pipe 84 % busy.
+// share their squares between the sides.  The common factor 12 h stays with the caller, as (12 h)^-2 under the
+// norm's root (Dims::wg).  235 FP64 instructions a cell and stage instead of about 1070:
+// 2.0 -> 0.55 ms a stage on a 105^3 grid, the FP64 pipe 79 % busy (266 instructions, with cubic corrections of FP32
+// seeds and both factors applied cell by cell: 0.60 ms).
 // S holds eighth powers of differences: beyond 2^60 (and for infinities and NaN) the cell takes the
 // formulas as written.
 __device__ __noinline__ double2 weno5_wide(double w0, double w1, double w2, double w3, double w4, double w5, double w6,
@@ -235,7 +226,7 @@ __device__ __noinline__ double2 weno5_wide(double w0, double w1, double w2, doub
     weno5<double>(w, h, r.x, r.y);
     return r;
 }
-__device__ __forceinline__ void weno5(const double w[7], double h, double &up, double &un) {
+__device__ __forceinline__ void weno5_12h(const double w[7], double h, double &up, double &un) {
     const double EPS = 1e-6 / 3.0, K = 13.0 / 3.0;
     const double b1 = w[2] - w[1], c1 = w[3] - w[2], d1 = w[4] - w[3], e1 = w[5] - w[4];
     const double a = b1 - (w[1] - w[0]), b = c1 - b1, c = d1 - c1, d = e1 - d1, e = (w[6] - w[5]) - e1;
@@ -245,48 +236,57 @@ __device__ __forceinline__ void weno5(const double w[7], double h, double &up, d
                         __double2hiint(e) & 0x7fffffff);
     if (big >= (1023 + 60) << 20) {
         const double2 r = weno5_wide(w[0], w[1], w[2], w[3], w[4], w[5], w[6], h);
-        up = r.x;
-        un = r.y;
+        up = r.x * (12.0 * h);
+        un = r.y * (12.0 * h);
         return;
     }
     const double xed = e - d, xdc = d - c, xcb = c - b, xba = b - a;
     const double ped = fma(K * xed, xed, EPS), pdc = fma(K * xdc, xdc, EPS), pcb = fma(K * xcb, xcb, EPS),
                  pba = fma(K * xba, xba, EPS);
-    const double ih = rcp64(h) * (1.0 / 12.0);
-    const double B2 = xdc - xcb;
-    auto side = [](double p0, double y0, double p1, double y1, double p2, double y2, double A_, double B_) {
+    const double B2 = xdc - xcb, B3 = 1.5 * B2;
+    auto side = [B3](double p0, double y0, double p1, double y1, double p2, double y2, double A_) {
         double q0 = fma(y0, y0, p0), q1 = fma(y1, y1, p1), q2 = fma(y2, y2, p2);
         q0 *= q0;
         q1 *= q1;
         q2 *= q2;
         const double n0 = q1 * q2, n2 = q0 * q1;
         const double S = fma(6.0, q0 * q2, fma(3.0, n2, n0));
-        return fma(n0, A_, 1.5 * n2 * B_) * rcp64(S);  // (4 n0 A + 6 n2 B) / (4 S)
+        return div64(fma(n0, A_, n2 * B3), S);  // (4 n0 A + 6 n2 B) / (4 S)
     };
-    const double ru = side(ped, fma(-2.0, d, xed), pdc, d + c, pcb, fma(2.0, c, xcb), xed - xdc, B2);
-    const double rn = side(pba, fma(2.0, b, xba), pcb, b + c, pdc, fma(2.0, c, -xdc), xcb - xba, B2);
-    up = fma(4.0, ru, D - B2) * ih;
-    un = fma(-4.0, rn, D + B2) * ih;
+    const double ru = side(ped, fma(-2.0, d, xed), pdc, d + c, pcb, fma(2.0, c, xcb), xed - xdc);
+    const double rn = side(pba, fma(2.0, b, xba), pcb, b + c, pdc, fma(2.0, c, -xdc), xcb - xba);
+    up = fma(4.0, ru, D - B2);
+    un = fma(-4.0, rn, D + B2);
+}
+__device__ __forceinline__ void weno5(const double w[7], double h, double &up, double &un) {
+    weno5_12h(w, h, up, un);
+    const double ih = div64(1.0 / 12.0, h);
+    up *= ih;
+    un *= ih;
 }
 
-template <class T>
-__device__ __forceinline__ void gradients(const T *__restrict__ g, const Dims &dm, int i, int j, int k, T h, T up[3],
-                                          T un[3]) {
+template <class T, class F>
+__device__ __forceinline__ void for_axes(const T *__restrict__ g, const Dims &dm, int i, int j, int k, F f) {
     T w[7];
 #pragma unroll
     for (int l = 0; l < 7; ++l) w[l] = __ldg(g + dm.cidx(i - 3 + l, j, k));
-    weno5(w, h, up[0], un[0]);
+    f(w, 0);
 #pragma unroll
     for (int l = 0; l < 7; ++l) w[l] = __ldg(g + dm.cidx(i, j - 3 + l, k));
-    weno5(w, h, up[1], un[1]);
+    f(w, 1);
 #pragma unroll
     for (int l = 0; l < 7; ++l) w[l] = __ldg(g + dm.cidx(i, j, k - 3 + l));
-    weno5(w, h, up[2], un[2]);
+    f(w, 2);
+}
+template <class T>
+__device__ __forceinline__ void gradients(const T *__restrict__ g, const Dims &dm, int i, int j, int k, T h, T up[3],
+                                          T un[3]) {
+    for_axes(g, dm, i, j, k, [&](const T *w, int a) { weno5(w, h, up[a], un[a]); });
 }
 
-// levelset::getNorm(Dun, Dup) (levelset.cpp:294-301).
+// levelset::getNorm(Dun, Dup) (levelset.cpp:294-301), of derivatives that carry a common factor 1 / sqrt(f2).
 template <class T>
-__device__ __forceinline__ T godunov(const T n[3], const T p[3]) {
+__device__ __forceinline__ T godunov(const T n[3], const T p[3], T f2 = (T)1) {
     using D = typename DivOf<T>::type;
     T v = 0;
 #pragma unroll
@@ -294,7 +294,7 @@ __device__ __forceinline__ T godunov(const T n[3], const T p[3]) {
         const T m = D::larger(D::pos(n[a]), D::neg(p[a]));
         v += m * m;
     }
-    return D::root(v);
+    return D::root(v * f2);
 }
 
 // Counts and deviations of a block's threads (256 at most) into the grid's.
@@ -337,11 +337,11 @@ __device__ __forceinline__ void count_block(unsigned bad, unsigned tot, double a
 // COUNT (stage 0 only): also countGradient of src = g (levelset.cpp:398-432) from the same WENO
 // gradients: among cells with |g| < band, |godunov(D-, D+) - 1| > thres into counts[0], the
 // cells into counts[1], the sum of the deviations into accum.
-template <int MODE, int STAGE, class T, bool COUNT = false>
-__global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, const T *__restrict__ src, T *g, T *u1,
-                                                    T *u2, const T *__restrict__ phi0, T band = (T)0,
-                                                    T thres = (T)0, unsigned long long *counts = nullptr,
-                                                    double *accum = nullptr) {
+template <int MODE, int STAGE, bool COUNT = false>
+__global__ void __launch_bounds__(256)
+    k_weno_stage(Dims dm, double h, double dtv, double eps, const double *__restrict__ src, double *g, double *u1,
+                 double *u2, const double *__restrict__ phi0, double band = 0, double thres = 0,
+                 unsigned long long *counts = nullptr, double *accum = nullptr) {
     // consecutive cells to consecutive threads: the FP64 pipe takes as long for a warp at a row's end
     // with few cells as for a full one (a fifth of the warps of a 105^3 grid)
     int i, j, k;
@@ -361,31 +361,30 @@ __global__ void __launch_bounds__(256) k_weno_stage(Dims dm, T h, T dtv, T eps, 
     unsigned bad = 0, tot = 0;
     double acc = 0.;
     if (in) {
-        T up[3], un[3];
-        gradients(src, dm, i, j, k, h, up, un);
+        double up[3], un[3];
+        for_axes(src, dm, i, j, k, [&](const double *w, int a) { weno5_12h(w, h, up[a], un[a]); });
         const long I = dm.idx(i, j, k);
-        T L;
+        double L;
         if (MODE == 0) {
-            L = dtv * godunov(un, up);
+            L = dtv * godunov(un, up, dm.wg);
         } else {
-            const T p0 = phi0[I];
-            const T sign = DivOf<T>::type::over_sqrt(p0, p0 * p0 + eps);
-            const T nd = sign > (T)0 ? godunov(un, up) : godunov(up, un);
-            L = dtv * sign * (nd - (T)1.0);
+            const double p0 = phi0[I];
+            const double sign = Div64::over_sqrt(p0, p0 * p0 + eps);
+            const double nd = sign > 0 ? godunov(un, up, dm.wg) : godunov(up, un, dm.wg);
+            L = dtv * sign * (nd - 1.0);
         }
-        using D = typename DivOf<T>::type;
         if (COUNT && fabs(src[I]) < band) {
-            const T nr = godunov(un, up);
+            const double nr = godunov(un, up, dm.wg);
             tot = 1;
-            bad = fabs(nr - (T)1.0) > thres ? 1u : 0u;
-            acc = fabs((double)nr - 1.0);
+            bad = fabs(nr - 1.0) > thres ? 1u : 0u;
+            acc = fabs(nr - 1.0);
         }
         if (STAGE == 0)
             u1[I] = g[I] - L;
         else if (STAGE == 1)
-            u2[I] = (3 * g[I] + u1[I] - L) * (T)0.25;
+            u2[I] = (3 * g[I] + u1[I] - L) * 0.25;
         else
-            g[I] = D::third(g[I] + 2 * (u2[I] - L));
+            g[I] = Div64::third(g[I] + 2 * (u2[I] - L));
     }
     if (COUNT) count_block(bad, tot, acc, counts, accum);
 }
@@ -908,11 +907,12 @@ template <class T> inline void stage_shape(int nx, int ny, int nz, dim3 &gr, dim
 }
 template <int MODE, int STAGE, class T, bool COUNT = false> auto stage_kernel() {
     if constexpr (sizeof(T) == 8)
-        return k_weno_stage<MODE, STAGE, T, COUNT>;
+        return k_weno_stage<MODE, STAGE, COUNT>;
     else
         return k_weno_stage32<MODE, STAGE, COUNT>;
 }
-inline Dims dims_of(const Grid &g) { return Dims{g.nx, g.ny, g.nz}; }
+inline double stage_wg(double h) { return 1.0 / (144.0 * h * h); }
+inline Dims dims_of(const Grid &g) { return Dims{g.nx, g.ny, g.nz, stage_wg(g.dx)}; }
 
 template <class T> T *gdata(Grid &g);
 template <> double *gdata<double>(Grid &g) { return g.data.ptr; }
@@ -1308,14 +1308,14 @@ extern "C" int ibim_levelset_evolve_static(double *grid_dev, int nx, int ny, int
     double dt = cfl * dx / vel;
     const int steps = (int)(final_t / dt) + 1;
     dt = final_t / (double)steps;
-    const Dims dm{nx, ny, nz};
+    const Dims dm{nx, ny, nz, stage_wg(dx)};
     dim3 gr, bl;
     stage_shape<double>(nx, ny, nz, gr, bl);
     const double dtv = dt * vel;
     for (int st = 0; st < steps; ++st) {
-        (count_launch(), k_weno_stage<0, 0, double><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., grid_dev, grid_dev, u1, u2, nullptr));
-        (count_launch(), k_weno_stage<0, 1, double><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., u1, grid_dev, u1, u2, nullptr));
-        (count_launch(), k_weno_stage<0, 2, double><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., u2, grid_dev, u1, u2, nullptr));
+        (count_launch(), k_weno_stage<0, 0><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., grid_dev, grid_dev, u1, u2, nullptr));
+        (count_launch(), k_weno_stage<0, 1><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., u1, grid_dev, u1, u2, nullptr));
+        (count_launch(), k_weno_stage<0, 2><<<gr, bl, 0, s>>>(dm, dx, dtv, 0., u2, grid_dev, u1, u2, nullptr));
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) {
