@@ -1424,8 +1424,12 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
     // pass has the FP64 pipe to itself (2,000 atoms: 61.9 -> 56.9 ms a matvec).  It has to be resident
     // before the products' CTAs queue, which a lower priority would wait for: m2l_oz64_run calls fork
     // ahead of its split kernel.
-    const bool with_m2l = use_oz64 && S.nchunks_oz64 > 0;
-    const int side = near_side_ctas() > 0 ? near_side_ctas() * c->num_sms : full;
+    // So does the float-float one beside the residual's products, with two CTAs an SM (what their shared memory
+    // leaves) and a drain launch (2,000-atom solve: 86.4 ms of GMRES with the near field first, 85.1 and 84.8
+    // with one and two); merged plans, whose chunks stop molecule by molecule, gain nothing and keep it first.
+    const bool with_m2l = use_oz64 ? S.nchunks_oz64 > 0 : ff && use_oz && !P.batched && S.nchunks_oz > 0;
+    const int side = near_side_ctas() > 0 ? near_side_ctas() * c->num_sms
+                                          : std::min(full, ff && with_m2l ? 2 * c->num_sms : full);
     bool forked = false;
     auto fork = [&] {
         IBIM_CUDA(cudaEventRecord(c->ev_near_fork, s));
@@ -1445,7 +1449,7 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
         translate_up(P, nc, dens, P.mult.ptr);
         P.local.zero();
         if (use_oz) {
-            m2l_oz_run(P, S);
+            m2l_oz_run(P, S, beside);
         } else if (use_oz64) {
             m2l_oz64_run(P, S, entry, beside);
         } else if (S.nchunks > 0) {

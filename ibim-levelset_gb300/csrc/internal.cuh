@@ -461,7 +461,8 @@ void m2l_oz_pack(Plan &P, const float2 *ff = nullptr);
 void m2l_pack_images_ff(Plan &P, const float2 *ff);
 // Test check: the one-pass images equal the separate passes' word for word (throws otherwise).
 void m2l_check_images_ff(Plan &P, const float2 *ff);
-void m2l_oz_run(Plan &P, const TargetSet &S);
+// beside: as for m2l_oz64_run.
+void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside = nullptr);
 // The FP64 operator's M2L as digit products: bytes of one operator's images at order p (0: the order
 // has none), whether nops of them may be kept on this device, the buffers, the cut of n operators
 // (of places ids) from FP64 ones, one contraction.

@@ -2595,8 +2595,9 @@ void m2l_check_images_ff(Plan &P, const float2 *ff) {
 }
 
 // V-list M2L of the FP64 operator by digit products on the tensor cores; mult -> local.
-void m2l_oz_run(Plan &P, const TargetSet &S) {
+void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside) {
     if (S.nchunks_oz == 0) return;
+    if (beside) beside();
     cudaStream_t s = P.ctx->stream;
     const int n4 = 4 * P.R, ns = P.oz_s;
     const int gsplit = 4 * P.ctx->num_sms;
