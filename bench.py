@@ -529,7 +529,7 @@ def run_ours(args):
            "profiled_pass": {"ms_per_step": statistics.mean(prof_ms), "steps": args.steps,
                              "note": "per-category CUDA events around every launch, in a pass after the timed "
                                      "regions; categories on the main stream include waits for SMs held by the "
-                                     "near field on the second stream (m2m, p2m)"},
+                                     "near field on the second stream (p2m)"},
            "peaks_measured": {"fp64_tflops": fp64_peak, "fp32_tflops": fp32_peak,
                               "hbm_gbs": peaks.get("hbm_gbs"), "bf16_tflops": peaks.get("bf16_tflops")}}
     if rank == 0:

@@ -55,7 +55,9 @@ extern "C" {
 #define IBIM_KERNEL_BIE_FUSED 16
 
 /* ---- precision modes ---- */
-#define IBIM_PRECISION_FP64 0  /* reference-exact FP64 path */
+/* FP64 path; the M2L of orders up to 7 as digit products of 54 to 56 bits on the tensor cores, no less exact
+ * than the FP64 sums they replace (the FP64 sums themselves where the images do not fit a third of the device) */
+#define IBIM_PRECISION_FP64 0
 #define IBIM_PRECISION_MIXED 1 /* FP32-class far/near field inside FP64-class iterative refinement */
 /* FP64 operator whose V-list M2L runs on the tensor cores as exact products of BF16 integer
  * digits (Ozaki scheme, a 42-bit cut into 6 digits of 7 bits, or 7 of 6 bits from order 6 up,
@@ -291,8 +293,8 @@ int ibim_batch_solve(ibim_ctx ctx, int nmol, const int *natoms, const double *ce
 /* ---- launch-parameter table and autotuner (no counterpart in the reference) ----
  * A plan of Chebyshev order p with N sources takes its launch parameters from the row of order p
  * with the largest min_points <= N: pairs per work segment of the FP32 and the float-float near
- * fields, and the tensor-core M2L's launch form (2 = two CTAs of two row tiles per SM, 4 = one CTA
- * of four, 0 = persistent, 6 / 7 = CTA pairs of 2-SM MMAs with one / two row-tile pairs per CTA;
+ * fields, and the tensor-core M2L's launch form (2 = persistent CTA pairs from order 4 and 64 pairs an operator,
+ * else two CTAs of two row tiles per SM, 4 = one CTA of four, 0 = persistent, 6 / 7 = CTA pairs of 2-SM MMAs with one / two row-tile pairs per CTA;
  * 0, 6 and 7 in the scaled FP16 operand form).  They change the partition of the same work only.
  * Without a row the defaults hold (2^17, 2^14, 2). */
 int ibim_tuning_set(int order, long min_points, long near_seg_pairs, long nearff_seg_pairs, int tc_form);
