@@ -103,21 +103,33 @@ __device__ __forceinline__ void cp_async16(uint32_t saddr, const void *g, uint32
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr), "l"(g), "r"(src_bytes));
 }
 
-// Wait for the mbarrier phase with the given parity; false when the bound is exceeded.
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+// Wait for the mbarrier phase with the given parity; false when the bound is exceeded.  CLUSTER: the phase counts
+// arrivals of the pair's other CTA's threads, whose work the wait has to acquire too.  (A commit's arrive, on either
+// CTA's barrier, is the completion of asynchronous operations and takes the plain wait, as a bulk copy's does.)
+template <bool CLUSTER = false> __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     for (long it = 0; it < TC_WAIT_LIMIT; ++it) {
         uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(mbar), "r"(parity)
-            : "memory");
+        if constexpr (CLUSTER)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(mbar), "r"(parity)
+                : "memory");
+        else
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(mbar), "r"(parity)
+                : "memory");
         if (ok) return true;
     }
     return false;
 }
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t mbar, uint32_t parity) { return mbar_wait<true>(mbar, parity); }
 
 // Byte offset of element (row, 4 * kchunk) of a 128 x 8 tile in the canonical no-swizzle
 // K-major layout: core matrix (row / 8, kchunk) at ((row / 8) * 2 + kchunk) * 128, row % 8 at 16 B.
@@ -796,7 +808,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
                 const int buf = st % TC2_NST;
                 const uint32_t par = (uint32_t)((st / TC2_NST) & 1);
                 if (!mbar_wait(smem_u32(&full_a[buf]), par) || !mbar_wait(smem_u32(&full_b[buf]), par) ||
-                    !mbar_wait(smem_u32(&peer_full[buf]), par) || abort_s) {
+                    !mbar_wait_cluster(smem_u32(&peer_full[buf]), par) || abort_s) {
                     abort_s = 1;
                     break;
                 }
@@ -931,12 +943,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 // tile_base + 2T in the even CTA and tile_base + 2T + 1 in the odd one; the chunk's MMA width N
 // is its pair count rounded up to 16, each CTA gathering N / 2 multipole rows.  Barriers as in
 // the TF32 pair kernel (k_m2l_tc2): the odd CTA's relay thread passes its full stages to the
-// even CTA (a relaxed arrive: the release form's cluster-scope fence on every stage made the kernel
-// 3.62 instead of 2.62 ms a launch), whose MMA thread multicasts its commits to both CTAs; every
+// even CTA, whose MMA thread multicasts its commits to both CTAs; every
 // wait is bounded, and both CTAs meet at cluster barriers only on paths every thread takes.  The
-// epilogue applies the FP16 form's row and column scales.  Measured on the 2,000-atom protein:
-// 2.56 ms a launch (one row-tile pair per CTA, two CTAs per SM) against 2.34 ms for two CTAs of
-// two row tiles per SM, so it is a launch form the tuning table may pick (6, 7), not the default.
+// epilogue applies the FP16 form's row and column scales.  The relay releases at cluster scope on every
+// stage: 3.62 ms a launch on the 2,000-atom protein, where two CTAs of two row tiles per SM take 2.34, so it is
+// a launch form the tuning table may pick (6, 7), not the default.  (A relaxed arrive, 2.62 ms, hands the odd CTA's
+// copies to no one.)
 // ---------------------------------------------------------------------------------------------
 template <int PT> struct Tc2hShape {
     static constexpr int STAGE = (2 * PT + 2) * TC_TILE_BYTES;  // operator hi/lo per row tile + multipole hi/lo
@@ -1060,7 +1072,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, PT == 1 
                 const int buf = st % NST;
                 const uint32_t par = (uint32_t)((st / NST) & 1);
                 if (!mbar_wait(smem_u32(&full_a[buf]), par) || !mbar_wait(smem_u32(&full_b[buf]), par) ||
-                    !mbar_wait(smem_u32(&peer_full[buf]), par) || abort_s) {
+                    !mbar_wait_cluster(smem_u32(&peer_full[buf]), par) || abort_s) {
                     abort_s = 1;
                     break;
                 }
@@ -1091,9 +1103,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, PT == 1 
                     abort_s = 1;
                     break;
                 }
-                // relaxed: the data this stage holds is already in this CTA's shared memory (the
-                // waits above acquired its completion) and is read there by this SM's tensor core
-                asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
                                  cluster_addr(smem_u32(&peer_full[buf]), 0))
                              : "memory");
             }
@@ -1215,9 +1225,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, PT == 1 
 // CTA's MMA thread issues for the pair and its commits free a stage in both, eight warps drain one
 // accumulator slot of 256 TMEM columns while the next unit's MMAs fill the other (four warps, eight
 // columns a step, took longer than the MMAs).
-// 4.14 -> 2.48 ms, 0.77 of the tensor rate; without its MMAs' last two products 2.14, without gathers 2.12,
-// without the adds into the locals 2.20: no one part bounds it.  At order 6 on 200 atoms (100 pairs an
-// operator) 1.21 -> 1.13 ms: 4.6 GB of operators out of HBM take 0.68.
+// 4.14 -> 2.84 ms alone, 0.67 of the tensor rate, of which the hand-over below takes 0.36; of the rest (2.48), without
+// its MMAs' last two products 2.14, without gathers 2.12, without the adds into the locals 2.20: no one part bounds it.
+// Hand-over of the odd CTA's multipole rows to the even CTA's MMA thread: each gathering lane's cp.async have landed
+// (wait_group) and are fenced to the async proxy; __syncwarp and lane 0's arrive release them in the odd CTA; its relay
+// thread's wait acquires them there and its arrive releases them at cluster scope; the MMA thread's wait acquires at
+// cluster scope.  One thread with no copies of its own pays the cluster-scope fence, off the gathering warps' path
+// (beside the near field on 5,000 atoms 3.16 ms; each gathering warp's lane 0 releasing at cluster scope itself 3.91, one
+// of them after a barrier of the four 3.70).
 // Every wait is bounded; one that runs out sets the error word and ends the CTA's roles.
 // ---------------------------------------------------------------------------------------------
 constexpr int HP_N = 256, HP_KB = 64, HP_NST = 3;
@@ -1273,8 +1288,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HP_THREADS, 2)  // 7
     if (tid == 0) {
         abort_s = 0;
         for (int i = 0; i < HP_NST; ++i) {
-            // the operator copies' expected bytes and both CTAs' gathering warps
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[i])), "r"(1 + 2 * HP_GATHER));
+            // this CTA's gathering warps; the even one's also the operator copies' expected bytes and the odd one's relay
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&full[i])),
+                         "r"(HP_GATHER + (rank == 0 ? 2 : 0)));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[i])));
         }
         for (int i = 0; i < 2; ++i) {
@@ -1335,12 +1351,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HP_THREADS, 2)  // 7
                 const int chunk = u / npt;
                 const uint32_t idesc = IDESC0 | ((uint32_t)(width(chunks[3 * chunk + 2]) >> 3) << 17);
                 const int slot = n & 1;
-                if (n >= 2) ok = mbar_wait(smem_u32(&acc_empty[slot]), (uint32_t)(((n >> 1) - 1) & 1));
+                if (n >= 2) ok = mbar_wait_cluster(smem_u32(&acc_empty[slot]), (uint32_t)(((n >> 1) - 1) & 1));
                 asm volatile("tcgen05.fence::after_thread_sync;");
                 const uint32_t d = tmem_d + (uint32_t)(slot * HP_N);
                 for (int kb = 0; kb < nkb && ok; ++kb, ++st) {
                     const int buf = (int)(st % HP_NST);
-                    ok = mbar_wait(smem_u32(&full[buf]), (uint32_t)((st / HP_NST) & 1)) && !abort_s;
+                    ok = mbar_wait_cluster(smem_u32(&full[buf]), (uint32_t)((st / HP_NST) & 1)) && !abort_s;
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;");
                     const uint32_t base = smem + (uint32_t)buf * HP_STAGE;
@@ -1360,6 +1376,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HP_THREADS, 2)  // 7
                 ++n;
             }
             if (!ok) abort_s = 1;
+        } else if (lane == 0) {  // odd CTA: its gathered stages handed to the even one's MMA thread
+            long st = 0;
+            bool ok = true;
+            for (int u = cluster; u < nunits && ok; u += nclusters)
+                for (int kb = 0; kb < nkb; ++kb, ++st) {
+                    const int buf = (int)(st % HP_NST);
+                    ok = mbar_wait(smem_u32(&full[buf]), (uint32_t)((st / HP_NST) & 1)) && !abort_s;
+                    if (!ok) break;
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                                     cluster_addr(smem_u32(&full[buf]), 0))
+                                 : "memory");
+                }
+            if (!ok) abort_s = 1;
         }
         __syncwarp();
     } else if (warp < 2 + HP_GATHER) {
@@ -1376,10 +1405,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HP_THREADS, 2)  // 7
         auto signal = [&](long s2) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0)  // relaxed: the data lies in this CTA's shared memory, read there by its tensor core
-                asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(
-                                 cluster_addr(smem_u32(&full[(int)(s2 % HP_NST)]), 0))
-                             : "memory");
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[(int)(s2 % HP_NST)])) : "memory");
         };
         for (int u = cluster; u < nunits && ok; u += nclusters) {
             const int chunk = u / npt;
@@ -2283,10 +2310,11 @@ static CUtensorMap map_2d(const void *base, long rows, long cols, int box_rows, 
 // better than a persistent one that takes each SM (eight molecules of 50 to 400 atoms: 171 against 199 ms).
 static bool tc_pair_form(const Plan &P) { return P.tc_h16 && P.tune.tc_form == 2 && P.p >= 4 && !P.batched; }
 
-// From 64 pairs an operator: with few, a unit is the copy of its operator and the one-CTA form's smaller
-// units overlap better (20 pairs an operator, 60 atoms: 0.18 ms against 0.16; 100 at order 6, 200 atoms:
-// 1.13 against 1.21).
-bool m2l_tc_pairs(const Plan &P, const TargetSet &S) { return tc_pair_form(P) && S.nvpairs >= 64L * P.nops; }
+// From 128 pairs an operator (one full chunk of the one-CTA form): with fewer, a unit is the copy of its operator, and
+// the one-CTA form's smaller units, without a hand-over between CTAs, overlap better (pairs an operator: 60 at order 4
+// 0.112 ms against 0.102; 97 at order 6 1.48 against 1.29, at order 5 0.47 both; 236 at order 5 0.96 against 1.22, at
+// order 6 3.13 against 3.29; 540 at order 5 1.80 against 2.54).
+bool m2l_tc_pairs(const Plan &P, const TargetSet &S) { return tc_pair_form(P) && S.nvpairs >= 128L * P.nops; }
 
 static void tc_maps(Plan &P) {
     if (!tc_pair_form(P)) return;
