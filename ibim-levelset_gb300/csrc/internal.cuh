@@ -380,7 +380,8 @@ struct Plan {
     double oz_key[5] = {-1, -1, -1, -1, -1};
     int oz_kpad = 0, oz_mtiles = 0, oz_s = 7;  // digit images: K padded, row tiles, digits
     DevBuf<uint16_t> oz_a, oz_b;
-    DevBuf<double> oz_sig, oz_tau;
+    DevBuf<double> oz_sig;
+    DevBuf<int> oz_tau;
     // the FP64 operator's own digit images (m2l_oz64_run), on FP64 plans whose images fit (oz64_ok)
     bool oz64_ok = false;
     struct Oz64 {
@@ -392,7 +393,7 @@ struct Plan {
     } oz64[ENTRY_BLOCK + 1];               // of the block's entries (built when asked for) and of the whole block
     int oz64_s = 8;                        // digits
     DevBuf<uint16_t> oz64_b;               // the multipoles' digits and scales
-    DevBuf<double> oz64_tau;
+    DevBuf<int> oz64_tau;
     double kp64[5] = {-1, -1, -1, -1, -1}, kp32[5] = {-1, -1, -1, -1, -1};  // kernel parameters of the cached operators
     bool ops64_ready = false, ops32_ready = false;
     // a plan merged over several molecules (batch.cu): the molecule of every node and each

@@ -20,6 +20,7 @@
 // into the target nodes' local expansions.
 
 #include <atomic>
+#include <cfloat>
 #include <cstdint>
 #include <cstdlib>
 #include <functional>
@@ -1825,11 +1826,23 @@ __device__ __forceinline__ void oz_digits(float2 v, int e, uint16_t *dig) {
     oz_digits_of<S>((f + (1LL << 15)) >> 16, dig);
 }
 
+// Scale exponent of an operator row or a node that holds a NaN or an infinity: integers cannot carry it, so the
+// digits are zeros, and the epilogue adds a NaN wherever that exponent takes part, as an FP64 sum over the row would.
+constexpr int OZ_NONFINITE = 1 << 20;
+__device__ __forceinline__ bool oz_nonfinite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+
 // Power-of-two scale >= m (1 for m == 0), returned as its exponent.
 __device__ __forceinline__ int oz_scale_exp(double m) {
     if (!(m > 0.0)) return 0;
     int e;
     frexp(m, &e);  // m = f 2^e, f in [0.5, 1)
+    return e;
+}
+
+__device__ __forceinline__ int oz_scale_exp_f32(float m) {
+    if (!(m > 0.f)) return 0;
+    int e;
+    frexpf(m, &e);  // m = f 2^e, f in [0.5, 1)
     return e;
 }
 
@@ -1840,18 +1853,19 @@ __device__ __forceinline__ int row_scale_exp(const double *__restrict__ col0, in
     unsigned long long mb = 0;
     for (int k = 0; k < n4; ++k)
         mb = max(mb, (unsigned long long)__double_as_longlong(col0[(long)k * n4]) & 0x7fffffffffffffffULL);
-    return oz_scale_exp(__longlong_as_double((long long)mb));
+    const double m = __longlong_as_double((long long)mb);
+    return oz_nonfinite(m) ? OZ_NONFINITE : oz_scale_exp(m);
 }
 __device__ __forceinline__ int row_scale_exp(const float2 *__restrict__ col0, int n4) {
     float m = 0.f;
+    bool fin = true;
     for (int k = 0; k < n4; ++k) {
         const float2 x = col0[(long)k * n4];
-        m = fmaxf(m, fabsf(x.x) + fabsf(x.y));
+        const float v = fabsf(x.x) + fabsf(x.y);
+        m = fmaxf(m, v);
+        fin = fin && v <= FLT_MAX;
     }
-    if (!(m > 0.f)) return 0;
-    int e;
-    frexpf(m, &e);  // m = f 2^e, f in [0.5, 1)
-    return e;
+    return fin ? oz_scale_exp_f32(m) : OZ_NONFINITE;
 }
 
 // Row scales of the operators (FP64 or float-float, column-major n4 x n4 per op):
@@ -1897,7 +1911,7 @@ __global__ void k_pack_ops_oz(int n4, int mtiles, int kpad, int nops, const OW *
             const int k = grp * 8 + q;
             const OW v = (r < n4 && k < n4) ? ops[(long)op * n4 * n4 + (long)k * n4 + r] : OW{};
             uint16_t dig[S];
-            oz_digits<S>(v, e, dig);
+            oz_digits<S>(e == OZ_NONFINITE ? OW{} : v, e, dig);
 #pragma unroll
             for (int d = 0; d < S; ++d) {
                 if (q & 1) w[d][q >> 1] |= (uint32_t)dig[d] << 16;
@@ -1942,26 +1956,28 @@ __global__ void k_scale_ops_ff2(int n4, int mtiles, int nops, int scale_exp, con
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
         const int r = (int)(i % mpad), op = (int)(i / mpad);
         float m = 0.f;
+        bool fin = true;
         if (r < n4) {
             const float2 *col0 = ops + (long)op * n4 * n4 + r;
             for (int k = 0; k < n4; ++k) {
                 const float2 x = col0[(long)k * n4];
-                m = fmaxf(m, fabsf(x.x) + fabsf(x.y));
+                const float v = fabsf(x.x) + fabsf(x.y);
+                m = fmaxf(m, v);
+                fin = fin && v <= FLT_MAX;
             }
         }
-        int e = 0;
-        if (m > 0.f) frexpf(m, &e);  // m = f 2^e, f in [0.5, 1)
+        const int e = fin ? oz_scale_exp_f32(m) : OZ_NONFINITE;
         rscale[i] = h16_scale(m);
         sig[i] = ldexp(1.0, e - scale_exp);
         sexp[i] = e;
     }
 }
 
-// Multipoles (FP64 [node][n4]) -> digits [node][stage][digit][16] and column scales tau = t_j.
+// Multipoles (FP64 [node][n4]) -> digits [node][stage][digit][16] and the exponents tau of the column scales t_j.
 // One warp per node.
 template <int S>
 __global__ void k_split_mult_oz(long nnodes, int n4, int kpad, const double *__restrict__ mult, uint16_t *b,
-                                double *tau) {
+                                int *tau) {
     const int lane = threadIdx.x & 31;
     const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1969,13 +1985,18 @@ __global__ void k_split_mult_oz(long nnodes, int n4, int kpad, const double *__r
     for (long node = warp; node < nnodes; node += nwarps) {
         const double *m = mult + node * n4;
         double mx = 0.0;
-        for (int k = lane; k < n4; k += 32) mx = fmax(mx, fabs(m[k]));
+        bool bad = false;
+        for (int k = lane; k < n4; k += 32) {
+            mx = fmax(mx, fabs(m[k]));
+            bad = bad || oz_nonfinite(m[k]);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const int e = oz_scale_exp(mx);
-        if (lane == 0) tau[node] = ldexp(1.0, e);
+        bad = __any_sync(0xffffffffu, bad);
+        const int e = bad ? OZ_NONFINITE : oz_scale_exp(mx);
+        if (lane == 0) tau[node] = e;
         for (int k = lane; k < kpad; k += 32) {
-            const double v = k < n4 ? m[k] : 0.0;
+            const double v = k < n4 && !bad ? m[k] : 0.0;
             uint16_t dig[S];
             oz_digits<S>(v, e, dig);
             const long base = ((node * nstage + k / OZ_KS) * S) * OZ_KS + (k % OZ_KS);
@@ -1985,17 +2006,22 @@ __global__ void k_split_mult_oz(long nnodes, int n4, int kpad, const double *__r
     }
 }
 
-// Exponent e of a positive power of two 2^e (normal range), from its bits.
+// Exponent e of a positive power of two 2^e (normal range), from its bits; infinity: OZ_NONFINITE.
 __device__ __forceinline__ int exp_of_pow2(double p) {
-    return (int)((__double_as_longlong(p) >> 52) & 0x7ff) - 1023;
+    const int e = (int)((__double_as_longlong(p) >> 52) & 0x7ff) - 1023;
+    return e > 1023 ? OZ_NONFINITE : e;
 }
 
 // The double nearest T 2^e (ties away from zero) for an integer 0 < |T| < 2^63, assembled from T's bits by integer
-// instructions while the result is a normal number, else by an FP64 multiply.
+// instructions while the result is a normal number, else by an FP64 multiply.  A NaN for the exponents that
+// OZ_NONFINITE takes part in, whatever T.
 __device__ __forceinline__ double pow2_scaled_ll(long long T, const int e) {
     const unsigned long long a = (unsigned long long)(T < 0 ? -T : T);
     const int lz = __clzll((long long)a), E = 63 - lz + e + 1023;  // biased exponent of the result
-    if (E < 1 || E > 2046) return ldexp((double)T, e);             // subnormal or overflowing result
+    if (E < 1 || E > 2046) {                                       // subnormal or overflowing result
+        if (e >= OZ_NONFINITE / 2) return __longlong_as_double(0x7ff8000000000000LL);
+        return ldexp((double)T, e);
+    }
     // 53 bits rounded; their leading one (and a carry beyond it) adds to the exponent field
     const unsigned long long m = ((a << (lz - 1)) + 512) >> 10;
     const unsigned long long bits = ((unsigned long long)(unsigned)(E - 1) << 52) + m;
@@ -2015,7 +2041,7 @@ template <int S>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_m2l_oz(int n4, int kpad, int mtiles, const int *__restrict__ chunks, const int *__restrict__ vsrc,
              const int *__restrict__ vtgt, const uint16_t *__restrict__ a, const double *__restrict__ sig,
-             const uint16_t *__restrict__ bdig, const double *__restrict__ tau, double *local, int *err,
+             const uint16_t *__restrict__ bdig, const int *__restrict__ tau, double *local, int *err,
              const int *__restrict__ chunk_mol, const int *__restrict__ mol_active,
              const MolImg *__restrict__ mol_img) {
     // a merged plan (batch.cu): chunks of molecules that have stopped iterating are skipped whole,
@@ -2046,7 +2072,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int sn = tid < cnt ? vsrc[b + tid] : -1;
         src_s[tid] = sn;
         tgt_s[tid] = tid < cnt ? vtgt[b + tid] : -1;
-        tau_e[tid] = sn >= 0 ? exp_of_pow2(tau[sn]) : 0;
+        tau_e[tid] = sn >= 0 ? tau[sn] : 0;
     }
     if (tid == 0) {
         abort_s = 0;
@@ -2225,8 +2251,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     int sh = F - F0;
                     if (S > 7) sh = min(26, max(1, __clzll(T < 0 ? -T : T) - 2));
                     T = (T << sh) + f32_fixed(__uint_as_float(v[OZ_ACC - 1][q]), F0 + sh);
-                    if (tg >= 0 && T != 0)
-                        atomicAdd(local + (long)tg * n4 + row, pow2_scaled_ll(T, erow + tau_e[c0 + q] - F0 - sh));
+                    const int e = erow + tau_e[c0 + q] - F0 - sh;
+                    if (tg >= 0 && (T != 0 || e >= OZ_NONFINITE / 2))
+                        atomicAdd(local + (long)tg * n4 + row, pow2_scaled_ll(T, e));
                 }
             }
         }
