@@ -249,6 +249,8 @@ Near64K make_near64(const KParams &k) {
     return n;
 }
 
+__device__ __forceinline__ bool nonfinite64(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+
 // FP32 value of a double below 2^127 in magnitude by its bits (truncated; below 2^-126: 0).
 __device__ __forceinline__ float near64_f32(double v) {
     const unsigned hi = __double2hiint(v), mag = hi & 0x7fffffff;
@@ -368,6 +370,8 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
              const double *__restrict__ local, double *out, int l2p_mask, int nseg, int *next, int ax_in, int ax_out) {
     constexpr int NC = KIND == NEAR_BLOCK ? 4 : 1;
     constexpr bool FG = KIND == NEAR_K1 || KIND == NEAR_K2;  // the one output is F
+    // Without screening K2 and K3 are zero and their terms are left out, but for NaN and infinite densities
+    constexpr bool ZEROS = MODE == NEAR_LAPLACE && (NC == 4 || KIND == NEAR_K2 || KIND == NEAR_K3);
     // x y | z m_x | m_y m_z | psi n_x | n_y n_z (n = m / 3), one kernel: x y | z m
     __shared__ double2 S[NEAR_TILE][NC == 4 ? 5 : 2];
     __shared__ double e2[MODE == NEAR_YUKAWA ? NEAR_EXP : 1];  // 2^(-j / 512)
@@ -409,25 +413,32 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                     __syncthreads();
                     // two threads a source
                     const int q = threadIdx.x >> 1;
+                    bool bad = false;  // (ZEROS) a NaN or an infinity
                     if (q < cnt) {
                         const long i = s0 + q;
                         if constexpr (NC == 1) {
-                            if (threadIdx.x & 1)
-                                S[q][1] = make_double2(sz[i], KIND == NEAR_K2 || KIND == NEAR_K4 ? dens[i] * psi_f : dens[i]);
-                            else
+                            if (threadIdx.x & 1) {
+                                const double m = dens[i];
+                                bad = nonfinite64(m);
+                                S[q][1] = make_double2(sz[i], KIND == NEAR_K2 || KIND == NEAR_K4 ? m * psi_f : m);
+                            } else
                                 S[q][0] = make_double2(sx[i], sy[i]);
                         } else if (threadIdx.x & 1) {
-                            const double m1 = dens[ns + i], m2 = dens[2 * ns + i];
+                            const double m1 = dens[ns + i], m2 = dens[2 * ns + i], psi = dens[3 * ns + i];
+                            bad = nonfinite64(m1) || nonfinite64(m2) || nonfinite64(psi);
                             S[q][2] = make_double2(m1, m2);
                             S[q][4] = make_double2(m1 * (1.0 / 3.0), m2 * (1.0 / 3.0));
-                            S[q][3].x = dens[3 * ns + i] * psi_f;
+                            S[q][3].x = psi * psi_f;
                         } else {
+                            const double m0 = dens[i];
+                            bad = nonfinite64(m0);
                             S[q][0] = make_double2(sx[i], sy[i]);
-                            S[q][1] = make_double2(sz[i], dens[i]);
-                            S[q][3].y = dens[i] * (1.0 / 3.0);
+                            S[q][1] = make_double2(sz[i], m0);
+                            S[q][3].y = m0 * (1.0 / 3.0);
                         }
                     }
-                    __syncthreads();
+                    if constexpr (ZEROS) bad = __syncthreads_or(bad);
+                    else __syncthreads();
                     if (active)
 #pragma unroll 2  // two pairs in flight a warp: 50.4 -> 48.1 ms for the electrostatics of 100 atoms
                         for (int q2 = ph; q2 < cnt; q2 += nph) {
@@ -445,6 +456,21 @@ __global__ void __launch_bounds__(NEAR_T, 3)  // 80 registers: two CTAs leave th
                                                   a4.y, acc);
                             }
                         }
+                    if constexpr (ZEROS)
+                        if (bad && active)  // 0 times them
+                            for (int q2 = ph; q2 < cnt; q2 += nph) {
+                                const double2 a0 = S[q2][0], a1 = S[q2][1];
+                                const double dx = a0.x - X, dy = a0.y - Y, dz = a1.x - Z;
+                                const bool inside = fma(dx, dx, fma(dy, dy, dz * dz)) < kp.vr2;
+                                if constexpr (NC == 1) {
+                                    if (KIND == NEAR_K2 || !inside) acc[0] += 0.0 * a1.y;
+                                } else {
+                                    acc[0] += 0.0 * S[q2][3].x;
+                                    const double dm = fma(dx, a1.y, fma(dy, S[q2][2].x, dz * S[q2][2].y));
+                                    if (!inside)
+                                        for (int o = 1; o < 4; ++o) acc[o] += 0.0 * dm;
+                                }
+                            }
                 }
             }
             if (MODE != NEAR_GENERAL) {

@@ -318,6 +318,45 @@ __device__ __forceinline__ float exp2_ftz(float x) {
     return y;
 }
 
+constexpr int NT32 = 128, NW32 = NT32 / 32, TILE32 = 64;  // threads, warps, sources a warp's tile
+
+__device__ __forceinline__ bool nonfinite32(float v) { return (__float_as_int(v) & 0x7f800000) == 0x7f800000; }
+
+// A lane's share of a tile that holds a NaN or an infinite density, pair by pair with every term as the formulas have
+// it: k_near32's packed form leaves out what is zero without screening and multiplies by zero inside the cutoff.
+// S: x, y, z, q m, q psi / k3q, source index; G without its factor k3q.
+__device__ __noinline__ float4 near32_as_written(const float (*S)[TILE32], int begin, int end, int step, float X, float Y,
+                                                 float Z, float kap, float kl2, float k2q, float eps, float ieps, float k3q,
+                                                 float vr2, float vr2_band, double vr2_64, const double *sx64,
+                                                 const double *sy64, const double *sz64, double tx, double ty, double tz) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q4 = begin; q4 < end; q4 += step)
+        for (int q = q4; q < q4 + 4; ++q) {
+            const float dx = S[0][q] - X, dy = S[1][q] - Y, dz = S[2][q] - Z, d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            const float psi = S[6][q] * k3q;
+            bool inside = d2 < vr2;
+            if (fabsf(d2 - vr2) < vr2_band) {
+                const int sj = __float_as_int(S[7][q]);
+                const double ex = sx64[sj] - tx, ey = sy64[sj] - ty, ez = sz64[sj] - tz;
+                inside = ex * ex + ey * ey + ez * ez < vr2_64;
+            }
+            if (inside) {
+                a.x = fmaf(-k2q, psi, a.x);
+                continue;
+            }
+            const float ir = rsqrt_ftz(d2), r = d2 * ir, ir2 = ir * ir, ir3 = ir2 * ir;
+            const float t = kap * r, e = exp2_ftz(kl2 * r), et1 = fmaf(e, t, e);
+            const float m0 = S[3][q], m1 = S[4][q], m2 = S[5][q], M = fmaf(dx, m0, fmaf(dy, m1, dz * m2)) * ir3;
+            a.x = fmaf(fmaf(eps, et1, -1.f), M, fmaf(-(1.f - e) * ir, psi, a.x));
+            const float cm = fmaf(fmaf(e, fmaf(t + 3.f, t, 3.f), -3.f) * ir2, M, fmaf(ieps, et1, -1.f) * S[6][q] * ir3);
+            const float hd = (1.f - et1) * ir3;
+            a.y = fmaf(dx, cm, fmaf(hd, m0, a.y));
+            a.z = fmaf(dy, cm, fmaf(hd, m1, a.z));
+            a.w = fmaf(dz, cm, fmaf(hd, m2, a.w));
+        }
+    return a;
+}
+
 // Near field + L2P in FP32 for one target leaf per block: source leaves staged in shared memory
 // in the target leaf's frame; per-tile partial sums are added with Kahan compensation.
 //
@@ -331,7 +370,6 @@ __device__ __forceinline__ float exp2_ftz(float x) {
 // taken by a quarter of the warps' steps.  K1 and K3 share M = d.m / r^3; G and psi carry K3's factor (k3q) outside
 // the pair loop.  Alone, on 2.05e9 pairs (5,000 atoms): 4.4 -> 3.6 ms; on 5.6e7 pairs (200 atoms, order 6):
 // 0.48 -> 0.16 ms.
-constexpr int NT32 = 128, NW32 = NT32 / 32, TILE32 = 64;  // threads, warps, sources a warp's tile
 // BATCH: a plan merged over several molecules (batch.cu); the kappa-dependent constants come from
 // the target leaf's molecule (kmol: kappa, -kappa log2 e, k2in / q4pi per molecule).
 template <bool BATCH>
@@ -397,6 +435,7 @@ __global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restri
             while (rr < r1) {
                 __syncwarp();
                 int filled = 0;
+                bool bad = false;  // a NaN or an infinity among the densities
                 // sequentially pack up to TILE32 sources; each lane copies its slots
                 int lrr = rr, lpos = pos;
                 while (lrr < r1 && filled < TILE32) {
@@ -411,6 +450,7 @@ __global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restri
                         const int sj = lpos + (own ? q : take - 1);
                         const float4 A = __ldg(src8 + 2 * sj), B = __ldg(src8 + 2 * sj + 1);
                         const int d = filled + q;
+                        bad = bad || nonfinite32(A.w) || nonfinite32(B.x) || nonfinite32(B.y) || nonfinite32(B.z);
                         S8[0][d] = A.x + ox;
                         S8[1][d] = A.y + oy;
                         S8[2][d] = A.z + oz;
@@ -430,12 +470,13 @@ __global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restri
                 rr = lrr;
                 pos = lpos;
                 __syncwarp();
+                bad = __any_sync(0xffffffffu, bad);
                 if (active) {
                     f2 a0 = 0ull, a1 = 0ull, a2 = 0ull, a3 = 0ull;
                     float ain = 0.f;
                     // the densities carry 1 / (4 pi): the K1, K2, K4 factors lose it and the K3 ones
                     // take k3f / q4pi (near_pair64 has the unscaled form)
-                    for (int q = 4 * ph; q < filled; q += 4 * nph) {
+                    for (int q = bad ? filled : 4 * ph; q < filled; q += 4 * nph) {
                         const ulonglong2 xs = *reinterpret_cast<const ulonglong2 *>(&S8[0][q]),
                                          ys = *reinterpret_cast<const ulonglong2 *>(&S8[1][q]),
                                          zs = *reinterpret_cast<const ulonglong2 *>(&S8[2][q]);
@@ -504,7 +545,16 @@ __global__ void __launch_bounds__(NT32, 5) k_near32(const ChebTables32 *__restri
                         }
                     }
                     const float2 b0 = up2(a0), b1 = up2(a1), b2 = up2(a2), b3 = up2(a3);
-                    const float part[4] = {fmaf(-k2q * kp.k3q, ain, b0.x + b0.y), b1.x + b1.y, b2.x + b2.y, b3.x + b3.y};
+                    float part[4] = {fmaf(-k2q * kp.k3q, ain, b0.x + b0.y), b1.x + b1.y, b2.x + b2.y, b3.x + b3.y};
+                    if (bad) {
+                        const float4 a = near32_as_written(S8, 4 * ph, filled, 4 * nph, X, Y, Z, kap, kl2, k2q, kp.eps,
+                                                           kp.ieps, kp.k3q, kp.vr2, kp.vr2_band, kp.vr2_64, sx64, sy64, sz64,
+                                                           tx64[tg64], ty64[tg64], tz64[tg64]);
+                        part[0] = a.x;
+                        part[1] = a.y;
+                        part[2] = a.z;
+                        part[3] = a.w;
+                    }
 #pragma unroll
                     for (int o = 0; o < 4; ++o) {  // Kahan: sum += part
                         const float yk = part[o] - cmp[o];

@@ -1,5 +1,6 @@
 """A NaN or an infinity in the input of an FP64 product reaches every target that the direct sum carries it to: all
-beyond the cutoff tau h of its source (inside it K2 alone remains).  Clouds of several levels, so that most targets see the source through the far field; digit
+beyond the cutoff tau h of its source (inside it K2 alone remains).  Kernels that are zero without screening carry it
+as well, 0 NaN being NaN.  Clouds of several levels, so that most targets see the source through the far field; digit
 products at orders up to 7, the FP64 pipe's contraction at 8.  The product after it, of finite densities, is finite."""
 
 import numpy as np
@@ -21,9 +22,9 @@ def cloud(ctx, n, order, leaf, **kw):
 
 
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
-@pytest.mark.parametrize("kappa", [0.4])
+@pytest.mark.parametrize("kappa", [0.0, 0.4])
 @pytest.mark.parametrize("order,precision", [(3, ibim.PRECISION_FP64), (5, ibim.PRECISION_FP64), (6, ibim.PRECISION_FP64),
-                                             (8, ibim.PRECISION_FP64)])
+                                             (8, ibim.PRECISION_FP64), (5, ibim.PRECISION_MIXED)])
 def test_block(ctx, order, precision, kappa, value):
     n = 1500
     plan, bad, outside = cloud(ctx, n, order, 40, precision=precision)
@@ -38,7 +39,7 @@ def test_block(ctx, order, precision, kappa, value):
     assert np.isfinite(plan.apply(ibim.KERNEL_BIE_FUSED, kp, np.ones((4, n)))).all()
 
 
-@pytest.mark.parametrize("kappa", [0.4])
+@pytest.mark.parametrize("kappa", [0.0, 0.4])
 @pytest.mark.parametrize("order", [4, 7])
 def test_matvec_and_scalar_kernels(ctx, order, kappa):
     n = 1200
