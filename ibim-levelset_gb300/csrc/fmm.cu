@@ -1347,7 +1347,7 @@ bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry) {
     const std::vector<int> &cls = P.op_cls_h;
     const int ncls = (int)cls.size() - 1;
     const int block = (int)std::min<size_t>(std::max(1, P.nops), std::max<size_t>(8, (1UL << 30) / (8 * per)));
-    m2l_oz64_alloc(P, entry);
+    m2l_oz64_alloc(P, entry, k);
     DevBuf<double> ops;
     ops.alloc(per * block, s);
     ProfScope ps_(PROF_OPS);

@@ -301,6 +301,15 @@ struct TargetSet {
     DevBuf<float> x_off32;             // per X pair: source centre - target centre
 };
 
+// Weights of psi against the dipole in the FP64 operator's digit images, as exponents (m2l_tc.cu): for F's and G's rows,
+// by source level (nodes begin[l] .. begin[l + 1]); nlev = 0: none.
+struct OzWeights {
+    static constexpr int MAXLEV = 19;  // maxlevel 18
+    int nlev = 0;
+    int begin[MAXLEV + 1] = {};
+    int w[2][MAXLEV] = {};
+};
+
 // Launch parameters a plan takes from the tuning table (tuning.cpp) for its order and size.
 struct Tuning {
     long near_seg_pairs = 1L << 17;    // FP32 near field: source-target pairs per work segment (CTA)
@@ -388,6 +397,7 @@ struct Plan {
         bool ready = false;
         double key[5] = {-1, -1, -1, -1, -1};
         int n = 0, kpad = 0, mtiles = 0;  // rows and columns, K padded, row tiles
+        OzWeights w;
         DevBuf<uint16_t> a;
         DevBuf<double> sig;
     } oz64[ENTRY_BLOCK + 1];               // of the block's entries (built when asked for) and of the whole block
@@ -467,9 +477,10 @@ void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside
 // The FP64 operator's M2L as digit products: bytes of one operator's images at order p (0: the order
 // has none), whether nops of them may be kept on this device, the buffers, the cut of n operators
 // (of places ids) from FP64 ones, one contraction.
+struct KParams;
 double m2l_oz64_op_bytes(int p);
 bool m2l_oz64_fits(int p, double nops, bool entries = false);  // entries: all the block's, one by one
-void m2l_oz64_alloc(Plan &P, int entry);
+void m2l_oz64_alloc(Plan &P, int entry, const KParams &k);
 void m2l_oz64_pack(Plan &P, int entry, const double *ops, const int *ids, int n);
 // beside: called before the multipoles' split (work for another stream that has to be on the SMs before the
 // contraction's many CTAs queue for them).

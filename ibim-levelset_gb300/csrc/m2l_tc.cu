@@ -1829,6 +1829,10 @@ __device__ __forceinline__ void oz_digits(float2 v, int e, uint16_t *dig) {
 // Scale exponent of an operator row or a node that holds a NaN or an infinity: integers cannot carry it, so the
 // digits are zeros, and the epilogue adds a NaN wherever that exponent takes part, as an FP64 sum over the row would.
 constexpr int OZ_NONFINITE = 1 << 20;
+// In a weight's place where the dipole's (minus it: psi's) kernels are zero: that group is left out, the other has weight 1.
+constexpr int OZ_W_DROP = 1 << 16;
+__device__ __forceinline__ int oz_weight(int w) { return abs(w) == OZ_W_DROP ? 0 : w; }
+constexpr int OZ_ZERO = -(1 << 28);  // exponent of a maximum of 0, below every other
 __device__ __forceinline__ bool oz_nonfinite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
 
 // Power-of-two scale >= m (1 for m == 0), returned as its exponent.
@@ -1846,17 +1850,44 @@ __device__ __forceinline__ int oz_scale_exp_f32(float m) {
     return e;
 }
 
-// Exponent of the power-of-two scale of one operator row (n4 entries, stride n4): FP64 entries
+// The FP64 operator's rows (F, then G) and columns (dipole, then psi) in a digit image.  The cut is a fixed point
+// below the product of a row's and a node's maximum, and K1 differs from K2, and K3 from K4, by a length (and by what
+// the screening leaves of either), as m does from psi: cut together, the error would be the largest of the four products,
+// K1 by psi in a unit where lengths are small, instead of the two that occur.  So psi carries a weight 2^w and
+// its operator columns 2^-w, with w such that both column groups of a row have the same size; w is one number for
+// F's rows and another for G's, per source level (OzWeights).  F's row tiles come first and their own copy of the
+// multipoles' digits belongs to them; mtf of them, 0 where an image's rows have one weight (a scalar kernel).
+struct OzRows {
+    int mtf, rf;  // F's row tiles and rows
+    // row of the operator at place r of the padded rows, or -1
+    __device__ __forceinline__ int at(int r, int n4) const {
+        if (mtf > 0) {
+            if (r < mtf * OZ_M) return r < rf ? r : -1;
+            r += rf - mtf * OZ_M;
+        }
+        return r < n4 ? r : -1;
+    }
+};
+
+// Exponent of the power-of-two scale of one operator row (n entries, stride n4): FP64 entries
 // by the maximum of |x|'s bit patterns (for non-negative doubles their order is the integer
 // order), float-float entries by the maximum of |hi| + |lo|.
-__device__ __forceinline__ int row_scale_exp(const double *__restrict__ col0, int n4) {
+__device__ __forceinline__ int row_scale_exp(const double *__restrict__ col0, int n4, int n) {
     unsigned long long mb = 0;
-    for (int k = 0; k < n4; ++k)
+    for (int k = 0; k < n; ++k)
         mb = max(mb, (unsigned long long)__double_as_longlong(col0[(long)k * n4]) & 0x7fffffffffffffffULL);
     const double m = __longlong_as_double((long long)mb);
-    return oz_nonfinite(m) ? OZ_NONFINITE : oz_scale_exp(m);
+    return oz_nonfinite(m) ? OZ_NONFINITE : (m > 0.0 ? oz_scale_exp(m) : OZ_ZERO);
 }
-__device__ __forceinline__ int row_scale_exp(const float2 *__restrict__ col0, int n4) {
+// The same with weighted psi columns (the last quarter of the n4).
+__device__ __forceinline__ int row_scale_exp(const double *__restrict__ col0, int n4, int wpsi, bool weighted) {
+    if (!weighted) return max(row_scale_exp(col0, n4, n4), -1000);
+    const int nm = n4 / 4 * 3, em = row_scale_exp(col0, n4, nm), ep = row_scale_exp(col0 + (long)nm * n4, n4, n4 - nm);
+    if (em == OZ_NONFINITE || ep == OZ_NONFINITE) return OZ_NONFINITE;
+    return max(max(wpsi == OZ_W_DROP ? OZ_ZERO : em, wpsi == -OZ_W_DROP || ep == OZ_ZERO ? OZ_ZERO : ep - oz_weight(wpsi)),
+               -1000);
+}
+__device__ __forceinline__ int row_scale_exp(const float2 *__restrict__ col0, int n4, int, bool) {
     float m = 0.f;
     bool fin = true;
     for (int k = 0; k < n4; ++k) {
@@ -1870,16 +1901,19 @@ __device__ __forceinline__ int row_scale_exp(const float2 *__restrict__ col0, in
 
 // Row scales of the operators (FP64 or float-float, column-major n4 x n4 per op):
 // sig[op][mtiles * 128] = s_r 2^(-2D) with s_r the power of two >= max_k |A_rk|, and the exponent
-// of s_r.  ids: the operators' places among the scales, else their own order.  One thread per (op, row); neighbouring threads read neighbouring rows of a column.
+// of s_r.  ids: the operators' places among the scales, else their own order.  One thread per (op, padded row);
+// neighbouring threads read neighbouring rows of a column.
 template <class OW>
 __global__ void k_scale_ops_oz(int n4, int mtiles, int nops, int scale_exp, const OW *__restrict__ ops, double *sig,
-                               int *sexp, const int *__restrict__ ids = nullptr) {
+                               int *sexp, const int *__restrict__ ids = nullptr, OzRows rows = OzRows{},
+                               OzWeights wt = OzWeights{}, const int *__restrict__ keys = nullptr) {
     const int mpad = mtiles * OZ_M;
     const long total = (long)nops * mpad;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int r = (int)(i % mpad), op = (int)(i / mpad);
-        const int e = r < n4 ? row_scale_exp(ops + (long)op * n4 * n4 + r, n4) : 0;
-        sig[ids ? (long)ids[op] * mpad + r : i] = ldexp(1.0, e - scale_exp);
+        const int pr = (int)(i % mpad), op = (int)(i / mpad), r = rows.at(pr, n4);
+        const int w = rows.mtf > 0 ? wt.w[pr < rows.mtf * OZ_M ? 0 : 1][keys[5 * (ids ? ids[op] : op) + 1]] : 0;
+        const int e = r >= 0 ? row_scale_exp(ops + (long)op * n4 * n4 + r, n4, w, rows.mtf > 0) : 0;
+        sig[ids ? (long)ids[op] * mpad + pr : i] = ldexp(1.0, e - scale_exp);
         sexp[i] = e;
     }
 }
@@ -1893,25 +1927,32 @@ __global__ void k_scale_ops_oz(int n4, int mtiles, int nops, int scale_exp, cons
 template <int S, class OW, bool H16 = false>
 __global__ void k_pack_ops_oz(int n4, int mtiles, int kpad, int nops, const OW *__restrict__ ops,
                               const int *__restrict__ sexp, uint4 *a, const float *__restrict__ rscale = nullptr,
-                              uint4 *a_hi = nullptr, uint4 *a_lo = nullptr, const int *__restrict__ ids = nullptr) {
+                              uint4 *a_hi = nullptr, uint4 *a_lo = nullptr, const int *__restrict__ ids = nullptr,
+                              OzRows rows = OzRows{}, OzWeights wt = OzWeights{}, const int *__restrict__ keys = nullptr) {
     static_assert(!H16 || std::is_same<OW, float2>::value, "FP16 images from float-float operators");
     static_assert(OZ_M == TC_M && OZ_KS == TC_KS16 && OZ_ATILE == TC_TILE_BYTES, "one tile layout");
     const int nstage = kpad / OZ_KS, mpad = mtiles * OZ_M, ngrp = kpad / 8;
     const long total = (long)nops * ngrp * mpad;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int r = (int)(i % mpad);  // rows fastest: coalesced column reads
+        const int pr = (int)(i % mpad), r = rows.at(pr, n4);  // rows fastest: coalesced column reads
         const long rest = i / mpad;
         const int grp = (int)(rest % ngrp), op = (int)(rest / ngrp);
-        const int e = sexp[(long)op * mpad + r];
+        const int e = sexp[(long)op * mpad + pr];
+        int w_psi = 0, k_psi = n4;  // the psi columns' weight, from k_psi on
+        if (rows.mtf > 0) {
+            w_psi = wt.w[pr < rows.mtf * OZ_M ? 0 : 1][keys[5 * (ids ? ids[op] : op) + 1]];
+            k_psi = n4 / 4 * 3;
+        }
         float inv = 1.f;
-        if constexpr (H16) inv = 1.f / rscale[(long)op * mpad + r];  // a power of two: exact
+        if constexpr (H16) inv = 1.f / rscale[(long)op * mpad + pr];  // a power of two: exact
         uint32_t w[S][4], wh[4], wl[4];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int k = grp * 8 + q;
-            const OW v = (r < n4 && k < n4) ? ops[(long)op * n4 * n4 + (long)k * n4 + r] : OW{};
+            const OW v = (r >= 0 && k < n4) ? ops[(long)op * n4 * n4 + (long)k * n4 + r] : OW{};
             uint16_t dig[S];
-            oz_digits<S>(e == OZ_NONFINITE ? OW{} : v, e, dig);
+            const bool zero = e == OZ_NONFINITE || w_psi == (k < k_psi ? OZ_W_DROP : -OZ_W_DROP);
+            oz_digits<S>(zero ? OW{} : v, k < k_psi || zero ? e : e + oz_weight(w_psi), dig);
 #pragma unroll
             for (int d = 0; d < S; ++d) {
                 if (q & 1) w[d][q >> 1] |= (uint32_t)dig[d] << 16;
@@ -1932,7 +1973,7 @@ __global__ void k_pack_ops_oz(int n4, int mtiles, int kpad, int nops, const OW *
                 }
             }
         }
-        const int t = r / OZ_M, row = r % OZ_M, st = grp / 2, half = grp & 1;
+        const int t = pr / OZ_M, row = pr % OZ_M, st = grp / 2, half = grp & 1;
         const long tile = ((long)(ids ? ids[op] : op) * mtiles + t) * nstage + st, tbase = tile * S;
         const uint32_t off = tile_off(row, half);  // byte offset of the 16-byte piece
 #pragma unroll
@@ -1974,34 +2015,48 @@ __global__ void k_scale_ops_ff2(int n4, int mtiles, int nops, int scale_exp, con
 }
 
 // Multipoles (FP64 [node][n4]) -> digits [node][stage][digit][16] and the exponents tau of the column scales t_j.
-// One warp per node.
+// One warp per node.  With weights: an image for F's rows and, after it, one for G's.
 template <int S>
 __global__ void k_split_mult_oz(long nnodes, int n4, int kpad, const double *__restrict__ mult, uint16_t *b,
-                                int *tau) {
+                                int *tau, OzWeights wt = OzWeights{}) {
     const int lane = threadIdx.x & 31;
     const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
     const int nstage = kpad / OZ_KS;
     for (long node = warp; node < nnodes; node += nwarps) {
         const double *m = mult + node * n4;
-        double mx = 0.0;
+        const bool weighted = S > 7 && wt.nlev > 0;
+        const int k_psi = weighted ? n4 / 4 * 3 : n4;
+        double mx = 0.0, px = 0.0;
         bool bad = false;
         for (int k = lane; k < n4; k += 32) {
-            mx = fmax(mx, fabs(m[k]));
+            if (k < k_psi) mx = fmax(mx, fabs(m[k]));
+            else px = fmax(px, fabs(m[k]));
             bad = bad || oz_nonfinite(m[k]);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (weighted) px = fmax(px, __shfl_xor_sync(0xffffffffu, px, o));
+        }
         bad = __any_sync(0xffffffffu, bad);
-        const int e = bad ? OZ_NONFINITE : oz_scale_exp(mx);
-        if (lane == 0) tau[node] = e;
-        for (int k = lane; k < kpad; k += 32) {
-            const double v = k < n4 && !bad ? m[k] : 0.0;
-            uint16_t dig[S];
-            oz_digits<S>(v, e, dig);
-            const long base = ((node * nstage + k / OZ_KS) * S) * OZ_KS + (k % OZ_KS);
+        int level = 0;
+        if (weighted)
+            while (level + 1 < wt.nlev && node >= wt.begin[level + 1]) ++level;
+        for (int img = 0; img < (weighted ? 2 : 1); ++img) {
+            const int wd = weighted ? wt.w[img][level] : 0, w = oz_weight(wd);
+            const int em = mx > 0.0 && wd != OZ_W_DROP ? oz_scale_exp(mx) : OZ_ZERO,
+                      ep = px > 0.0 && wd != -OZ_W_DROP ? oz_scale_exp(px) + w : OZ_ZERO;
+            const int e = bad ? OZ_NONFINITE : (max(em, ep) == OZ_ZERO ? 0 : max(em, ep));
+            if (lane == 0) tau[img * nnodes + node] = e;
+            for (int k = lane; k < kpad; k += 32) {
+                const bool psi = k >= k_psi, some = k < n4 && !bad && (psi ? ep : em) != OZ_ZERO;
+                uint16_t dig[S];
+                oz_digits<S>(some ? m[k] : 0.0, some && psi ? e - w : e, dig);
+                const long base = (((img * nnodes + node) * nstage + k / OZ_KS) * S) * OZ_KS + (k % OZ_KS);
 #pragma unroll
-            for (int d = 0; d < S; ++d) b[base + (long)d * OZ_KS] = dig[d];
+                for (int d = 0; d < S; ++d) b[base + (long)d * OZ_KS] = dig[d];
+            }
         }
     }
 }
@@ -2043,7 +2098,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
              const int *__restrict__ vtgt, const uint16_t *__restrict__ a, const double *__restrict__ sig,
              const uint16_t *__restrict__ bdig, const int *__restrict__ tau, double *local, int *err,
              const int *__restrict__ chunk_mol, const int *__restrict__ mol_active,
-             const MolImg *__restrict__ mol_img) {
+             const MolImg *__restrict__ mol_img, OzRows rows = OzRows{}, long nnodes = 0) {
     // a merged plan (batch.cu): chunks of molecules that have stopped iterating are skipped whole,
     // the others read their molecule's own digit images
     if (chunk_mol) {
@@ -2065,6 +2120,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const int op = chunks[3 * blockIdx.x], b = chunks[3 * blockIdx.x + 1], cnt = chunks[3 * blockIdx.x + 2];
     const int t = blockIdx.y;
     const int nstage = kpad / OZ_KS;
+    if (S > 7 && rows.mtf > 0 && t >= rows.mtf) {  // G's copy of the multipoles' digits
+        bdig += nnodes * nstage * (S * OZ_KS);
+        tau += nnodes;
+    }
     // MMA width of this chunk: its pairs rounded up to 16; gathers and epilogue stop there too
     const int neff = max(16, (cnt + 15) & ~15);
     const uint32_t idesc = kIdescOz | ((uint32_t)(neff >> 3) << 17);
@@ -2205,8 +2264,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         // against 13.1 (the residual).
         constexpr int D = SH::D, F = SH::F, CW = SH::CW;
         const int lg = warp & 3, h = warp >> 2;
-        const int row = t * OZ_M + 32 * lg + lane;
-        const int erow = row < n4 ? exp_of_pow2(sig[(long)op * mtiles * OZ_M + row]) : 0;
+        const int pr = t * OZ_M + 32 * lg + lane, row = S > 7 ? rows.at(pr, n4) : (pr < n4 ? pr : -1);
+        const int erow = row >= 0 ? exp_of_pow2(sig[(long)op * mtiles * OZ_M + pr]) : 0;
 #pragma unroll 1
         for (int c0 = OZ_N / 2 * h; c0 < min(OZ_N / 2 * (h + 1), neff); c0 += CW) {
             uint32_t v[OZ_ACC][CW];
@@ -2229,7 +2288,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                         : "r"(ta));
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < n4) {
+            if (row >= 0) {
 #pragma unroll
                 for (int q = 0; q < CW; ++q) {
                     const int tg = tgt_s[c0 + q];
@@ -2561,10 +2620,10 @@ void m2l_oz_pack(Plan &P, const float2 *ff) {
     auto pack = [&](auto kf, auto kd) {
         if (ff)
             (count_launch(), kf<<<gp, 256, 0, s>>>(n4, P.oz_mtiles, P.oz_kpad, P.nops, ff, sexp.ptr, a, nullptr,
-                                                   nullptr, nullptr, nullptr));
+                                                   nullptr, nullptr, nullptr, OzRows{}, OzWeights{}, nullptr));
         else
             (count_launch(), kd<<<gp, 256, 0, s>>>(n4, P.oz_mtiles, P.oz_kpad, P.nops, P.ops64.ptr, sexp.ptr, a,
-                                                   nullptr, nullptr, nullptr, nullptr));
+                                                   nullptr, nullptr, nullptr, nullptr, OzRows{}, OzWeights{}, nullptr));
     };
     if (S == 6)
         pack(k_pack_ops_oz<6, float2>, k_pack_ops_oz<6, double>);
@@ -2673,7 +2732,7 @@ void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside
         (count_launch(), kern<<<grid, OZ_THREADS, smem, s>>>(n4, P.oz_kpad, P.oz_mtiles, S.v_chunk_oz.ptr, S.v_src.ptr,
                                                             S.v_tgt.ptr, P.oz_a.ptr, P.oz_sig.ptr, P.oz_b.ptr,
                                                             P.oz_tau.ptr, P.local.ptr, P.tc_err.ptr, S.chunk_mol_oz.ptr,
-                                                            P.mol_active.ptr, P.mol_img.ptr));
+                                                            P.mol_active.ptr, P.mol_img.ptr, OzRows{}, 0L));
     }
     IBIM_CHECK_LAUNCH();
 }
@@ -2682,8 +2741,9 @@ void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside
 // M2L of the FP64 operator (IBIM_PRECISION_FP64) as digit products.  GB300 does 1.25 TFLOP/s on the
 // FP64 pipe and 1.9 PFLOP/s of BF16 MMAs, so the 36 (45) digit pairs of a 56-bit (54-bit) cut cost a
 // fifteenth of the FP64 contraction: 744 -> 37 ms a product on a 2,000-atom protein (1.70 M pairs,
-// order 5), 46 ms beside the near field, which has the FP64 pipe to itself.  It is no less exact: with K = 4p^3 terms the FP64 chain of K multiply-adds leaves about
-// sqrt(K / 2) 2^-53 of its partial sums, the cut 2^-57 (2^-55) of row and column maximum per term,
+// order 5), 46 ms beside the near field, which has the FP64 pipe to itself.  Error: with K = 4p^3 terms the FP64 chain
+// of K multiply-adds leaves about sqrt(K / 2) 2^-53 of its partial sums, the cut 2^-57 (2^-55) of row and column maximum
+// per term, of the dipole's columns or psi's, whichever product is the larger (OzRows, measured at oz64_weights);
 // groups 0 .. 5 (0 .. 6) exact in FP32 (|G_k| <= K 2^(2D) (1 + (k - 1) / 4) <= 2^24 for K = 500,
 // D = 7 and K = 1372, D = 6) and the last two, 2^-42 below, sharing one accumulator.
 // Seven (eight) accumulators leave 64 pairs a chunk in the 512 TMEM columns.  Orders up to 7; order
@@ -2692,12 +2752,59 @@ void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside
 // ---------------------------------------------------------------------------------------------
 static int oz64_digits(int p) { return p <= 5 ? 8 : 9; }
 
-static double oz64_image_bytes(int p, int n4) {
-    const double kpad = (n4 + OZ_KS - 1) / OZ_KS * OZ_KS, mpad = (n4 + OZ_M - 1) / OZ_M * OZ_M;
-    return 2.0 * oz64_digits(p) * kpad * mpad;
+static OzRows oz64_rows(int R, bool block) { return block ? OzRows{(R + OZ_M - 1) / OZ_M, R} : OzRows{0, 0}; }
+static int oz64_mtiles(int R, bool block) {
+    return block ? (R + OZ_M - 1) / OZ_M + (3 * R + OZ_M - 1) / OZ_M : (R + OZ_M - 1) / OZ_M;
 }
 
-double m2l_oz64_op_bytes(int p) { return p > 7 ? 0. : oz64_image_bytes(p, 4 * p * p * p); }
+static double oz64_image_bytes(int p, bool block) {
+    const int R = p * p * p, n = block ? 4 * R : R;
+    return 2.0 * oz64_digits(p) * ((n + OZ_KS - 1) / OZ_KS * OZ_KS) * ((double)oz64_mtiles(R, block) * OZ_M);
+}
+
+double m2l_oz64_op_bytes(int p) { return p > 7 ? 0. : oz64_image_bytes(p, true); }
+
+// The weights of psi: at each source level the power of two nearest |K2| / |K1| (F's rows) and |K4| / |K3| (G's) at four
+// half-widths, in the midst of the V pairs' 2 to 10.  Off an operator's own ratio by d bits, the cut's error there
+// grows by up to d bits where the smaller group has the larger part of the sum; far operators, whose ratios are the
+// ones that differ, add little to it.  Errors of FMMs of 6,000 to 16,000 points against 80-bit ones, in units from
+// 1e-10 to 1e6 Angstrom, psi from 1e-6 to 1e6 times the dipole, screening t = kappa h from 0 to 1: 0.4 to 1.07 times the FP64 sums'
+// (with the ratios at 2 half-widths up to 2.1, at 1.5 up to 5; cut together up to 1e9).
+// Without screening K2 and K3 are zero: psi leaves F's copy of the multipoles and the dipole G's.
+static OzWeights oz64_weights(const Plan &P, const KParams &k) {
+    OzWeights W;
+    const TreeHost &T = P.tree;
+    W.nlev = T.nlevels;
+    IBIM_REQUIRE(W.nlev <= OzWeights::MAXLEV, "too many tree levels");
+    for (int l = 0; l <= W.nlev; ++l) W.begin[l] = T.level_begin[l];
+    for (int l = 0; l < W.nlev; ++l) {
+        double rs = 0.;
+        for (int a = 0; a < 3; ++a) {
+            const double v = T.radius[3 * (size_t)T.level_begin[l] + a];
+            if (v > 0. && (rs == 0. || v < rs)) rs = v;
+        }
+        double A[4] = {0., 0., 0., 0.};  // K1 .. K4, 4 pi left out but in K3
+        for (double q : {4., 5.}) {      // two: K1 may pass through zero
+            const double r = q * rs, t = k.kappa * r, e = std::exp(-t);
+            // 1 - e^-t (1 + t) and 3 - e^-t (3 + 3 t + t^2), without their cancellation for small t
+            const double u1 = std::fabs(t) < 1e-2 ? t * t * (0.5 - t / 3.) : 1. - e * (1. + t);
+            const double u3 = std::fabs(t) < 1e-2 ? t * t * (0.5 - t * t / 8.) : 3. - e * (3. + t * (3. + t));
+            A[0] = std::max(A[0], std::fabs(k.eps - 1. - k.eps * u1) / (r * r));
+            A[1] = std::max(A[1], -std::expm1(-t) / r);
+            A[2] = std::max(A[2], std::max(std::fabs(u1), std::fabs(u3)) / (r * r * r) * (k.k3f / k.q4pi));
+            A[3] = std::max(A[3], std::fabs(1. - k.ieps + k.ieps * u1) / (r * r));
+        }
+        for (int i = 0; i < 2; ++i) {
+            const double m = A[2 * i], psi = A[2 * i + 1];
+            int &w = W.w[i][l];
+            if (!(std::isfinite(m) && std::isfinite(psi)) || (m == 0. && psi == 0.)) w = 0;
+            else if (psi == 0.) w = -OZ_W_DROP;
+            else if (m == 0.) w = OZ_W_DROP;
+            else w = (int)std::lrint(std::max(-1000., std::min(1000., std::log2(psi) - std::log2(m))));
+        }
+    }
+    return W;
+}
 
 bool m2l_oz64_fits(int p, double nops, bool entries) {
     if (p > 7 || !m2l_tc_supported()) return false;
@@ -2711,24 +2818,27 @@ bool m2l_oz64_fits(int p, double nops, bool entries) {
         IBIM_CUDA(cudaMemGetInfo(&free_b, &t));
         if (dev < 64) total[dev].store(t);
     }
-    return (entries ? ENTRY_BLOCK * oz64_image_bytes(p, p * p * p) : m2l_oz64_op_bytes(p)) * nops <= t / 3.0;
+    return (entries ? ENTRY_BLOCK * oz64_image_bytes(p, false) : m2l_oz64_op_bytes(p)) * nops <= t / 3.0;
 }
 
-void m2l_oz64_alloc(Plan &P, int entry) {
+void m2l_oz64_alloc(Plan &P, int entry, const KParams &k) {
     cudaStream_t s = P.ctx->stream;
     auto &Z = P.oz64[entry];
-    Z.n = entry == ENTRY_BLOCK ? 4 * P.R : P.R;
+    const bool whole = entry == ENTRY_BLOCK;
+    Z.n = whole ? 4 * P.R : P.R;
     Z.kpad = (Z.n + OZ_KS - 1) / OZ_KS * OZ_KS;
-    Z.mtiles = (Z.n + OZ_M - 1) / OZ_M;
+    Z.mtiles = oz64_mtiles(P.R, whole);
+    Z.w = whole ? oz64_weights(P, k) : OzWeights{};
+    const size_t copies = whole ? 2 : 1;
     P.oz64_s = oz64_digits(P.p);
     const size_t stages = Z.kpad / OZ_KS, rows = (size_t)P.nops * Z.mtiles;
     if (Z.a.n != rows * stages * P.oz64_s * (OZ_ATILE / 2)) {
         Z.a.alloc(rows * stages * P.oz64_s * (OZ_ATILE / 2), s);
         Z.sig.alloc(rows * OZ_M, s);
     }
-    const size_t nb = (size_t)P.tree.nnodes * stages * P.oz64_s * OZ_KS;
+    const size_t nb = copies * P.tree.nnodes * stages * P.oz64_s * OZ_KS;
     if (P.oz64_b.n < nb) P.oz64_b.alloc(nb, s);
-    if (P.oz64_tau.n < (size_t)P.tree.nnodes) P.oz64_tau.alloc((size_t)P.tree.nnodes, s);
+    if (P.oz64_tau.n < copies * P.tree.nnodes) P.oz64_tau.alloc(copies * P.tree.nnodes, s);
     if (!P.tc_err.ptr) {
         P.tc_err.alloc(1, s);
         P.tc_err.zero();
@@ -2744,16 +2854,18 @@ void m2l_oz64_pack(Plan &P, int entry, const double *ops, const int *ids, int n)
     cudaStream_t s = P.ctx->stream;
     auto &Z = P.oz64[entry];
     const int n4 = Z.n, D = P.oz64_s == 8 ? OzShape<8>::D : OzShape<9>::D;
+    const OzRows rw = oz64_rows(P.R, entry == ENTRY_BLOCK);
     const long rows = (long)n * Z.mtiles * OZ_M;
     DevBuf<int> sexp;
     sexp.alloc((size_t)rows, s);
     const int gs = (int)std::min<long>((rows + 255) / 256, 32L * P.ctx->num_sms);
     const int gp = (int)std::min<long>((rows * (Z.kpad / 8) + 255) / 256, 64L * P.ctx->num_sms);
     (count_launch(), k_scale_ops_oz<double><<<gs, 256, 0, s>>>(n4, Z.mtiles, n, 2 * D, ops, Z.sig.ptr,
-                                                               sexp.ptr, ids));
+                                                               sexp.ptr, ids, rw, Z.w, P.op_key.ptr));
     uint4 *a = reinterpret_cast<uint4 *>(Z.a.ptr);
     auto kern = P.oz64_s == 8 ? k_pack_ops_oz<8, double> : k_pack_ops_oz<9, double>;
-    (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr, ids));
+    (count_launch(), kern<<<gp, 256, 0, s>>>(n4, Z.mtiles, Z.kpad, n, ops, sexp.ptr, a, nullptr, nullptr, nullptr, ids,
+                                             rw, Z.w, P.op_key.ptr));
     IBIM_CHECK_LAUNCH();
 }
 
@@ -2767,12 +2879,13 @@ void m2l_oz64_run(Plan &P, const TargetSet &S, int entry, const std::function<vo
     if (beside) beside();
     auto split = ns == 8 ? k_split_mult_oz<8> : k_split_mult_oz<9>;
     (count_launch(), split<<<4 * P.ctx->num_sms, 256, 0, s>>>(P.tree.nnodes, n4, Z.kpad, P.mult.ptr, P.oz64_b.ptr,
-                                                                P.oz64_tau.ptr));
+                                                                P.oz64_tau.ptr, Z.w));
     auto kern = ns == 8 ? k_m2l_oz<8> : k_m2l_oz<9>;
     const int smem = ns == 8 ? OzShape<8>::SMEM : OzShape<9>::SMEM;
     (count_launch(), kern<<<dim3(S.nchunks_oz64, Z.mtiles), OZ_THREADS, smem, s>>>(
         n4, Z.kpad, Z.mtiles, S.v_chunk_oz64.ptr, S.v_src.ptr, S.v_tgt.ptr, Z.a.ptr, Z.sig.ptr, P.oz64_b.ptr,
-        P.oz64_tau.ptr, P.local.ptr, P.tc_err.ptr, nullptr, nullptr, nullptr));
+        P.oz64_tau.ptr, P.local.ptr, P.tc_err.ptr, nullptr, nullptr, nullptr, oz64_rows(P.R, entry == ENTRY_BLOCK),
+        P.tree.nnodes));
     IBIM_CHECK_LAUNCH();
 }
 

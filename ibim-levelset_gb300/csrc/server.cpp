@@ -91,7 +91,7 @@ static double fmm_bytes(const ibim_config &cfg, double N, double nodes, double o
     if (cfg.precision == IBIM_PRECISION_FP64) {
         const bool cut = m2l_oz64_fits(cfg.np, ops);
         per_op = cut ? m2l_oz64_op_bytes(cfg.np) : n4 * n4 * 8.0;
-        per_node = n4 * 16.0 + (cut ? 20.0 * kpad : 0.0);
+        per_node = n4 * 16.0 + (cut ? 40.0 * kpad : 0.0);
         scratch = cut ? std::min(ops * n4 * n4 * 8.0, 1.1e9) : 0.0;
     } else {
         per_op = 2.0 * mpad * kpad * 2.0 + digits * mpad * kpad * 2.0 + n4 * n4 * 8.0;
