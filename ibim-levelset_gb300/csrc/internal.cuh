@@ -75,8 +75,8 @@ struct DevBuf {
     void alloc(size_t count, cudaStream_t s) {
         release();
         stream = s;
-        n = count;
         if (count) ptr = static_cast<T *>(device_alloc(sizeof(T) * count, s));
+        n = count;  // 0 where the allocation threw: callers compare n before they allocate again
     }
     void release() {
         if (ptr) cudaFreeAsync(ptr, stream);
