@@ -859,7 +859,8 @@ int ibim_fmm_apply(ibim_plan p, int kernel, const ibim_kernel_params *kp, const 
         DevBuf<double> hin;
         hin.alloc((size_t)rows * ns, s);
         hin.upload(in, (size_t)rows * ns);
-        const bool one = rows == 1 && fmm_one_entry(P);  // the kernel's own entry of the block alone
+        const int entry = rows == 1 ? 4 * kKernelMap[kernel].field + kKernelMap[kernel].slot : ENTRY_BLOCK;
+        const bool one = rows == 1 && fmm_one_entry(P, *kp, entry);  // the kernel's own entry of the block alone
         if (!one) P.dens4.zero();
         if (rows == 4) {
             for (int d = 0; d < 4; ++d) permute(c, ns, P.src_perm.ptr, hin.ptr + d * ns, P.dens4.ptr + d * ns, false);
@@ -868,7 +869,7 @@ int ibim_fmm_apply(ibim_plan p, int kernel, const ibim_kernel_params *kp, const 
                     false);
         }
         if (one)
-            fmm_run_entry(P, 0, *kp, P.dens4.ptr, S.out4.ptr, 4 * kKernelMap[kernel].field + kKernelMap[kernel].slot);
+            fmm_run_entry(P, 0, *kp, P.dens4.ptr, S.out4.ptr, entry);
         else
             fmm_run(P, 0, *kp, P.dens4.ptr, S.out4.ptr, P.precision);
         DevBuf<double> hout;

@@ -1333,16 +1333,9 @@ void near64_lists(Plan &P, TargetSet &S) {
 
 // The FP64 operator's digit images, whole or of one entry of the block: the operators in blocks of at most
 // 1 GB, each cut and dropped.
-bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry) {
-    if (!P.oz64_ok) return false;
-    double key[5];
-    kp_key(kp, key);
-    auto &Z = P.oz64[entry];
-    if (Z.ready && same_key(Z.key, key)) return true;
-    Z.ready = false;
+static void build_oz64_images(Plan &P, const KParams &k, int entry) {
     cudaStream_t s = P.ctx->stream;
     const int R = P.R, n = entry == ENTRY_BLOCK ? 4 * R : R;
-    const KParams k = make_kparams(kp, P.tube->h);
     const size_t per = (size_t)n * n;
     const std::vector<int> &cls = P.op_cls_h;
     const int ncls = (int)cls.size() - 1;
@@ -1358,9 +1351,44 @@ bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry) {
         IBIM_CHECK_LAUNCH();
         m2l_oz64_pack(P, entry, ops.ptr, P.op_ord.ptr + cls[c], cls[e] - cls[c]);
     }
-    for (int i = 0; i < 5; ++i) Z.key[i] = key[i];
-    Z.ready = true;
-    return true;
+}
+
+// The images take about twice the memory of the operators that k_m2l_v64 reads, so a plan whose neighbours leave the
+// device too little for them takes that contraction (a single kernel: the block), for the rest of its life, instead of
+// failing.  Images of single kernels, which the plan keeps between calls, go first.
+bool fmm_ensure_oz64_images(Plan &P, const ibim_kernel_params &kp, int entry) {
+    if (!P.oz64_ok) return false;
+    double key[5];
+    kp_key(kp, key);
+    auto &Z = P.oz64[entry];
+    if (Z.ready && same_key(Z.key, key)) return true;
+    Z.ready = false;
+    const KParams k = make_kparams(kp, P.tube->h);
+    auto drop = [](Plan::Oz64 &z) {
+        z.ready = false;
+        z.a.release();
+        z.sig.release();
+    };
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        try {
+            if (Z.a.ptr || m2l_oz64_room(P, entry)) {
+                build_oz64_images(P, k, entry);
+                for (int i = 0; i < 5; ++i) Z.key[i] = key[i];
+                Z.ready = true;
+                return true;
+            }
+        } catch (const Error &e) {
+            if (e.status != IBIM_ERR_OUT_OF_MEMORY) throw;
+        }
+        drop(Z);
+        for (int i = 0; i < ENTRY_BLOCK; ++i) drop(P.oz64[i]);
+    }
+    if (entry == ENTRY_BLOCK) {
+        P.oz64_ok = false;
+        P.oz64_b.release();
+        P.oz64_tau.release();
+    }
+    return false;
 }
 
 void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp) {
@@ -1371,9 +1399,10 @@ void fmm_prepare_fp64(Plan &P, const ibim_kernel_params &kp) {
 // (a sixteenth of the products, images of their own built on the first call of each kernel and kept), half
 // the near field's instructions.  150 atoms at order 6: 16.5 -> 3.3 ms a product, 40 -> 18 ms the first one.
 // Plans without room for all 16 entries' images beside the block's, without digit images, or with X pairs
-// evaluated on the fly run the block with the other densities zero.
-bool fmm_one_entry(const Plan &P) {
-    return P.precision == IBIM_PRECISION_FP64 && P.oz64_ok && P.x_as_ops && m2l_oz64_fits(P.p, P.nops, true);
+// evaluated on the fly run the block with the other densities zero.  Builds the entry's images.
+bool fmm_one_entry(Plan &P, const ibim_kernel_params &kp, int entry) {
+    return P.precision == IBIM_PRECISION_FP64 && P.oz64_ok && P.x_as_ops && m2l_oz64_fits(P.p, P.nops, true) &&
+           fmm_ensure_oz64_images(P, kp, entry);
 }
 
 // One FP64 FMM: dens (nc x ns, tree order) -> out (nc x nt of target set ts, tree order), nc = 4 for the block,
@@ -1383,12 +1412,11 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
                          int entry = ENTRY_BLOCK) {
     IBIM_REQUIRE(ts >= 0 && ts < (int)P.targets.size(), "no such target set");
     const bool use_oz = m2l_sliced && (4 * P.R + 15) / 16 * 16 <= M2L_OZ_MAXK;
-    const bool use_oz64 = !m2l_sliced && P.oz64_ok;
+    const bool use_oz64 = !m2l_sliced && fmm_ensure_oz64_images(P, kpp, entry);
+    IBIM_REQUIRE(use_oz64 || entry == ENTRY_BLOCK, "the plan has no images of single kernels");
     if (use_oz)
         fmm_ensure_oz_images(P, kpp);
-    else if (use_oz64)
-        fmm_ensure_oz64_images(P, kpp, entry);
-    else
+    else if (!use_oz64)
         fmm_prepare_operators(P, kpp, IBIM_PRECISION_FP64);
     const TargetSet &S = *P.targets[ts];
     Ctx *c = P.ctx;
@@ -1510,7 +1538,6 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
 }
 
 void fmm_run_entry(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int entry) {
-    IBIM_REQUIRE(fmm_one_entry(P), "the plan has no images of single kernels");
     fmm_run_fp64(P, ts, kp, dens, out, false, entry);
 }
 

@@ -438,7 +438,7 @@ struct Plan {
 void fmm_prepare_operators(Plan &P, const ibim_kernel_params &kp, int precision);
 // One scalar kernel's FMM in FP64, an entry of the block: dens ns, out nt.  Only where fmm_one_entry: FP64 plans with
 // digit images, whose 16 entries' images fit too (else the block runs with the other densities zero).
-bool fmm_one_entry(const Plan &P);
+bool fmm_one_entry(Plan &P, const ibim_kernel_params &kp, int entry);
 void fmm_run_entry(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int entry);
 void fmm_run_mixed(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out);
 void fmm_run(Plan &P, int ts, const ibim_kernel_params &kp, const double *dens, double *out, int precision);
@@ -480,6 +480,8 @@ void m2l_oz_run(Plan &P, const TargetSet &S, const std::function<void()> &beside
 struct KParams;
 double m2l_oz64_op_bytes(int p);
 bool m2l_oz64_fits(int p, double nops, bool entries = false);  // entries: all the block's, one by one
+// Whether the device has room for a plan's images now: for twice them and the scratch of building them.
+bool m2l_oz64_room(const Plan &P, int entry);
 void m2l_oz64_alloc(Plan &P, int entry, const KParams &k);
 void m2l_oz64_pack(Plan &P, int entry, const double *ops, const int *ids, int n);
 // beside: called before the multipoles' split (work for another stream that has to be on the SMs before the

@@ -2806,9 +2806,7 @@ static OzWeights oz64_weights(const Plan &P, const KParams &k) {
     return W;
 }
 
-bool m2l_oz64_fits(int p, double nops, bool entries) {
-    if (p > 7 || !m2l_tc_supported()) return false;
-    if (nops <= 0.) return true;
+static double device_bytes() {
     static std::atomic<size_t> total[64];  // each device's memory, asked for once
     int dev = 0;
     IBIM_CUDA(cudaGetDevice(&dev));
@@ -2818,7 +2816,32 @@ bool m2l_oz64_fits(int p, double nops, bool entries) {
         IBIM_CUDA(cudaMemGetInfo(&free_b, &t));
         if (dev < 64) total[dev].store(t);
     }
-    return (entries ? ENTRY_BLOCK * oz64_image_bytes(p, false) : m2l_oz64_op_bytes(p)) * nops <= t / 3.0;
+    return (double)t;
+}
+
+bool m2l_oz64_fits(int p, double nops, bool entries) {
+    if (p > 7 || !m2l_tc_supported()) return false;
+    if (nops <= 0.) return true;
+    return (entries ? ENTRY_BLOCK * oz64_image_bytes(p, false) : m2l_oz64_op_bytes(p)) * nops <= device_bytes() / 3.0;
+}
+
+// Small images are not worth the question (a sixty-fourth of the device's memory: 4 GB).
+bool m2l_oz64_room(const Plan &P, int entry) {
+    const bool block = entry == ENTRY_BLOCK;
+    const double n = (block ? 4. : 1.) * P.R, ops = n * n * 8. * P.nops;
+    const double need = oz64_image_bytes(P.p, block) * P.nops + std::min(ops, 1.1e9) +
+                        (block ? 2. : 1.) * P.tree.nnodes * n * 2. * oz64_digits(P.p);
+    if (need < device_bytes() / 64.) return true;
+    size_t free_b = 0, t = 0;
+    IBIM_CUDA(cudaMemGetInfo(&free_b, &t));
+    int dev = 0;
+    IBIM_CUDA(cudaGetDevice(&dev));
+    cudaMemPool_t pool;
+    IBIM_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+    uint64_t reserved = 0, used = 0;
+    IBIM_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    IBIM_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    return 2. * need <= (double)free_b + (double)(reserved - used);
 }
 
 void m2l_oz64_alloc(Plan &P, int entry, const KParams &k) {

@@ -69,3 +69,24 @@ ref = tube.plan(5, 12, 10).apply(ibim.KERNEL_BIE_FUSED, kp, dens)
 for o in range(4):
     close(out[o], ref[o])
 """)
+
+
+@pytest.mark.parametrize("left", [1.6, 3.3, 6.5])
+def test_product_without_room_for_its_images(left):
+    """Room for the FP64 operators but not, or barely, for their digit images: the product runs all the same.  Both
+    contractions are FP64 sums within 2e-13 of the oracle's (test_fp64_digits_gpu.py), so within 4e-13 of each other."""
+    pytest.importorskip("torch")
+    child(r"""
+hog = take(%g * ops64)
+m = dens[0]
+out = plan.apply(ibim.KERNEL_BIE_FUSED, kp, dens)
+one = [plan.apply(k, kp, m) for k in range(len(ibim.KERNELS))]
+again = plan.apply(ibim.KERNEL_BIE_FUSED, ibim.kernel_params(0.5, 80.0, 2.0, 1.0), dens)
+release()
+fresh = tube.plan(5, 12, 10)
+for o in range(4):
+    close(out[o], fresh.apply(ibim.KERNEL_BIE_FUSED, kp, dens)[o])
+    close(again[o], fresh.apply(ibim.KERNEL_BIE_FUSED, ibim.kernel_params(0.5, 80.0, 2.0, 1.0), dens)[o])
+for k in range(len(ibim.KERNELS)):
+    close(one[k], fresh.apply(k, kp, m))
+""" % left)
