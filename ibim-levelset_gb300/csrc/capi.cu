@@ -1177,7 +1177,7 @@ int ibim_autotune(ibim_ctx ctx, const double *centers, const double *charges, co
             t.tc_form = f;
             consider(t);
         }
-        for (long v : {1L << 15, 1L << 16, 1L << 18}) {
+        for (long v : {1L << 11, 1L << 13, 1L << 15}) {  // beside the plan's own choice of 2^11 to 2^14
             Tuning t = best;
             t.near_seg_pairs = v;
             consider(t);

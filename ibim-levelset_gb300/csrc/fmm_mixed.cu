@@ -677,9 +677,10 @@ void mixed_lists_host(const Plan &P, TargetSet &S) {
         for (int u : T.U[i]) add_run(u);
         for (int w : T.W[i]) add_run(w);
     }
-    // a segment is one warp's: at least four a resident warp, 2^11 to 2^14 pairs
-    const long cap32 = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (80L * P.ctx->num_sms)));
-    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, std::min(P.tune.near_seg_pairs, cap32), 64);
+    // a segment is one warp's: at least four a resident warp, 2^11 to 2^14 pairs; or as the tuning table has it
+    const long own = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (80L * P.ctx->num_sms)));
+    const long cap32 = P.tune.near_seg_pairs == Tuning::NEAR_AUTO ? own : P.tune.near_seg_pairs;
+    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, cap32, 64);
     S.nnear32_seg = tl32.empty() ? 0 : (int)S.h_seg32.size() / 4;
     S.nearff_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_segff, P.tune.nearff_seg_pairs, 128);
     S.nnearff_seg = tl32.empty() ? 0 : (int)S.h_segff.size() / 4;

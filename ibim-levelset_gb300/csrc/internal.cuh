@@ -312,7 +312,10 @@ struct OzWeights {
 
 // Launch parameters a plan takes from the tuning table (tuning.cpp) for its order and size.
 struct Tuning {
-    long near_seg_pairs = 1L << 17;    // FP32 near field: source-target pairs per work segment (CTA)
+    // FP32 near field: source-target pairs a work segment, which is one warp's; at the default the plan sizes them
+    // by its own pairs (mixed_lists_host)
+    static constexpr long NEAR_AUTO = 1L << 17;
+    long near_seg_pairs = NEAR_AUTO;
     long nearff_seg_pairs = 1L << 14;  // float-float near field
     int tc_form = 2;  // tensor-core M2L: 2 = two CTAs of two row tiles per SM, 4 = one CTA of four,
                       // 0 = persistent; 6, 7 = CTA pairs (2-SM MMAs of M = 256) with one or two

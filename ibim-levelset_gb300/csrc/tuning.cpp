@@ -1,7 +1,7 @@
 // Launch-parameter table: per Chebyshev order, rows (min_points, FP32 near-field segment pairs,
 // float-float segment pairs, tensor-core M2L launch form).  A plan takes the row of its order with
 // the largest min_points not above its source count (make_plan); without one the defaults hold
-// (2^17, 2^14, two CTAs per SM).  The rows come from the autotuner (ibim_autotune: timed matvecs
+// (2^17, which leaves the FP32 segments to the plan, 2^14, and form 2).  The rows come from the autotuner (ibim_autotune: timed matvecs
 // of a prepared solve per candidate, see capi.cu), loaded from a table file (ibim_tuning_load) or
 // set one by one (ibim_tuning_set).  No counterpart in the reference.
 //

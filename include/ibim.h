@@ -294,8 +294,8 @@ int ibim_batch_solve(ibim_ctx ctx, int nmol, const int *natoms, const double *ce
 
 /* ---- launch-parameter table and autotuner (no counterpart in the reference) ----
  * A plan of Chebyshev order p with N sources takes its launch parameters from the row of order p
- * with the largest min_points <= N: pairs per work segment of the FP32 and the float-float near
- * fields, and the tensor-core M2L's launch form (2 = persistent CTA pairs from order 4 and 128 pairs an operator,
+ * with the largest min_points <= N: pairs per work segment of the FP32 (one warp's; 2^17: as many as the plan's own
+ * pairs ask for, 2^11 to 2^14) and the float-float near fields, and the tensor-core M2L's launch form (2 = persistent CTA pairs from order 4 and 128 pairs an operator,
  * else two CTAs of two row tiles per SM, 4 = one CTA of four, 0 = persistent, 6 / 7 = CTA pairs of 2-SM MMAs with one / two row-tile pairs per CTA;
  * 0, 6 and 7 in the scaled FP16 operand form).  They change the partition of the same work only.
  * Without a row the defaults hold (2^17, 2^14, 2). */
