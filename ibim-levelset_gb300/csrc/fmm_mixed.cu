@@ -644,14 +644,33 @@ void mixed_lists_host(const Plan &P, TargetSet &S) {
             tl32.push_back(i);
             nt32.push_back((int)(S.end[i] - S.begin[i]));
         }
+    // a segment is one warp's: at least four a resident warp, 2^11 to 2^14 pairs; or as the tuning table has it
+    const long own = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (80L * P.ctx->num_sms)));
+    const long cap32 = P.tune.near_seg_pairs == Tuning::NEAR_AUTO ? own : P.tune.near_seg_pairs;
+    const long min_src = 64;
+    // Source leaves of more points than one segment's are listed in pieces, so that several warps share a pair of large
+    // leaves (one leaf of 4,000 points: 26.6 ms in one warp, 12.7 where a CTA had it, 0.55 in pieces).
+    int most = 0;
+    for (int n : dfs_leaf)
+        if (nn > 0) most = std::max(most, T.src_end[n] - T.src_begin[n]);
+    auto piece = [&](long k) { return std::max(min_src, cap32 / std::max(1, nt32[k])); };
     const long ntl = (long)tl32.size();
     std::vector<int> ptr(ntl + 1, 0);
 #pragma omp parallel for schedule(static)
     for (long k = 0; k < ntl; ++k) {
         const int i = tl32[k];
+        const long len = piece(k);
         int c = 0;
-        for (int u : T.U[i]) c += cnt[u];
-        for (int w : T.W[i]) c += cnt[w];
+        auto count = [&](int root) {
+            if (most <= len) {
+                c += cnt[root];
+                return;
+            }
+            for (int r = first[root]; r < first[root] + cnt[root]; ++r)
+                c += div_up(T.src_end[dfs_leaf[r]] - T.src_begin[dfs_leaf[r]], len);
+        };
+        for (int u : T.U[i]) count(u);
+        for (int w : T.W[i]) count(w);
         ptr[k + 1] = c;
     }
     for (long k = 0; k < ntl; ++k) ptr[k + 1] += ptr[k];
@@ -661,26 +680,26 @@ void mixed_lists_host(const Plan &P, TargetSet &S) {
 #pragma omp parallel for schedule(dynamic, 64)
     for (long k = 0; k < ntl; ++k) {
         const int i = tl32[k];
+        const long len = piece(k);
         long q = ptr[k];
         auto add_run = [&](int root) {
-            for (int r = first[root]; r < first[root] + cnt[root]; ++r, ++q) {
+            for (int r = first[root]; r < first[root] + cnt[root]; ++r) {
                 const int n = dfs_leaf[r];
-                rng[2 * q] = T.src_begin[n];
-                rng[2 * q + 1] = T.src_end[n];
-                for (int a = 0; a < 3; ++a) {
-                    const double d = T.center[3 * n + a] - T.center[3 * i + a];
-                    off[3 * q + a] = (float)d;
-                    offl[3 * q + a] = (float)(d - (double)(float)d);
+                for (long b = T.src_begin[n]; b < T.src_end[n]; b += len, ++q) {
+                    rng[2 * q] = (int)b;
+                    rng[2 * q + 1] = (int)std::min<long>(b + len, T.src_end[n]);
+                    for (int a = 0; a < 3; ++a) {
+                        const double d = T.center[3 * n + a] - T.center[3 * i + a];
+                        off[3 * q + a] = (float)d;
+                        offl[3 * q + a] = (float)(d - (double)(float)d);
+                    }
                 }
             }
         };
         for (int u : T.U[i]) add_run(u);
         for (int w : T.W[i]) add_run(w);
     }
-    // a segment is one warp's: at least four a resident warp, 2^11 to 2^14 pairs; or as the tuning table has it
-    const long own = std::min(1L << 14, std::max(1L << 11, S.near_pairs / (80L * P.ctx->num_sms)));
-    const long cap32 = P.tune.near_seg_pairs == Tuning::NEAR_AUTO ? own : P.tune.near_seg_pairs;
-    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, cap32, 64);
+    S.near32_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_seg32, cap32, min_src);
     S.nnear32_seg = tl32.empty() ? 0 : (int)S.h_seg32.size() / 4;
     S.nearff_atomic = near_segments(tl32, nt32, ptr, rng, false, S.h_segff, P.tune.nearff_seg_pairs, 128);
     S.nnearff_seg = tl32.empty() ? 0 : (int)S.h_segff.size() / 4;

@@ -1,4 +1,4 @@
-"""The FP32 near field's work segments: the tuning table's size is the size they have."""
+"""The FP32 near field's work segments: the tuning table's size is the size they have, and large leaves are cut."""
 
 import os
 
@@ -41,3 +41,22 @@ def test_table_sets_the_segments(ctx, restore_table):
     size = np.abs(a).max(1, keepdims=True)
     assert 1e-12 < (np.abs(a - b) / size).max() < 2e-6
     assert (np.abs(a - product(1 << 17)) / size).max() < 1e-14  # the default: left to the plan
+
+
+@pytest.mark.parametrize("n,leaf", [(300, 400), (1100, 1200), (5003, 1300)])
+def test_large_leaves_in_pieces(ctx, restore_table, n, leaf):
+    """Leaves of more points than a segment's are cut: the sums round otherwise than in one segment a leaf, and agree with
+    the FP64 operator as mixed products do (1.5e-5 of the largest value, test_m2l_pair_gpu.py)."""
+    p, nrm, w = sphere_points(n, 2)
+    dens = np.random.default_rng(3).uniform(-1.0, 1.0, (4, n))
+    kp = ibim.kernel_params(0.3, 80.0, 2.0, 1.0)
+    tube = ctx.tube(p, nrm, w, H)
+    lib = ibim.lib()
+    lib.ibim_tuning_clear()
+    a = tube.plan(4, leaf, 10, precision=ibim.PRECISION_MIXED).apply(ibim.KERNEL_BIE_FUSED, kp, dens)
+    assert lib.ibim_tuning_set(4, 0, 1 << 24, 1 << 14, 2) == ibim.OK
+    b = tube.plan(4, leaf, 10, precision=ibim.PRECISION_MIXED).apply(ibim.KERNEL_BIE_FUSED, kp, dens)
+    ref = tube.plan(4, leaf, 10).apply(ibim.KERNEL_BIE_FUSED, kp, dens)
+    size = np.abs(ref).max(1, keepdims=True)
+    assert 1e-12 < (np.abs(a - b) / size).max()
+    assert (np.abs(a - ref) / size).max() < 1.5e-5 and (np.abs(b - ref) / size).max() < 1.5e-5
