@@ -1451,7 +1451,7 @@ static void fmm_run_fp64(Plan &P, int ts, const ibim_kernel_params &kpp, const d
         ProfScope ps_(PROF_NEAR64, count_work ? 70.0 * S.near_pairs : 0., count_work ? 56.0 * P.ns + 40.0 * S.nt : 0.,
                       st);
         const Near64K nk = make_near64(kp);
-        // the fast forms take FP32 seeds of d2 >= (tau h)^2 and n >= 0 of 2^-n/128
+        // the fast forms take FP32 seeds of d2 >= (tau h)^2 and n >= 0 of 2^(-n / 512)
         const int mode = !(kp.vr2 >= 1e-30) ? NEAR_GENERAL
                                             : (kp.kappa > 0. ? NEAR_YUKAWA : (kp.kappa == 0. ? NEAR_LAPLACE : NEAR_GENERAL));
         const int slot = entry & 3, field = entry >> 2;

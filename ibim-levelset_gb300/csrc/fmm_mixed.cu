@@ -32,7 +32,6 @@ struct KParams32 {
     float kappa_l2;     // -kappa log2(e): e^(-kappa r) = 2^(kappa_l2 r)
     float vr2_band;     // |d2 - vr2| below this: the cutoff is decided in FP64
     double vr2_64;      // the FP64 kernels' (tau h)^2
-    float vr2_guard;    // vr2 + 2 vr2_band: every pair inside the cutoff or its band lies below
 };
 
 static KParams32 to32(const KParams &k) {
@@ -40,7 +39,7 @@ static KParams32 to32(const KParams &k) {
                      (float)(k.vr * k.vr),  (float)k.k2in, (float)k.q4pi,
                      (float)k.k3f,          (float)(k.k2in / k.q4pi), (float)(k.k3f / k.q4pi),
                      (float)(-k.kappa * 1.4426950408889634),
-                     (float)(1e-4 * k.vr2), k.vr2, (float)(k.vr2 * (1.0 + 2e-4))};
+                     (float)(1e-4 * k.vr2), k.vr2};
 }
 
 namespace {

@@ -120,7 +120,8 @@ template <class T> struct HostArr {
     size_t size() const { return n; }
 };
 
-// Kernel categories timed with CUDA events when profiling is enabled on a context.
+// Kernel categories timed with CUDA events when profiling is enabled on a context.  PROF_M2M keeps its number and
+// has no launches: the upward pass is one (PROF_P2M).
 enum ProfCat {
     PROF_EXPAND = 0, PROF_WENO, PROF_COUNT, PROF_FLOOD, PROF_TUBE, PROF_OPS, PROF_P2M, PROF_M2M, PROF_M2L_V,
     PROF_M2L_X, PROF_L2L, PROF_NEAR, PROF_RHS, PROF_GMRES, PROF_M2L_V64, PROF_M2L_X64, PROF_NEAR64, PROF_M2L_VOZ,

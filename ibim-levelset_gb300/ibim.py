@@ -55,6 +55,7 @@ EXPORTS = [
     "ibim_grid_set_geometry", "ibim_batch_solve", "ibim_server_create_lockstep", "ibim_fmm_bytes_estimate",
     "ibim_tuning_set", "ibim_tuning_clear", "ibim_tuning_get", "ibim_tuning_load", "ibim_autotune",
 ]
+# "m2m" reports no launches: the whole upward pass is one, under "p2m"
 PROFILE_CATEGORIES = ["expand", "weno_stage", "count_gradient", "flood_fill", "tube_extract", "m2l_operators", "p2m",
                       "m2m", "m2l_v", "m2l_x", "l2l", "near_l2p", "rhs", "gmres_vectors", "m2l_v_fp64", "m2l_x_fp64",
                       "near_l2p_fp64", "m2l_v_sliced", "l2p", "l2p_fp64", "near_ff"]
