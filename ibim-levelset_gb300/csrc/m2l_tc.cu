@@ -2790,7 +2790,7 @@ static OzWeights oz64_weights(const Plan &P, const KParams &k) {
             const double u1 = std::fabs(t) < 1e-2 ? t * t * (0.5 - t / 3.) : 1. - e * (1. + t);
             const double u3 = std::fabs(t) < 1e-2 ? t * t * (0.5 - t * t / 8.) : 3. - e * (3. + t * (3. + t));
             A[0] = std::max(A[0], std::fabs(k.eps - 1. - k.eps * u1) / (r * r));
-            A[1] = std::max(A[1], -std::expm1(-t) / r);
+            A[1] = std::max(A[1], std::fabs(std::expm1(-t)) / r);
             A[2] = std::max(A[2], std::max(std::fabs(u1), std::fabs(u3)) / (r * r * r) * (k.k3f / k.q4pi));
             A[3] = std::max(A[3], std::fabs(1. - k.ieps + k.ieps * u1) / (r * r));
         }

@@ -142,7 +142,7 @@ int ibim_ctx_trim(ibim_ctx ctx);
 long ibim_launch_count(void);
 /* Per-category kernel timing with CUDA events on the stream each launch runs on.  mask bit k
  * enables category k: 0 expand, 1 WENO stage, 2 gradient count, 3 flood fill, 4 tube extraction,
- * 5 M2L operators, 6 P2M, 7 M2M, 8 M2L (V list), 9 M2L (X list), 10 L2L, 11 near field (+ L2P
+ * 5 M2L operators, 6 P2M and M2M, 7 none, 8 M2L (V list), 9 M2L (X list), 10 L2L, 11 near field (+ L2P
  * when it runs after the far field), 12 right-hand side, 13 GMRES vector kernels; FP64 versions of
  * 8, 9 and 11 are categories 14, 15 and 16 (categories 6-11 then count the mixed-precision
  * kernels); 17 is the V-list M2L of the mixed path's refinement residual (BF16 integer slices on

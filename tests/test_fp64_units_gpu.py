@@ -52,3 +52,9 @@ def test_one_half_alone(ctx, half, kappa):
     dens[3:] = 0.0 if half == 0 else dens[3:]
     dens[:3] = 0.0 if half == 1 else dens[:3]
     compare(ctx, 5, 40, 1500, 1.0, kappa, 1.0, dens)
+
+
+@pytest.mark.parametrize("ratio", [1.0, 1e6])
+def test_negative_kappa(ctx, ratio):
+    """Growing exponentials, which a product takes though a solve does not: neither kernel pair vanishes."""
+    compare(ctx, 5, 40, 1200, 1.0, -0.05, ratio)
