@@ -2767,9 +2767,9 @@ double m2l_oz64_op_bytes(int p) { return p > 7 ? 0. : oz64_image_bytes(p, true);
 // The weights of psi: at each source level the power of two nearest |K2| / |K1| (F's rows) and |K4| / |K3| (G's) at four
 // half-widths, in the midst of the V pairs' 2 to 10.  Off an operator's own ratio by d bits, the cut's error there
 // grows by up to d bits where the smaller group has the larger part of the sum; far operators, whose ratios are the
-// ones that differ, add little to it.  Errors of FMMs of 6,000 to 16,000 points against 80-bit ones, in units from
-// 1e-10 to 1e6 Angstrom, psi from 1e-6 to 1e6 times the dipole, screening t = kappa h from 0 to 1: 0.4 to 1.07 times the FP64 sums'
-// (with the ratios at 2 half-widths up to 2.1, at 1.5 up to 5; cut together up to 1e9).
+// ones that differ, add little to it.  Norm errors of 45 FMMs of 6,000 to 16,000 points against 80-bit ones, lengths in
+// 1e-10 to 1e6 units an Angstrom, psi from 1e-6 to 1e6 times the dipole, t = kappa h from 0 to 1: 0.40 to 1.17 times the FP64
+// sums', 0.84 in the mean of F (with the ratios at 2 half-widths up to 2.1, at 1.5 up to 5; cut together up to 1e9).
 // Without screening K2 and K3 are zero: psi leaves F's copy of the multipoles and the dipole G's.
 static OzWeights oz64_weights(const Plan &P, const KParams &k) {
     OzWeights W;

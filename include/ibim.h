@@ -57,7 +57,7 @@ extern "C" {
 /* ---- precision modes ---- */
 /* FP64 path; the M2L of orders up to 7 as digit products on the tensor cores: operator rows and multipoles cut to
  * 56 bits (orders to 5) or 54 (6, 7) below their largest value, the dipole and dphi apart, in any unit of length.  Norm
- * errors against 80-bit FMMs are 0.4 to 1.1 times those of the FP64 sums (which run where the images do not fit a third
+ * errors against 80-bit FMMs are 0.4 to 1.2 times those of the FP64 sums (which run where the images do not fit a third
  * of the device's memory, and at order 8).  A NaN or an infinity in the input gives NaN wherever it would be summed. */
 #define IBIM_PRECISION_FP64 0
 #define IBIM_PRECISION_MIXED 1 /* FP32-class far/near field inside FP64-class iterative refinement */
